@@ -73,6 +73,22 @@ SIGNATURES = {
 }
 
 _lib = None
+_ops = None
+
+
+def ops():
+    """The torch binding of the same library (``binding/cgnn_torch.cpp``): the layers' host path."""
+    global _ops
+    if _ops is None:
+        import torch  # noqa: F401  (the binding resolves against its libraries)
+        lib()  # and against this one
+        try:
+            from . import _cgnn_torch
+        except ImportError as e:
+            raise ImportError(f"{PKG / '_cgnn_torch.so'} is missing or does not load ({e}): build it with "
+                              "`python -m compressgnn_b200.build`") from e
+        _ops = _cgnn_torch
+    return _ops
 
 
 def lib():

@@ -2,6 +2,8 @@
 
 ``libcgnn_b200.so``   -- the sm_100a CUDA kernels behind the C ABI of ``include/cgnn_b200.h``
                          (``csrc/*.cu``, compiled by nvcc, one object per file, in parallel).
+``_cgnn_torch.so``    -- the same library bound to torch tensors with the layers' autograd nodes
+                         (``binding/*.cpp``, g++ against torch's headers).
 ``libcgnn_host.so``   -- host-side graph preparation (``host/*.cpp``, g++ with OpenMP), when
                          its sources exist.
 
@@ -20,6 +22,8 @@ HOST = PKG / "host"
 OBJ = PKG / "_build"
 CUDA_LIB = PKG / "libcgnn_b200.so"
 HOST_LIB = PKG / "libcgnn_host.so"
+BINDING = PKG / "binding"
+BINDING_LIB = PKG / "_cgnn_torch.so"
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
@@ -83,8 +87,30 @@ def build_host(verbose=False):
     return HOST_LIB
 
 
+def build_binding(verbose=False):
+    """Compile ``binding/*.cpp`` into ``_cgnn_torch.so`` (needs ``libcgnn_b200.so``, which it links against)."""
+    import sysconfig
+    sources = sorted(BINDING.glob("*.cpp"))
+    headers = sorted((PKG.parent / "include").glob("*.h"))
+    if not _stale(BINDING_LIB, sources + headers):
+        return BINDING_LIB
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    includes = include_paths() + [sysconfig.get_paths()["include"], str(Path(cuda_home) / "include")]
+    torch_lib = str(Path(torch.__file__).parent / "lib")
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_cgnn_torch",
+          "-DTORCH_API_INCLUDE_EXTENSION_H"] + [a for p in includes for a in ("-isystem", p)] +
+         [str(s) for s in sources] +
+         ["-o", str(BINDING_LIB), "-L" + str(PKG), "-lcgnn_b200", "-L" + torch_lib, "-lc10", "-lc10_cuda",
+          "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-L" + str(Path(cuda_home) / "lib64"), "-lcudart",
+          "-Wl,-rpath,$ORIGIN"], verbose)
+    return BINDING_LIB
+
+
 def build_all(verbose=False):
     lib, _ = build_cuda(verbose)
+    build_binding(verbose)
     return lib, build_host(verbose)
 
 
@@ -93,4 +119,5 @@ if __name__ == "__main__":
     if "--ptxas" in sys.argv:
         print("\n".join(out[1]))
     print(out[0])
+    print(build_binding(verbose=True))
     print(build_host(verbose=True))

@@ -30,7 +30,6 @@ from dataclasses import dataclass
 from typing import Any, Optional, Tuple
 
 import torch
-from torch.autograd.function import once_differentiable
 
 from .. import runtime as _native
 
@@ -43,20 +42,15 @@ def _require_cuda(x):
 # ---------------------------------------------------------------------------------------------
 # autograd functions
 # ---------------------------------------------------------------------------------------------
-class _Mean(torch.autograd.Function):
-    """``reps[g] = mean of the rows of x whose index is g``; first-order gradient only."""
+class _Mean:
+    """``_Mean.apply(x, index, counts)``: ``reps[g] = mean of the rows of x whose index is g``; first-order
+    gradient only (the autograd node is the native binding's)."""
 
     @staticmethod
-    def forward(ctx, x, index, counts):
+    def apply(x, index, counts):
         _require_cuda(x)
-        ctx.save_for_backward(index, counts)
-        return _native.cluster_mean(x.contiguous(), index, counts)
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad):
-        index, counts = ctx.saved_tensors
-        return _native.cluster_mean_backward(grad.contiguous(), index, counts), None, None
+        plan = _native.index_plan(index, counts.numel()).native if x.numel() else None
+        return _native.ops().mean(x, index, counts, plan)
 
 
 def _assign(input, planes, bits, workspace=None, process_group=None):
@@ -73,21 +67,14 @@ def _assign(input, planes, bits, workspace=None, process_group=None):
         return _native.cluster_assign_from_projection(partial, workspace)
 
 
-class Compressgnn_Cluster_Function(torch.autograd.Function):
-    """Assignment and mean in one uncached call (the reference's older entry point)."""
+class Compressgnn_Cluster_Function:
+    """``apply(input, random_vectors, param_H, is_training)``: assignment and mean in one uncached call (the
+    reference's older entry point); returns ``(reps, index, active)``."""
 
     @staticmethod
-    def forward(ctx, input, random_vectors, param_H, is_training):
+    def apply(input, random_vectors, param_H, is_training):
         index, counts, active = _assign(input, random_vectors, param_H)
-        ctx.save_for_backward(index, counts)
-        ctx.mark_non_differentiable(index)
-        return _native.cluster_mean(input.contiguous(), index, counts), index, active
-
-    @staticmethod
-    @once_differentiable
-    def backward(ctx, grad, _index_grad, _active_grad):
-        index, counts = ctx.saved_tensors
-        return _native.cluster_mean_backward(grad.contiguous(), index, counts), None, None, None
+        return _Mean.apply(input, index, counts), index, active
 
 
 # ---------------------------------------------------------------------------------------------

@@ -7,42 +7,18 @@ activation), and the bias gradient comes out of the same native call as the repr
 gradient.
 """
 import torch
-from torch.autograd.function import once_differentiable
 
 from .. import runtime as _native
 
 
-class _Reconstruct(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, src, index, bias, relu, dropout_p=0.0):
-        index = index.contiguous()
-        seed = 0
-        if dropout_p > 0.0:
-            # a fresh 63-bit key per call from torch's host generator (follows torch.manual_seed; no device sync)
-            seed = int(torch.randint(0, 2**63 - 1, (1,), dtype=torch.int64).item())
-        output = _native.cluster_reconstruct(src.contiguous(), index,
-                                             None if bias is None else bias.contiguous(), relu, dropout_p, seed)
-        ctx.save_for_backward(index, output)
-        ctx.groups, ctx.relu, ctx.has_bias, ctx.dropout_p = src.size(0), relu, bias is not None, dropout_p
-        return output
+class _Reconstruct:
+    """``apply(src, index, bias, relu, dropout_p=0.0)``: the native gather with its autograd node (in the
+    binding).  A fresh dropout key per call comes from torch's host generator."""
 
     @staticmethod
-    @once_differentiable
-    def backward(ctx, grad):
-        index, output = ctx.saved_tensors
-        # `output` is this Function's own forward result.  Without dropout the rows of a group are identical
-        # and one mask row per group suffices; with dropout every row has its own zeros (dropped or clamped
-        # elements alike), so the gradient rows are masked one by one and the sums rescaled.
-        dropped = ctx.dropout_p > 0.0
-        result = _native.cluster_reconstruct_backward(grad.contiguous(), index, output, ctx.groups,
-                                                      ctx.relu, return_bias_grad=ctx.has_bias,
-                                                      output_is_forward_result=not dropped)
-        if dropped:
-            scale = 1.0 / (1.0 - ctx.dropout_p)
-            result = tuple(t.mul_(scale) for t in result) if ctx.has_bias else result.mul_(scale)
-        if ctx.has_bias:
-            return result[0], None, result[1], None, None
-        return result, None, None, None, None
+    def apply(src, index, bias, relu, dropout_p=0.0):
+        return _native.ops().reconstruct(src, index, bias, relu, dropout_p,
+                                         _native.known_index_plan(index, src.size(0)))
 
 
 class Compressgnn_Reconstruct(torch.nn.Module):

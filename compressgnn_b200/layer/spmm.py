@@ -46,21 +46,15 @@ def _rule_buffer(graph, like, given):
 def _whole_pass(graph, x, backward, record, out, rule_out):
     """One direction in one native call (two when ``record`` asks for the time of the vertex pass)."""
     plan = graph.propagation_plan()
-    table = plan.whole_pass(backward, x.size(1), x.dtype)
+    if record is None:
+        return plan.native.run(x, backward, out, rule_out)
     rule_out = _rule_buffer(graph, x, rule_out)
     if out is None:
         out = torch.empty((graph.vertex_cnt, x.size(1)), dtype=x.dtype, device=x.device)
-    elif out.shape != (graph.vertex_cnt, x.size(1)) or out.dtype != x.dtype or not out.is_contiguous():
-        raise RuntimeError("out does not match the graph and the feature matrix")
-    if out.numel() == 0:
-        return out
-    with _native.on_device(x.device):
-        if record is None:
-            return _native.propagate_pass(table, x, rule_out, out)
-        last = table["n"] - 1
-        _native.propagate_pass(table, x, rule_out, out, 0, last - 1)
-        return _timed(record, "bwd_out" if backward else "fwd_out",
-                      lambda: _native.propagate_pass(table, x, rule_out, out, last, last))
+    last = plan.launches - 1
+    plan.native.run(x, backward, out, rule_out, 0, last - 1)
+    return _timed(record, "bwd_out" if backward else "fwd_out",
+                  lambda: plan.native.run(x, backward, out, rule_out, last, last))
 
 
 def _forward(graph, x, record=None, out=None, rule_out=None, per_block=False):
@@ -109,15 +103,14 @@ def compress_spmm(graph, x_j):
     return _forward(graph, x_j)
 
 
-class Compressgnn_SPMM_Function(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, graph, x_j):
-        ctx.graph = graph
-        return _forward(graph, x_j)
+class Compressgnn_SPMM_Function:
+    """``apply(graph, x_j)``: the propagation as a differentiable operator.  The autograd node lives in the
+    native binding, so neither direction runs interpreter code beyond this call."""
 
     @staticmethod
-    def backward(ctx, grad_output: Tensor):
-        return None, _backward(ctx.graph, grad_output)
+    def apply(graph, x_j):
+        _require_cuda(x_j)
+        return graph.propagation_plan().native.apply(x_j, False)
 
 
 class Compressgnn_SPMM(torch.nn.Module):

@@ -22,7 +22,7 @@ from collections import OrderedDict
 
 import torch
 
-from ._lib import check, lib  # noqa: F401  (lib is re-exported for the layer modules)
+from ._lib import check, lib, ops  # noqa: F401  (lib is re-exported for the layer modules)
 
 _METHODS = ("rowbalance_parreduce", "rowbalance_seqreduce", "rowbalance_rowcache",
             "nnzbalance_parreduce", "nnzbalance_seqreduce", "nnzbalance_rowcache")
@@ -92,11 +92,20 @@ def _require(cond, msg):
 class SegmentPlan:
     """Owner of a native ``cgnn_plan`` and of its scratch buffers."""
 
-    def __init__(self, handle, device):
-        self._handle = handle
+    def __init__(self, native, device):
+        """``native``: the plan's owner in the binding, or the address of a ``cgnn_plan`` to own."""
+        device = torch.device(device)
+        if isinstance(native, int):
+            native = ops().Plan(native, device.index if device.index is not None else torch.cuda.current_device())
+        self.native = native
         self.device = device
-        self._scratch = {}
         self._values = _TensorKeyedCache(limit=8)
+
+    def __getattr__(self, name):
+        """The plan's figures (``rows``, ``nnz``, ``split``, ...), read from the library when first asked for."""
+        if name.startswith("_") or name in ("native", "device"):
+            raise AttributeError(name)
+        handle = self.handle
         info = (ctypes.c_int64 * 8)()
         check(lib().cgnn_plan_info(handle, info))
         (self.rows, self.nnz, self.split, self.long_rows, self.chunks, self.direct_units,
@@ -107,10 +116,13 @@ class SegmentPlan:
         hist = (ctypes.c_int64 * 4)()
         check(lib().cgnn_plan_degrees(handle, hist))
         self.degree_p50, self.degree_p99, self.degree_max = int(hist[0]), int(hist[1]), int(hist[2])
+        if name not in self.__dict__:
+            raise AttributeError(name)
+        return self.__dict__[name]
 
     @property
     def handle(self):
-        return ctypes.c_void_p(self._handle)
+        return ctypes.c_void_p(self.native.handle)
 
     @classmethod
     def from_csr(cls, rowptr, col, rowptr1=None, col1=None, split=0):
@@ -170,21 +182,8 @@ class SegmentPlan:
     def scratch(self, width, dtype_code):
         """(pointer, bytes) of this plan's scratch for launches ``width`` columns wide on the
         current stream; allocated zeroed on first use (the ticket words must start at 0)."""
-        key = (int(width), dtype_code, _stream_ptr(self.device))
-        buf = self._scratch.get(key)
-        if buf is None:
-            nbytes = lib().cgnn_plan_scratch_bytes(self.handle, int(width), dtype_code)
-            buf = torch.zeros(max(int(nbytes), 16), dtype=torch.uint8, device=self.device)
-            self._scratch[key] = buf
-        return ctypes.c_void_p(buf.data_ptr()), buf.numel()
-
-    def __del__(self):
-        handle, self._handle = getattr(self, "_handle", None), None
-        if handle:
-            try:
-                lib().cgnn_plan_destroy(ctypes.c_void_p(handle))
-            except Exception:  # interpreter shutdown
-                pass
+        address, nbytes = self.native.scratch(int(width), dtype_code, _stream_ptr(self.device))
+        return ctypes.c_void_p(address), nbytes
 
 
 class _TensorKeyedCache:
@@ -239,6 +238,12 @@ def csr_plan(vlist, elist):
         plan = SegmentPlan.from_csr(vlist, elist)
         _csr_plans.put((vlist, elist), plan)
     return plan
+
+
+def known_index_plan(index, groups):
+    """The binding's plan of an assignment made here, or None for an index from elsewhere."""
+    plan = _index_plans.get((index,), (groups,))
+    return None if plan is None else plan.native
 
 
 def index_plan(index, groups):
@@ -306,21 +311,6 @@ def spmm_pair_with_plan(plan, value0, mat0, value1, mat1, out=None, accumulate=F
         check(lib().cgnn_spmm_pair(plan.handle, code, width, _ptr(value), _ptr(mat0), _ptr(mat1),
                                    _ptr(out), 1 if accumulate else 0, sp, sb,
                                    _stream_ptr(mat0.device)))
-    return out
-
-
-def propagate_pass(table, x, rule_out, out, first=0, last=None):
-    """Issue the launches ``first .. last`` of one propagation direction (``table`` from
-    ``PropagationPlan.whole_pass``) in one native call: rules gather from ``x`` into ``rule_out``, the
-    rule levels run in place, the fused vertex pass writes ``out``."""
-    n_rules, (need0, need1) = table["source_rows"]
-    rule_side, x_side = (need0, need1) if table["rule_term"] == 0 else (need1, need0)
-    _require(x.size(0) >= max(n_rules, x_side) and rule_out.size(0) >= rule_side,
-             "propagate: the graph refers to rows beyond the feature or rule matrix")
-    check(lib().cgnn_propagate(table["n"], table["plans"], table["vals"], table["scratch"], table["scratch_bytes"],
-                               table["code"], x.size(1), x.data_ptr(), rule_out.data_ptr() if rule_out.numel() else None,
-                               out.data_ptr(), table["rule_term"], first, table["n"] - 1 if last is None else last,
-                               table["stream"]))
     return out
 
 
@@ -452,11 +442,11 @@ def cluster_assign(input, planes, bits, workspace):
     if n == 0:
         return (torch.empty(0, dtype=torch.int64, device=device),
                 torch.zeros(1, dtype=torch.int32, device=device), 0)
-    with on_device(device):
-        codes = torch.empty(n, dtype=torch.int32, device=device)
-        check(lib().cgnn_cluster_codes(_dtype_code(input), _ptr(input), _ptr(planes), n,
-                                       input.size(1), bits, _ptr(codes), _stream_ptr(device)))
-        return _assign_from_codes(codes, n, bits, workspace, device)
+    need = lib().cgnn_cluster_workspace_bytes(n, bits)
+    _require(workspace[2].dtype == torch.uint8 and workspace[2].numel() >= need, "Workspace dtype/capacity mismatch")
+    ids, counts, active, plan = ops().assign(input, planes, bits, workspace[2])
+    _index_plans.put((ids,), SegmentPlan(plan, device), (active + 1,))
+    return ids, counts, active
 
 
 def cluster_assign_from_projection(proj, workspace):
