@@ -44,6 +44,13 @@ cgnn_stream_t current_stream(const Tensor &t) {
 
 void *data(const Tensor &t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr; }
 
+// These operators carry no forward-mode derivative: a dual number is refused, its tangent never dropped.
+void refuse_dual(const char *what, at::TensorList inputs) {
+    for (const Tensor &t : inputs)
+        TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(t), what,
+                                    " does not support forward-mode automatic differentiation");
+}
+
 // Owner of a native plan and of its scratch: one zero-initialised buffer per (width, dtype, stream), since
 // a launch leaves the ticket words zero and launches on one stream are ordered.
 class Plan {
@@ -233,6 +240,7 @@ std::shared_ptr<N> new_node() {
 
 // One direction with autograd (its derivative is the other direction).
 Tensor Propagation::apply(const Tensor &x, bool backward) {
+    refuse_dual("the propagation", {x});
     Tensor out;
     {
         at::AutoDispatchBelowADInplaceOrView below;
@@ -373,6 +381,7 @@ struct MeanBackward : public Node {
 };
 
 Tensor mean_autograd(const Tensor &x_in, const Tensor &index, const Tensor &counts, const PlanPtr &plan) {
+    refuse_dual("the bucket mean", {x_in});
     check_matrix(x_in);
     check_index(index, x_in);
     check_counts(counts, x_in);
@@ -451,6 +460,7 @@ Tensor reconstruct_autograd(const Tensor &src, const Tensor &index_in, const c10
     const Tensor index = index_in.contiguous();
     check_index(index, src);
     const Tensor bias = bias_in.has_value() ? *bias_in : Tensor();
+    refuse_dual("the reconstruction", {src, bias});
     check_bias(bias, src.size(1), src);
     TORCH_CHECK(p >= 0.0 && p < 1.0, "dropout probability must lie in [0, 1)");
     TORCH_CHECK(p == 0.0 || relu, "the fused dropout follows a ReLU (the backward reads its mask off the zeros)");
@@ -519,6 +529,7 @@ Tensor transform_autograd(const Tensor &x_in, const Tensor &index, const Tensor 
     TORCH_CHECK(x_in.numel() == 0 || (plan && plan->rows == counts.numel() && plan->nnz == index.numel()),
                 "transform: plan does not match index/count");
     const Tensor bias = bias_in.has_value() ? *bias_in : Tensor();
+    refuse_dual("the transformation", {x_in, weight, bias});
     check_bias(bias, weight.size(0), x_in);
     TORCH_CHECK(p >= 0.0 && p < 1.0, "dropout probability must lie in [0, 1)");
     TORCH_CHECK(p == 0.0 || relu, "the fused dropout follows a ReLU (the backward reads its mask off the zeros)");

@@ -410,3 +410,20 @@ def test_host_propagation_queue_matches_resident_passes(depth):
         pipe.forward(sources[0][:, :8].contiguous(), results[0])
     with pytest.raises(RuntimeError):
         pipe.forward(sources[0].cuda(), results[0])
+
+
+def test_forward_mode_is_refused():
+    """The native autograd nodes have no forward-mode derivative; a dual input raises and loses no tangent."""
+    import torch.autograd.forward_ad as fwd
+    from compressgnn_b200.layer import Compressgnn_Reconstruct
+    from compressgnn_b200.layer.spmm import Compressgnn_SPMM_Function
+    data = make_data(width=8)
+    data.to("cuda")
+    index = torch.randint(0, 4, (20,), device="cuda")
+    with fwd.dual_level():
+        x = fwd.make_dual(data.x, torch.ones_like(data.x))
+        reps = fwd.make_dual(torch.randn(4, 8, device="cuda"), torch.ones(4, 8, device="cuda"))
+        with pytest.raises(RuntimeError, match="forward-mode"):
+            Compressgnn_SPMM_Function.apply(data.edge_index, x)
+        with pytest.raises(RuntimeError, match="forward-mode"):
+            Compressgnn_Reconstruct()(reps, index)
