@@ -66,6 +66,11 @@ SIGNATURES = {
     "cgnn_sample_claim": (_c_int, [_c_ptr, _c_i64, _c_i64, _c_ptr, _c_ptr, _c_ptr, _c_ptr]),
     "cgnn_sample_relabel": (_c_int, [_c_ptr, _c_i64, _c_i64, _c_ptr, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr,
                                      _c_ptr, _c_ptr]),
+    "cgnn_sample_hops_bytes": (_c_size, [_c_ptr, _c_i64, _c_int, _c_ptr, _c_i64]),
+    "cgnn_sample_hops": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_int, _c_ptr, _c_i64, ctypes.c_uint64, _c_ptr, _c_ptr,
+                                  _c_size, _c_ptr, _c_ptr]),
+    "cgnn_sample_hops_result": (_c_int, [_c_ptr, _c_i64, _c_int, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
+                                         _c_ptr, _c_ptr, _c_ptr]),
     "cgnn_compress_csr_batch": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_int, _c_int, _c_ptr, _c_ptr]),
     "cgnn_compressed_info": (_c_int, [_c_ptr, _c_ptr]),
     "cgnn_compressed_copy": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr]),

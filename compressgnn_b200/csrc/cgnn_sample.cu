@@ -22,6 +22,10 @@
 // level numbered by the descent depth, which finds them only for rules without nested rules; on such
 // graphs both orders below are the reference's, on deeper ones they are what its comments describe.
 #include <algorithm>
+#include <vector>
+#include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "cgnn_common.cuh"
 
@@ -210,6 +214,255 @@ __global__ void seed_kernel(const int64_t *samples, int64_t count, int64_t n, in
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// All hops of a batch without a host round trip (cgnn_sample_hops).
+//
+// What bounds a batch is latency: 60 k edges are a few microseconds of traffic, but hop by hop the host had to
+// learn two sizes per hop (edges, new vertices) before it could allocate and go on, the picks were
+// one thread's chain of dependent index reads, and ~15 small launches stood between them.  Here
+// frontier node i of a hop owns `stride` = min(fan-out, largest degree) pick slots, so the buffers are
+// sized by a bound the host knows beforehand and the true sizes stay on the device:
+//   * a slot's position counts over the whole batch (seeds first, then hop after hop), and first[v] keeps
+//     the smallest position that named vertex v -- earlier hops have smaller positions, so one
+//     table serves seeds and all hops and nothing is committed in between;
+//   * ONE scan per hop over the slots counts edges (high word) and new vertices (low word), started from the
+//     totals of the hop before it; its value at first[v] IS the local id of v;
+//   * a warp picks for one node: the children of up to 32 rules are listed per step, and the lookups of Floyd's
+//     draws run side by side.
+// A batch of 1024 seeds with fan-outs 25 and 10 on the 325 k-node graph: 505 -> 131 us; the two pick kernels were 150 us of
+// it.  Going hop by hop stays for batches whose slots would exceed MAX_POSITIONS.
+// ---------------------------------------------------------------------------------------
+constexpr int32_t EMPTY_SLOT = -1;  // picked[]: no pick here
+constexpr int32_t BAD_VERTEX = -2;  // picked[]: an edge to a vertex outside the graph (reported; local id 0)
+constexpr int64_t MAX_POSITIONS = 8 << 20;  // see cgnn_sample_hops_bytes
+
+// counts[h], h = 0 .. hops + 1: (edges << 32 | samples) before hop h - 1 has run; counts[0] = 0, counts[1] = the seeds
+__global__ void hops_begin_kernel(const int64_t *seeds, int64_t batch, int64_t n, int64_t *samples, int32_t *first,
+                                  uint64_t *prefix, uint64_t *counts) {
+    GRID_STRIDE(i, batch) {
+        const int64_t v = seeds[i];
+        samples[i] = v;
+        prefix[i] = (uint64_t)i;
+        if (v >= 0 && v < n) atomicMin(&first[v], (int32_t)i);  // a repeated seed keeps its first position
+        else atomicOr(&g_sample_status, STATUS_BAD_INDEX);
+        if (i == 0) {
+            counts[0] = 0;
+            counts[1] = (uint64_t)batch;
+        }
+    }
+}
+
+__device__ __forceinline__ int32_t warp_exclusive(int32_t x, int lane, int32_t *sum) {
+    int32_t s = x;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, s, d);
+        if (lane >= d) s += t;
+    }
+    *sum = __shfl_sync(0xffffffffu, s, 31);
+    return s - x;
+}
+
+// Hands the children of the listed rules queue[0 .. rules) under (ptr, col), in list order, to store(position,
+// child) with positions from `used` up, below `most`; returns the position reached.  APPEND: the children join
+// the list itself while it is walked (`used` is its length).
+template <bool APPEND, typename Store>
+__device__ __forceinline__ int32_t list_children(const int64_t *ptr, const int64_t *col, const int32_t *queue,
+                                                 int32_t rules, int32_t used, int32_t most, int lane, Store store) {
+    for (int32_t head = 0; head < (APPEND ? used : rules); ) {
+        const int32_t chunk = min(32, (APPEND ? used : rules) - head);
+        int64_t b = 0;
+        int32_t cnt = 0, sum = 0;
+        if (lane < chunk) {
+            const int32_t rule = queue[head + lane];
+            b = ptr[rule];
+            cnt = (int32_t)max(min(ptr[rule + 1] - b, (int64_t)most), (int64_t)0);
+        }
+        const int32_t at = used + warp_exclusive(cnt, lane, &sum);
+        for (int32_t c = 0; c < cnt && at + c < most; ++c) store(at + c, col[b + c]);
+        used = min(most, used + sum);
+        head += chunk;
+        __syncwarp();
+        if (!APPEND && used == most) break;
+    }
+    return used;
+}
+
+// One warp per frontier node (grid-stride over the bound `nodes`; nodes past the real frontier leave empty
+// slots).  `queue` has the layout of `picked`.
+__global__ void __launch_bounds__(THREADS) hops_pick_kernel(const GraphView g, const int64_t *samples, const uint64_t *counts,
+                                                            int64_t nodes, int32_t stride, int64_t fanout, uint32_t hop,
+                                                            uint64_t seed, int32_t base, int32_t *picked, int32_t *queue,
+                                                            int32_t *first) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (THREADS / 32);
+    const int64_t begin = (uint32_t)counts[0], end = (uint32_t)counts[1];
+    for (int64_t i = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); i < nodes; i += warps) {
+        int32_t *slots = picked + i * stride, *list = queue + i * stride;
+        const int32_t base_i = base + (int32_t)(i * stride);
+        int64_t node = -1, degree = 0;
+        if (begin + i < end) {
+            node = samples[begin + i];
+            if (node >= 0 && node < g.n) degree = g.v_degree[node];
+            else if (lane == 0) atomicOr(&g_sample_status, STATUS_BAD_INDEX);
+        }
+        const int32_t k = degree <= 0 ? 0 : (int32_t)min(degree, (int64_t)stride);
+        auto pick = [&](int32_t t, int64_t v) {
+            if (v < 0 || v >= g.n) {
+                atomicOr(&g_sample_status, STATUS_BAD_INDEX);
+                slots[t] = BAD_VERTEX;
+                return;
+            }
+            slots[t] = (int32_t)v;
+            if (first[v] > base_i + t) atomicMin(&first[v], base_i + t);
+        };
+        if (k > 0 && fanout >= degree) {  // everything, in list order
+            const int64_t vb = g.v2v_ptr[node], rb = g.v2r_ptr[node];
+            int32_t out = (int32_t)max(min(g.v2v_ptr[node + 1] - vb, (int64_t)k), (int64_t)0);
+            int32_t rules = (int32_t)max(min(g.v2r_ptr[node + 1] - rb, (int64_t)k), (int64_t)0);
+            for (int32_t t = lane; t < out; t += 32) pick(t, g.v2v_col[vb + t]);
+            if (out < k) {
+                // breadth-first list of the rules below the node (each holds >= 1 vertex: rules <= k)
+                for (int32_t t = lane; t < rules; t += 32) list[t] = (int32_t)g.v2r_col[rb + t];
+                __syncwarp();
+                rules = list_children<true>(g.r2r_ptr, g.r2r_col, list, 0, rules, k, lane,
+                                            [&](int32_t t, int64_t rule) { list[t] = (int32_t)rule; });
+                out = list_children<false>(g.r2v_ptr, g.r2v_col, list, rules, out, k, lane, pick);
+            }
+            if (out < k) {
+                if (lane == 0) atomicOr(&g_sample_status, STATUS_BAD_CSR);  // the degree table does not match the graph
+                for (int32_t t = out + lane; t < k; t += 32) pick(t, node);
+            }
+        } else if (k > 0) {  // Floyd: k distinct indices below degree; list[] keeps the indices of earlier chunks
+            const int64_t frontier_id = begin + i;
+            for (int32_t t0 = 0; t0 < k; t0 += 32) {
+                const int32_t t = t0 + lane, j = (int32_t)(degree - k + t);  // j >= 1
+                int32_t index = -1 - lane;                                   // idle lanes: equal to nothing
+                if (t < k) {
+                    const uint32_t word =
+                        philox_first_word((uint32_t)frontier_id, (uint32_t)(frontier_id >> 32), (uint32_t)t, hop, seed);
+                    index = (int32_t)(((uint64_t)word * (uint64_t)j) >> 32);  // uniform below j
+                }
+                bool taken = false;
+                for (int32_t s = 0; s < t0; ++s) taken |= list[s] == index;
+                if (taken) index = j;
+                const int32_t drawn = index;
+                const int32_t chunk = min(32, k - t0);
+                for (int32_t u = 0; u < chunk; ++u) {  // lane u is final when its turn comes
+                    const int32_t other = __shfl_sync(0xffffffffu, index, u);
+                    if (!taken && lane > u && t < k && other == drawn) {
+                        taken = true;
+                        index = j;
+                    }
+                }
+                if (t < k) {
+                    list[t] = index;
+                    int64_t v = neighbor_at(g, node, index);
+                    if (v < 0) {
+                        atomicOr(&g_sample_status, STATUS_BAD_CSR);
+                        v = node;
+                    }
+                    pick(t, v);
+                }
+                __syncwarp();
+            }
+        }
+        for (int32_t t = k + lane; t < stride; t += 32) slots[t] = EMPTY_SLOT;
+        __syncwarp();
+    }
+}
+
+// What slot p of the hop adds to the totals: one edge (high word), one vertex (low word) if it is the first to name it.
+struct SlotCount {
+    const int32_t *picked, *first;
+    int32_t base;
+    __device__ uint64_t operator()(int32_t p) const {
+        const int32_t v = picked[p];
+        if (v == EMPTY_SLOT) return 0;
+        return (1ull << 32) | (v >= 0 && first[v] == base + p ? 1ull : 0ull);
+    }
+};
+using SlotIterator = thrust::transform_iterator<SlotCount, thrust::counting_iterator<int32_t>, uint64_t, uint64_t>;
+
+__global__ void hops_relabel_kernel(SlotCount slot, int64_t slots, int32_t stride, const uint64_t *prefix, uint64_t *counts,
+                                    int32_t *rows, int32_t *cols, int64_t *samples) {
+    const int32_t begin = (int32_t)(uint32_t)counts[0];
+    GRID_STRIDE(p, slots) {
+        const int32_t v = slot.picked[p];
+        const uint64_t here = prefix[slot.base + p], adds = slot((int32_t)p);
+        if (v != EMPTY_SLOT) {
+            const uint32_t edge = (uint32_t)(here >> 32);
+            rows[edge] = begin + (int32_t)((uint32_t)p / (uint32_t)stride);
+            cols[edge] = v >= 0 ? (int32_t)(uint32_t)prefix[slot.first[v]] : 0;
+            if (adds & 1) samples[(uint32_t)here] = v;
+        }
+        if (p == slots - 1) counts[2] = here + adds;
+    }
+}
+
+// The results in their own arrays, and the table back to "nothing seen" for the next batch.
+__global__ void hops_finish_kernel(const int64_t *samples, const int32_t *rows, const int32_t *cols, int64_t nodes,
+                                   int64_t edges, int64_t n, int32_t *first, int64_t *samples_out, int64_t *rows_out,
+                                   int64_t *cols_out) {
+    GRID_STRIDE(i, nodes) {
+        const int64_t v = samples[i];
+        samples_out[i] = v;
+        if (v >= 0 && v < n) first[v] = NO_LOCAL_ID;
+    }
+    GRID_STRIDE(e, edges) {
+        rows_out[e] = rows[e];
+        cols_out[e] = cols[e];
+    }
+}
+
+// Slots of every hop and the layout of the workspace (the scan's scratch comes last).
+struct HopsLayout {
+    std::vector<int64_t> nodes, stride;  // per hop: bound of the frontier, slots per node
+    int64_t slots = 0, room = 0;         // all slots; bound of the samples
+    size_t counts = 0, samples = 0, prefix = 0, picked = 0, rows = 0, cols = 0, temp = 0, temp_bytes = 0, total = 0;
+    bool fits = false;
+};
+
+static HopsLayout hops_layout(const cgnn_sample_graph *g, int64_t batch, int hops, const int64_t *fanouts,
+                              int64_t largest_degree, bool with_temp = true) {
+    HopsLayout L;
+    if (batch > MAX_POSITIONS || g->vertices >= INT32_MAX || g->rules >= INT32_MAX || largest_degree >= INT32_MAX) return L;
+    int64_t frontier = batch, most = 0;
+    L.room = batch;
+    for (int h = 0; h < hops; ++h) {
+        const int64_t stride = std::min(fanouts[h], largest_degree);
+        if (stride <= 0 || frontier == 0) break;  // nothing from here on
+        if (stride > MAX_POSITIONS || frontier * stride + L.slots + batch > MAX_POSITIONS) return L;
+        L.nodes.push_back(frontier);
+        L.stride.push_back(stride);
+        const int64_t slots = frontier * stride;
+        most = std::max(most, slots);
+        L.slots += slots;
+        frontier = std::min(slots, g->vertices);
+    }
+    L.room = batch + std::min(L.slots, g->vertices);
+    if (most > 0 && with_temp)
+        cub::DeviceScan::ExclusiveScan(nullptr, L.temp_bytes, SlotIterator(thrust::counting_iterator<int32_t>(0), SlotCount{}),
+                                       (uint64_t *)nullptr, ::cuda::std::plus<>{},
+                                       cub::FutureValue<uint64_t>((uint64_t *)nullptr), (int)most);
+    size_t used = 0;
+    auto span = [&](size_t bytes) {
+        const size_t at = used;
+        used += align_up(std::max<size_t>(bytes, 16), 256);
+        return at;
+    };
+    L.counts = span(((size_t)hops + 2) * 8);
+    L.samples = span((size_t)L.room * 8);
+    L.prefix = span((size_t)(batch + L.slots) * 8);
+    L.picked = span((size_t)L.slots * 4);
+    L.rows = span((size_t)L.slots * 4);
+    L.cols = span((size_t)L.slots * 4);
+    L.temp = span(L.temp_bytes);
+    L.total = used;
+    L.fits = true;
+    return L;
+}
+
 static GraphView view_of(const cgnn_sample_graph *g) {
     GraphView v;
     v.v2v_ptr = g->v2v_ptr, v.v2v_col = g->v2v_col, v.v2r_ptr = g->v2r_ptr, v.v2r_col = g->v2r_col;
@@ -287,6 +540,75 @@ int cgnn_sample_relabel(const int64_t *picked, int64_t total, int64_t vertices, 
                                                              target, samples);
     CGNN_LAUNCH_CHECK();
     commit_kernel<<<blocks_for(total), THREADS, 0, stream>>>(picked, total, is_new, rank, end, local_of, first);
+    CGNN_LAUNCH_CHECK();
+    return CGNN_OK;
+}
+
+size_t cgnn_sample_hops_bytes(const cgnn_sample_graph *graph, int64_t batch, int hops, const int64_t *fanouts,
+                              int64_t largest_degree) {
+    if (graph == nullptr || batch <= 0 || hops < 0 || (hops > 0 && fanouts == nullptr)) return 0;
+    const HopsLayout L = hops_layout(graph, batch, hops, fanouts, largest_degree);
+    return L.fits ? L.total : 0;
+}
+
+int cgnn_sample_hops(const cgnn_sample_graph *graph, const int64_t *seeds, int64_t batch, int hops, const int64_t *fanouts,
+                     int64_t largest_degree, uint64_t seed, int32_t *first, void *workspace, size_t workspace_bytes,
+                     int64_t sizes[2], cgnn_stream_t stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    CGNN_REQUIRE(graph && seeds && first && workspace && sizes && batch > 0 && hops >= 0 && (hops == 0 || fanouts),
+                 "sample_hops: null argument");
+    const HopsLayout L = hops_layout(graph, batch, hops, fanouts, largest_degree);
+    CGNN_REQUIRE(L.fits && workspace_bytes >= L.total, "sample_hops: the workspace does not fit this batch");
+    CGNN_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "sample_hops: workspace must be 256-byte aligned");
+    char *base = reinterpret_cast<char *>(workspace);
+    uint64_t *counts = reinterpret_cast<uint64_t *>(base + L.counts), *prefix = reinterpret_cast<uint64_t *>(base + L.prefix);
+    int64_t *samples = reinterpret_cast<int64_t *>(base + L.samples);
+    int32_t *picked = reinterpret_cast<int32_t *>(base + L.picked), *rows = reinterpret_cast<int32_t *>(base + L.rows);
+    int32_t *cols = reinterpret_cast<int32_t *>(base + L.cols);
+    const GraphView view = view_of(graph);
+    hops_begin_kernel<<<blocks_for(batch), THREADS, 0, stream>>>(seeds, batch, graph->vertices, samples, first, prefix, counts);
+    CGNN_LAUNCH_CHECK();
+    int64_t done = 0;  // slots of the hops before this one
+    const int run = (int)L.nodes.size();
+    for (int h = 0; h < run; ++h) {
+        const int64_t nodes = L.nodes[h], stride = L.stride[h], slots = nodes * stride;
+        const SlotCount slot{picked + done, first, (int32_t)(batch + done)};
+        // the rule lists use the slots' own part of `rows`: edges are written below it (edges <= slots so far)
+        const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(nodes, THREADS / 32), 148 * 64);
+        hops_pick_kernel<<<grid, THREADS, 0, stream>>>(view, samples, counts + h, nodes, (int32_t)stride, fanouts[h],
+                                                       (uint32_t)h, seed, slot.base, picked + done, rows + done, first);
+        CGNN_LAUNCH_CHECK();
+        size_t temp_bytes = L.temp_bytes;
+        CGNN_CUDA(cub::DeviceScan::ExclusiveScan(base + L.temp, temp_bytes,
+                                                 SlotIterator(thrust::counting_iterator<int32_t>(0), slot),
+                                                 prefix + slot.base, ::cuda::std::plus<>{},
+                                                 cub::FutureValue<uint64_t>(counts + h + 1), (int)slots, stream));
+        hops_relabel_kernel<<<blocks_for(slots), THREADS, 0, stream>>>(slot, slots, (int32_t)stride, prefix, counts + h, rows,
+                                                                       cols, samples);
+        CGNN_LAUNCH_CHECK();
+        done += slots;
+    }
+    uint64_t last = 0;
+    CGNN_CUDA(cudaMemcpyAsync(&last, counts + run + 1, sizeof(last), cudaMemcpyDeviceToHost, stream));
+    CGNN_CUDA(cudaStreamSynchronize(stream));
+    sizes[0] = (int64_t)(last & 0xffffffffu);
+    sizes[1] = (int64_t)(last >> 32);
+    return CGNN_OK;
+}
+
+int cgnn_sample_hops_result(const cgnn_sample_graph *graph, int64_t batch, int hops, const int64_t *fanouts,
+                            int64_t largest_degree, const int64_t sizes[2], int32_t *first, const void *workspace,
+                            int64_t *samples_out, int64_t *rows_out, int64_t *cols_out, cgnn_stream_t stream) {
+    CGNN_REQUIRE(graph && first && workspace && sizes && batch > 0, "sample_hops_result: null argument");
+    const HopsLayout L = hops_layout(graph, batch, hops, fanouts, largest_degree, false);
+    CGNN_REQUIRE(L.fits && sizes[0] >= 0 && sizes[0] <= L.room && sizes[1] >= 0 && sizes[1] <= L.slots &&
+                     samples_out != nullptr && (sizes[1] == 0 || (rows_out != nullptr && cols_out != nullptr)),
+                 "sample_hops_result: the sizes do not fit this batch");
+    const char *base = reinterpret_cast<const char *>(workspace);
+    hops_finish_kernel<<<blocks_for(std::max(sizes[0], sizes[1])), THREADS, 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const int64_t *>(base + L.samples), reinterpret_cast<const int32_t *>(base + L.rows),
+        reinterpret_cast<const int32_t *>(base + L.cols), sizes[0], sizes[1], graph->vertices, first, samples_out, rows_out,
+        cols_out);
     CGNN_LAUNCH_CHECK();
     return CGNN_OK;
 }

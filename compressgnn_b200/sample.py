@@ -78,6 +78,7 @@ class CompressGraphSampler:
                  "degree arrays do not match the graph")
         self._graph = _GraphStruct(*[t.data_ptr() if t.numel() else None for t in self._arrays],
                                    self.vertices, self.rules)
+        self._largest_degree = int(self._arrays[8].max().item()) if self.vertices else 0
         self._local_of = torch.full((self.vertices,), _NONE, dtype=torch.int32, device=device)
         self._first = torch.full((self.vertices,), _NONE, dtype=torch.int32, device=device)
 
@@ -97,6 +98,39 @@ class CompressGraphSampler:
         _require(seeds.dim() == 1, "input_node must be one-dimensional")
         if seed is None:
             seed = int(torch.randint(0, 2 ** 63 - 1, (1,), dtype=torch.int64).item())
+        fanouts = [min(max(int(k), -1), 2 ** 62) for k in num_neighbors]
+        if seeds.numel():
+            packed = (ctypes.c_int64 * max(len(fanouts), 1))(*fanouts)
+            room = lib().cgnn_sample_hops_bytes(ctypes.byref(self._graph), seeds.numel(), len(fanouts), packed,
+                                                self._largest_degree)
+            if room:
+                return self._all_hops(seeds, len(fanouts), packed, room, seed)
+        return self._hop_by_hop(seeds, fanouts, seed)
+
+    def _all_hops(self, seeds, hops, fanouts, room, seed):
+        """Every hop on the device in a workspace of ``room`` bytes; one synchronisation, for the sizes."""
+        device, g, batch = self.device, ctypes.byref(self._graph), seeds.numel()
+        with on_device(device):
+            stream = _stream_ptr(device)
+            workspace = torch.empty(room, dtype=torch.uint8, device=device)
+            sizes = (ctypes.c_int64 * 2)()
+            try:
+                check(lib().cgnn_sample_hops(g, _ptr(seeds), batch, hops, fanouts, self._largest_degree,
+                                             ctypes.c_uint64(seed), _ptr(self._first), _ptr(workspace), room, sizes,
+                                             stream))
+                samples = torch.empty(sizes[0], dtype=torch.int64, device=device)
+                rows, cols = (torch.empty(sizes[1], dtype=torch.int64, device=device) for _ in range(2))
+                check(lib().cgnn_sample_hops_result(g, batch, hops, fanouts, self._largest_degree, sizes,
+                                                    _ptr(self._first), _ptr(workspace), _ptr(samples), _ptr(rows),
+                                                    _ptr(cols), stream))
+            except BaseException:
+                self._first.fill_(_NONE)  # a batch that stopped half way may have left claims behind
+                raise
+        return samples, rows, cols
+
+    def _hop_by_hop(self, seeds, num_neighbors, seed):
+        """One hop at a time with exact sizes (two synchronisations per hop): batches whose slot bound is too large."""
+        device = self.device
         g = ctypes.byref(self._graph)
         rows, cols = [], []
         samples = seeds.clone()

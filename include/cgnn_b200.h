@@ -322,6 +322,22 @@ int cgnn_sample_claim(const int64_t *picked, int64_t total, int64_t vertices, co
 int cgnn_sample_relabel(const int64_t *picked, int64_t total, int64_t vertices, const int64_t *is_new,
                         const int64_t *rank, int64_t end, int32_t *local_of, int32_t *first,
                         int64_t *target, int64_t *samples, cgnn_stream_t stream);
+/* All hops of a batch in one call, the same result: the hops run back to back in a workspace sized by an upper
+ * bound (every frontier node owns min(fanout, largest_degree) slots), one synchronisation returns the
+ * sizes, and cgnn_sample_hops_result writes the three arrays and clears `first` for the next batch.
+ *   cgnn_sample_hops_bytes  workspace (256-byte aligned), or 0 when the bound exceeds 8 Mi slots -- wide
+ *                           fan-outs over many hops, whose slots would be mostly empty: go hop by hop
+ *   sizes                   [0] samples, [1] edges
+ * largest_degree: the maximum of vertex_degree; first: int32[vertices], INT32_MAX before the first batch. */
+size_t cgnn_sample_hops_bytes(const cgnn_sample_graph *graph, int64_t batch, int hops,
+                              const int64_t *fanouts, int64_t largest_degree);
+int cgnn_sample_hops(const cgnn_sample_graph *graph, const int64_t *seeds, int64_t batch, int hops,
+                     const int64_t *fanouts, int64_t largest_degree, uint64_t seed, int32_t *first,
+                     void *workspace, size_t workspace_bytes, int64_t sizes[2], cgnn_stream_t stream);
+int cgnn_sample_hops_result(const cgnn_sample_graph *graph, int64_t batch, int hops,
+                            const int64_t *fanouts, int64_t largest_degree, const int64_t sizes[2],
+                            int32_t *first, const void *workspace, int64_t *samples_out,
+                            int64_t *rows_out, int64_t *cols_out, cgnn_stream_t stream);
 
 #ifdef __cplusplus
 }

@@ -96,6 +96,39 @@ def test_nested_rules_and_the_sampler_object():
     rt.raise_on_device_status()
 
 
+@pytest.mark.parametrize("fanouts", [[1], [32], [33, 2], [70, 3], [25, 10], [400, 1], [4, 0, 3], [3, -1], [2, 2, 2, 2], []])
+def test_all_hops_at_once_equal_hop_by_hop(fanouts):
+    """Both routes of a call on the same batches: one node, repeated seeds, more nodes than a block of warps,
+    draws beyond one warp's lanes, take-all nodes with nested rules, empty hops."""
+    from compressgnn_b200 import runtime as rt
+    graph = nested_graph().to("cuda")
+    sampler = graph.neighbor_sampler()
+    rng = np.random.default_rng(3)
+    for batch in (1, 5, 64, 1500):
+        seeds = cu(rng.choice(graph.vertex_cnt, size=batch, replace=True))
+        slow = sampler._hop_by_hop(seeds, fanouts, 17)
+        fast = sampler(seeds, fanouts, seed=17)
+        for mine, theirs in zip(fast, slow):
+            assert mine.dtype == theirs.dtype and torch.equal(mine, theirs)
+        assert bool((sampler._first == 2 ** 31 - 1).all())
+    rt.raise_on_device_status()
+
+
+def test_wide_fanouts_go_hop_by_hop():
+    """A slot bound beyond the workspace limit takes the exact route; the answer is the same."""
+    graph = nested_graph().to("cuda")
+    sampler = graph.neighbor_sampler()
+    seeds = torch.arange(500, device="cuda")
+    called = []
+    exact = sampler._hop_by_hop
+    sampler._hop_by_hop = lambda *a: called.append(a) or exact(*a)
+    wide = sampler(seeds, [10 ** 9] * 200, seed=1)
+    assert called
+    del sampler._hop_by_hop
+    narrow = sampler(seeds, [10 ** 9], seed=1)
+    assert all(torch.equal(a[:b.numel()], b) for a, b in zip(wide, narrow))
+
+
 def test_batches_of_the_benchmark_graph():
     """1024 seeds, fan-outs 25 and 10 on the 325 k-node graph: counts, membership and numbering."""
     import bench
@@ -151,4 +184,3 @@ def test_plain_graph_form(vectors):
         for mine, theirs in zip(got, want):
             np.testing.assert_array_equal(mine.cpu().numpy(), theirs)
     rt.raise_on_device_status()
-
