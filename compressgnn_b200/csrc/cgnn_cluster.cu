@@ -574,10 +574,10 @@ __global__ void codes_from_proj_kernel(const T *proj, int64_t n, int bits, int32
 
 // ---------------------------------------------------------------------------------------
 // Compaction of raw codes.  Workspace layout (all int32 unless noted), n rows:
-//   keys[2][n]  vals[2][n]  cid[n]  segstart[n+2]  active[1]  pad  | cub temp (bytes)
+//   keys[2][n]  vals[2][n]  cid[n]  segstart[n+2]  active[1]  pad  stats  | cub temp (bytes)
 // After cgnn_cluster_assign: vals[0] = permutation (rows sorted by code, ascending row
 // inside a bucket), segstart[b] = first sorted position of bucket b (b = 1..active),
-// segstart[0] = 0 (bucket 0 is always empty), segstart[active+1] = n.
+// segstart[0] = 0 (bucket 0 is always empty), segstart[active+1] = n; cid[i] = bucket of sorted position i.
 // ---------------------------------------------------------------------------------------
 struct AssignLayout {
     int32_t *keys[2];
@@ -585,6 +585,7 @@ struct AssignLayout {
     int32_t *cid;
     int32_t *segstart;
     int32_t *active;
+    int *stats;
     void *temp;
     size_t temp_bytes;
     size_t total;
@@ -610,6 +611,7 @@ static AssignLayout assign_layout(void *base, int64_t n) {
     L.cid = reinterpret_cast<int32_t *>(p + off); off += nn;
     L.segstart = reinterpret_cast<int32_t *>(p + off); off += nn + 256;
     L.active = reinterpret_cast<int32_t *>(p + off); off += 256;
+    L.stats = reinterpret_cast<int *>(p + off); off += align_up(PLAN_STATS_WORDS * sizeof(int), 256);
     L.temp = p + off;
     L.temp_bytes = cub_temp_bytes(n);
     L.total = off + L.temp_bytes;
@@ -788,8 +790,8 @@ int cgnn_cluster_assign(const int32_t *codes, int64_t n, int bits, void *workspa
                                                         L.active);
     CGNN_LAUNCH_CHECK();
     // One synchronisation fetches `active`.  With it comes what the export step needs to build the
-    // bucket plan without another round trip: when the buckets are few enough for one CTA to scan
-    // (at most 2^20: the usual bit counts), the row statistics of the plan, taken on the device and
+    // bucket plan without another round trip: when there are at most 2^22 buckets (PLAN_DEVICE_MAX_ROWS:
+    // the usual bit counts), the row statistics of the plan, taken on the device and
     // written behind `active`; otherwise, speculatively, the head of the segment-start array.
     HostSegments &hs = host_segments();
     std::lock_guard<std::mutex> guard(hs.lock);
@@ -799,7 +801,8 @@ int cgnn_cluster_assign(const int32_t *codes, int64_t n, int bits, void *workspa
     hs.on_device = std::min<int64_t>(n, (int64_t)1 << bits) + 1 <= PLAN_DEVICE_MAX_ROWS;
     if (hs.on_device) {
         int32_t *header_dev = L.active + 16;  // inside the 256-byte slot of `active`
-        rc = plan_stats_on_device(L.segstart, L.active, n, 0, header_dev, stream);
+        rc = plan_stats_on_device(L.segstart, L.active, n, std::min<int64_t>(n, (int64_t)1 << bits) + 1, L.stats, header_dev,
+                                  stream);
         if (rc != CGNN_OK) return rc;
         int32_t *host = hs.reserve(16 + PLAN_HEADER_WORDS);
         CGNN_CUDA(cudaMemcpyAsync(host, L.active, sizeof(int32_t) * (16 + PLAN_HEADER_WORDS), cudaMemcpyDeviceToHost,
@@ -847,7 +850,7 @@ int cgnn_cluster_assign_export(const void *workspace, int64_t n, int64_t active,
         HostSegments &hs = host_segments();
         std::lock_guard<std::mutex> guard(hs.lock);
         if (hs.workspace == workspace && hs.n == n && hs.on_device && split == 0 && hs.start[0] == active) {
-            rc = plan_fill_on_device(p, L.segstart, L.vals[0], hs.start + 16, stream);
+            rc = plan_fill_on_device(p, L.segstart, L.vals[0], L.cid, hs.start + 16, stream);
         } else {
             const bool have = hs.workspace == workspace && hs.n == n && !hs.on_device && hs.valid == active + 2;
             rc = plan_build(p, rp, cl, split, stream, have ? hs.start + 1 : nullptr, false);

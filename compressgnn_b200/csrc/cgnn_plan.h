@@ -54,15 +54,19 @@ int plan_build(cgnn_plan *p, const int32_t *const rowptr[2], const int32_t *cons
 //                          to the host together with whatever else it waits for;
 //   plan_fill_on_device    (after the wait, header on the host) allocates the plan and lets kernels
 //                          write its lists and entries; no further wait, no host-side pass over the rows.
-// Rows are limited to PLAN_DEVICE_MAX_ROWS (one CTA scans them); the block has no values.
+// Rows are limited to PLAN_DEVICE_MAX_ROWS: every tile of 1024 rows adds up the totals of the tiles before it, work
+// that grows with the square of the rows (4 M rows: 170 MB of cached reads).  The block has no values;
+// `most_rows` bounds the row count before it is known, `stats` is device scratch of PLAN_STATS_WORDS ints and
+// row_of[i] the row of entry i.
 constexpr int PLAN_HEADER_WORDS = 16;
-constexpr int64_t PLAN_DEVICE_MAX_ROWS = 1 << 20;
+constexpr int PLAN_STATS_WORDS = 4160;
+constexpr int64_t PLAN_DEVICE_MAX_ROWS = 1 << 22;
 enum PlanHeader { PH_ROWS = 0, PH_SPLIT, PH_COMPACT, PH_IDENTITY, PH_DIRECT, PH_LONG, PH_ITEMS, PH_P50, PH_P99,
                   PH_MAX, PH_SHORT_ENTRIES, PH_VALID };
-int plan_stats_on_device(const int32_t *rowptr, const int32_t *last_row_dev, int64_t nnz, int split,
+int plan_stats_on_device(const int32_t *rowptr, const int32_t *last_row_dev, int64_t nnz, int64_t most_rows, int *stats,
                          int32_t *header_dev, cudaStream_t stream);
-int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col, const int32_t *header_host,
-                        cudaStream_t stream);
+int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col, const int32_t *row_of,
+                        const int32_t *header_host, cudaStream_t stream);
 
 // Device status word of each translation unit (read-and-clear).
 int segreduce_status(int *out);

@@ -1437,141 +1437,203 @@ int plan_build(cgnn_plan *p, const int32_t *const rowptr[2], const int32_t *cons
 }
 
 // ---------------------------------------------------------------------------------------
-// Plan construction on the device (see cgnn_plan.h): the decisions of plan_build, taken by one CTA.
+// Plan construction on the device (see cgnn_plan.h): the decisions of plan_build.
+//
+// What bounds it is the number of SMs at work and the longest serial stretch.  One CTA used to take the
+// statistics, one CTA the five prefix sums (34 and 59 us at 60 k rows, 121 us when the row pointers did
+// not fit its shared memory), and one warp copied a row's entries, however long (348 us when a few buckets
+// hold most of 325 k nodes).  Now the statistics are one pass over the whole GPU into a row-length histogram
+// that the last block to finish evaluates, the prefix sums go tile by tile (partial sums first), and
+// the entries are copied one per thread.  An assignment refresh of 2.45 M x 128 rows, 16 bits:
+// 546 -> 475 us.
 // ---------------------------------------------------------------------------------------
 constexpr int PLAN_CTA = 1024;
-constexpr int PLAN_HIST_CAP = 4096;
+constexpr int PLAN_HIST_CAP = 4096;  // lengths of PLAN_HIST_CAP and more share the last bin
+// stats[]: the histogram, then
+enum PlanStats { PS_MAX = PLAN_HIST_CAP + 1, PS_CAPPED_64, PS_CAPPED_128, PS_DONE, PS_END };  // (chunks of the rows in the
+                                                                                              // last bin for both splits)
+static_assert(PS_END <= PLAN_STATS_WORDS, "the statistics do not fit their slot");
 
 __global__ void __launch_bounds__(PLAN_CTA) plan_stats_kernel(const int32_t *rowptr, const int32_t *last_row_dev,
-                                                              int64_t nnz, int split_request, int32_t *header) {
+                                                              int64_t nnz, int *stats, int32_t *header) {
     __shared__ int hist[PLAN_HIST_CAP + 1];
-    __shared__ int s_max, s_split, s_short, s_long, s_items, s_short_entries;
+    __shared__ int s_last, s_p50, s_p99, s_short, s_not_long, s_items, s_short_entries;
     const int rows = *last_row_dev + 1;
     for (int i = threadIdx.x; i <= PLAN_HIST_CAP; i += PLAN_CTA) hist[i] = 0;
-    if (threadIdx.x == 0) s_max = s_short = s_long = s_items = s_short_entries = 0;
     __syncthreads();
-    int longest = 0;
-    for (int r = threadIdx.x; r < rows; r += PLAN_CTA) {
+    int longest = 0, capped64 = 0, capped128 = 0;
+    for (int r = blockIdx.x * PLAN_CTA + threadIdx.x; r < rows; r += gridDim.x * PLAN_CTA) {
         const int d = rowptr[r + 1] - rowptr[r];
         atomicAdd(&hist[min(d, PLAN_HIST_CAP)], 1);
         longest = max(longest, d);
-    }
-    atomicMax(&s_max, longest);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // smallest length whose cumulative count reaches ceil(q * rows): the host path's percentile
-        const int want50 = (rows + 1) / 2, want99 = (int)((99ll * rows + 99) / 100);
-        int seen = 0, p50 = -1, p99 = -1;
-        for (int d = 0; d <= PLAN_HIST_CAP && p99 < 0; ++d) {
-            seen += hist[d];
-            if (p50 < 0 && seen >= want50) p50 = d;
-            if (seen >= want99) p99 = d;
+        if (d >= PLAN_HIST_CAP) {
+            capped64 += (d + 63) / 64;
+            capped128 += (d + 127) / 128;
         }
-        header[PH_P50] = max(p50, 0);
-        header[PH_P99] = max(p99, 0);
-        s_split = split_request > 0 ? split_request : ((nnz > 64ll * rows || p99 > 512) ? 128 : 64);
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((threadIdx.x & 31) == 0) atomicMax(&stats[PS_MAX], longest);
+    if (capped64) {
+        atomicAdd(&stats[PS_CAPPED_64], capped64);
+        atomicAdd(&stats[PS_CAPPED_128], capped128);
     }
     __syncthreads();
-    const int split = s_split;
-    int n_short = 0, n_long = 0, n_items = 0, short_entries = 0;
-    for (int r = threadIdx.x; r < rows; r += PLAN_CTA) {
-        const int d = rowptr[r + 1] - rowptr[r];
+    for (int i = threadIdx.x; i <= PLAN_HIST_CAP; i += PLAN_CTA)
+        if (hist[i]) atomicAdd(&stats[i], hist[i]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&stats[PS_DONE], 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // ---- the last block: thread t owns the bins 4 t .. 4 t + 3 (rows in the last bin are all long) ----
+    static_assert(PLAN_HIST_CAP == 4 * PLAN_CTA, "four bins to a thread");
+    __shared__ int warp_sum[PLAN_CTA / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, bin0 = 4 * threadIdx.x;
+    int bins[4], own = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) own += bins[k] = __ldcg(&stats[bin0 + k]);
+    int seen = own;
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, seen, m);
+        if (lane >= m) seen += t;
+    }
+    if (lane == 31) warp_sum[warp] = seen;
+    if (threadIdx.x == 0) {
+        s_p50 = s_p99 = PLAN_HIST_CAP;
+        s_short = s_not_long = s_short_entries = 0;
+    }
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) seen += warp_sum[w];
+    seen -= own;
+    // smallest length whose cumulative count reaches ceil(q * rows): the host path's percentile
+    const int want50 = (rows + 1) / 2, want99 = (int)((99ll * rows + 99) / 100);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int upto = seen + bins[k];
+        if (seen < want50 && upto >= want50) s_p50 = bin0 + k;
+        if (seen < want99 && upto >= want99) s_p99 = bin0 + k;
+        seen = upto;
+    }
+    __syncthreads();
+    const int split = (nnz > 64ll * rows || s_p99 > 512) ? 128 : 64;
+    if (threadIdx.x == 0) s_items = __ldcg(&stats[split == 64 ? PS_CAPPED_64 : PS_CAPPED_128]);
+    __syncthreads();
+    int items = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int d = bin0 + k;
         if (d > split) {
-            ++n_long;
-            n_items += (d + split - 1) / split;
-        } else {
-            n_short += d > 0;
-            short_entries += d;
+            items += bins[k] * ((d + split - 1) / split);
+        } else if (bins[k]) {
+            atomicAdd(&s_not_long, bins[k]);
+            if (d > 0) atomicAdd(&s_short, bins[k]);
+            atomicAdd(&s_short_entries, bins[k] * d);
         }
     }
-    atomicAdd(&s_short, n_short);
-    atomicAdd(&s_long, n_long);
-    atomicAdd(&s_items, n_items);
-    atomicAdd(&s_short_entries, short_entries);
+    if (items) atomicAdd(&s_items, items);
     __syncthreads();
     if (threadIdx.x == 0) {
+        const int n_long = rows - s_not_long;
         const int compact = rows >= 1024 && 2ll * s_short < rows;
+        header[PH_P50] = s_p50;
+        header[PH_P99] = s_p99;
         header[PH_ROWS] = rows;
         header[PH_SPLIT] = split;
         header[PH_COMPACT] = compact;
-        header[PH_IDENTITY] = !compact && s_long == 0;
-        header[PH_DIRECT] = compact ? s_short : rows - s_long;
-        header[PH_LONG] = s_long;
+        header[PH_IDENTITY] = !compact && n_long == 0;
+        header[PH_DIRECT] = compact ? s_short : rows - n_long;
+        header[PH_LONG] = n_long;
         header[PH_ITEMS] = s_items;
-        header[PH_MAX] = s_max;
+        header[PH_MAX] = __ldcg(&stats[PS_MAX]);
         header[PH_SHORT_ENTRIES] = s_short_entries;
         header[PH_VALID] = 1;
     }
 }
 
-// One CTA: thread t owns a contiguous slice of the rows; five block-wide prefix sums place its listed
-// rows, long rows, chunks and entries; a second walk over the slice writes the lists.
-constexpr int PLAN_STAGED_ROWS = 50000;  // (rows + 1) * 4 bytes of dynamic shared memory beside the 20 KB of `scan`
-__global__ void __launch_bounds__(PLAN_CTA) plan_fill_kernel(const int32_t *rowptr, int rows, int split, int compact,
-                                                             int identity, int staged, int32_t *uptr, int32_t *urow,
-                                                             int4 *longs, int32_t *dst) {
-    __shared__ int scan[5][PLAN_CTA + 1];
-    extern __shared__ int32_t staged_rowptr[];
-    // A thread's slice of the row pointers is contiguous, so its reads from global memory are a chain of
-    // uncoalesced loads (about 90 us for 30 k rows); when the array fits it is first copied to shared memory
-    // with coalesced loads and both walks read it from there.
-    if (staged) {
-        for (int i = threadIdx.x; i <= rows; i += PLAN_CTA) staged_rowptr[i] = rowptr[i];
-        __syncthreads();
-        rowptr = staged_rowptr;
-    }
-    const int per = (rows + PLAN_CTA - 1) / PLAN_CTA;
-    const int r0 = min(rows, (int)threadIdx.x * per), r1 = min(rows, r0 + per);
-    int mine[5] = {0, 0, 0, 0, 0};  // listed rows, their entries, long rows, their entries, chunks
-    for (int r = r0; r < r1; ++r) {
-        const int d = rowptr[r + 1] - rowptr[r];
-        if (d > split) {
-            ++mine[2];
-            mine[3] += d;
-            mine[4] += (d + split - 1) / split;
-        } else if (!(compact && d == 0)) {
-            ++mine[0];
-            mine[1] += d;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 5; ++q) scan[q][threadIdx.x + 1] = mine[q];
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 5; ++q) scan[q][0] = 0;
+// What one row adds to the five running totals: listed rows, their entries, long rows, their entries, chunks.
+__device__ __forceinline__ void plan_row_adds(int d, int split, int compact, int (&adds)[5]) {
+    const bool is_long = d > split, listed = !is_long && !(compact && d == 0);
+    adds[0] = listed;
+    adds[1] = listed ? d : 0;
+    adds[2] = is_long;
+    adds[3] = is_long ? d : 0;
+    adds[4] = is_long ? (d + split - 1) / split : 0;
+}
+
+// Totals of each tile of PLAN_CTA rows.
+__global__ void __launch_bounds__(PLAN_CTA) plan_tiles_kernel(const int32_t *rowptr, int rows, int split, int compact,
+                                                              int *tiles) {
+    __shared__ int sum[5];
+    if (threadIdx.x < 5) sum[threadIdx.x] = 0;
     __syncthreads();
-    // inclusive prefix sums in place (Hillis-Steele over PLAN_CTA + 1 slots, slot 0 stays 0)
-    for (int step = 1; step <= PLAN_CTA; step <<= 1) {
-        int add[5];
-        const int i = threadIdx.x + 1;
+    const int r = blockIdx.x * PLAN_CTA + threadIdx.x;
+    int adds[5] = {0, 0, 0, 0, 0};
+    if (r < rows) plan_row_adds(rowptr[r + 1] - rowptr[r], split, compact, adds);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) add[q] = i >= step ? scan[q][i - step] : 0;
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 5; ++q) scan[q][i] += add[q];
-        __syncthreads();
+    for (int q = 0; q < 5; ++q) {
+        const int w = __reduce_add_sync(0xffffffffu, adds[q]);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&sum[q], w);
     }
-    int listed = scan[0][threadIdx.x], pos = scan[1][threadIdx.x], lrow = scan[2][threadIdx.x];
-    const int short_total = scan[1][PLAN_CTA];
-    int lpos = short_total + scan[3][threadIdx.x], item = scan[4][threadIdx.x];
-    for (int r = r0; r < r1; ++r) {
-        const int d = rowptr[r + 1] - rowptr[r];
-        if (d > split) {
-            const int chunks = (d + split - 1) / split;
-            longs[lrow++] = make_int4(r, item, chunks, lpos);
-            dst[r] = lpos;
-            item += chunks;
-            lpos += d;
-        } else if (!(compact && d == 0)) {
-            uptr[listed] = pos;
-            if (!identity) urow[listed] = r;
-            ++listed;
-            dst[r] = pos;
-            pos += d;
-        } else {
-            dst[r] = 0;
+    __syncthreads();
+    if (threadIdx.x < 5) tiles[blockIdx.x * 5 + threadIdx.x] = sum[threadIdx.x];
+}
+
+// The work lists of one tile of rows: totals of the tiles before it, a scan over its own rows, then one row a thread.
+__global__ void __launch_bounds__(PLAN_CTA) plan_fill_kernel(const int32_t *rowptr, int rows, int split, int compact,
+                                                             int short_total, const int *tiles, int32_t *uptr, int32_t *urow,
+                                                             int4 *longs, int32_t *dst) {
+    __shared__ int before[5], warp_sum[5][PLAN_CTA / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 5) before[threadIdx.x] = 0;
+    __syncthreads();
+    int ahead[5] = {0, 0, 0, 0, 0};
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += PLAN_CTA)
+#pragma unroll
+        for (int q = 0; q < 5; ++q) ahead[q] += tiles[t * 5 + q];
+    const int r = blockIdx.x * PLAN_CTA + threadIdx.x;
+    int adds[5] = {0, 0, 0, 0, 0}, at[5];
+    const int d = r < rows ? rowptr[r + 1] - rowptr[r] : 0;
+    if (r < rows) plan_row_adds(d, split, compact, adds);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        const int w = __reduce_add_sync(0xffffffffu, ahead[q]);
+        if (lane == 0 && w) atomicAdd(&before[q], w);
+        at[q] = adds[q];
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, at[q], m);
+            if (lane >= m) at[q] += t;
         }
+        if (lane == 31) warp_sum[q][warp] = at[q];
     }
-    if (threadIdx.x == PLAN_CTA - 1) uptr[scan[0][PLAN_CTA]] = short_total;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+        at[q] += before[q] - adds[q] + __reduce_add_sync(0xffffffffu, lane < warp ? warp_sum[q][lane] : 0);
+    }
+    if (r >= rows) return;
+    if (adds[2]) {
+        longs[at[2]] = make_int4(r, at[4], adds[4], short_total + at[3]);
+        dst[r] = short_total + at[3];
+    } else if (adds[0]) {
+        uptr[at[0]] = at[1];
+        if (urow) urow[at[0]] = r;
+        dst[r] = at[1];
+    } else {
+        dst[r] = 0;
+    }
+    if (r == rows - 1) uptr[at[0] + adds[0]] = short_total;
+}
+
+// Entry i of the sorted order (row row_of[i], column col[i]) to its place in the plan.
+__global__ void __launch_bounds__(256) plan_entries_kernel(const int32_t *rowptr, const int32_t *col, const int32_t *row_of,
+                                                           const int32_t *dst, int total, int32_t *entries) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+        const int r = row_of[i];
+        entries[dst[r] + (i - rowptr[r])] = col[i];
+    }
 }
 
 // One thread per chunk: find its long row (the last one whose first chunk is not beyond it).
@@ -1591,15 +1653,16 @@ __global__ void plan_items_kernel(const int32_t *rowptr, const int4 *longs, int 
     }
 }
 
-int plan_stats_on_device(const int32_t *rowptr, const int32_t *last_row_dev, int64_t nnz, int split,
+int plan_stats_on_device(const int32_t *rowptr, const int32_t *last_row_dev, int64_t nnz, int64_t most_rows, int *stats,
                          int32_t *header_dev, cudaStream_t stream) {
-    CGNN_CUDA(cudaMemsetAsync(header_dev, 0, sizeof(int32_t) * PLAN_HEADER_WORDS, stream));
-    plan_stats_kernel<<<1, PLAN_CTA, 0, stream>>>(rowptr, last_row_dev, nnz, split, header_dev);
+    CGNN_CUDA(cudaMemsetAsync(stats, 0, sizeof(int) * PLAN_STATS_WORDS, stream));
+    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(most_rows, PLAN_CTA), 148));
+    plan_stats_kernel<<<blocks, PLAN_CTA, 0, stream>>>(rowptr, last_row_dev, nnz, stats, header_dev);
     CGNN_LAUNCH_CHECK();
     return CGNN_OK;
 }
 
-int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col, const int32_t *h,
+int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col, const int32_t *row_of, const int32_t *h,
                         cudaStream_t stream) {
     CGNN_REQUIRE(h[PH_VALID] == 1 && h[PH_ROWS] == p->rows, "plan: the device-side row statistics do not match");
     const int64_t rows = p->rows, total = p->nnz[0];
@@ -1621,8 +1684,9 @@ int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col,
     const size_t o_items = o_urow + span(identity ? 0 : (size_t)p->n_direct * 4);
     const size_t o_longs = o_items + span((size_t)p->n_items * 16);
     const size_t o_dst = o_longs + span((size_t)p->n_long * 16);
-    const size_t o_maxsrc = o_dst + span((size_t)rows * 4);
-    const size_t o_entries = o_maxsrc + span(2 * 4);
+    const int64_t tiles = ceil_div(rows, PLAN_CTA);
+    const size_t o_tiles = o_dst + span((size_t)rows * 4);
+    const size_t o_entries = o_tiles + span((size_t)tiles * 5 * 4);
     const size_t bytes = o_entries + span((size_t)total * 4);
     p->home = stream;
     p->pooled = pool_alloc(&p->block, bytes, stream) == cudaSuccess;
@@ -1643,16 +1707,11 @@ int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col,
     p->entries = reinterpret_cast<int32_t *>(base + o_entries);
     p->vperm = nullptr;
     int32_t *dst = reinterpret_cast<int32_t *>(base + o_dst);
-    int32_t *max_source = reinterpret_cast<int32_t *>(base + o_maxsrc);
-    CGNN_CUDA(cudaMemsetAsync(max_source, 0xff, 2 * sizeof(int32_t), stream));
-    const bool staged = rows < PLAN_STAGED_ROWS;
-    const size_t staged_bytes = staged ? ((size_t)rows + 1) * sizeof(int32_t) : 0;
-    if (staged)  // per device and cheap: repeated at every call rather than tracked
-        CGNN_CUDA(cudaFuncSetAttribute(plan_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       PLAN_STAGED_ROWS * (int)sizeof(int32_t)));
-    plan_fill_kernel<<<1, PLAN_CTA, staged_bytes, stream>>>(rowptr, (int)rows, p->split, p->compact, identity ? 1 : 0,
-                                                            staged ? 1 : 0, p->uptr,
-                                                            reinterpret_cast<int32_t *>(base + o_urow), p->longs, dst);
+    int *tile_sums = reinterpret_cast<int *>(base + o_tiles);
+    plan_tiles_kernel<<<(unsigned)tiles, PLAN_CTA, 0, stream>>>(rowptr, (int)rows, p->split, p->compact, tile_sums);
+    CGNN_LAUNCH_CHECK();
+    plan_fill_kernel<<<(unsigned)tiles, PLAN_CTA, 0, stream>>>(rowptr, (int)rows, p->split, p->compact, h[PH_SHORT_ENTRIES],
+                                                               tile_sums, p->uptr, p->urow, p->longs, dst);
     CGNN_LAUNCH_CHECK();
     if (p->n_items > 0) {
         const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(p->n_items, 256), 148 * 8);
@@ -1661,9 +1720,8 @@ int plan_fill_on_device(cgnn_plan *p, const int32_t *rowptr, const int32_t *col,
         CGNN_LAUNCH_CHECK();
     }
     if (total > 0) {
-        const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(rows, 8), 148 * 16));
-        scatter_entries_kernel<<<blocks, 256, 0, stream>>>(rowptr, col, dst, nullptr, rows, 0, 0, p->entries, nullptr,
-                                                           max_source);
+        const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(total, 256), 148 * 16);
+        plan_entries_kernel<<<blocks, 256, 0, stream>>>(rowptr, col, row_of, dst, (int)total, p->entries);
         CGNN_LAUNCH_CHECK();
     }
     return CGNN_OK;

@@ -214,3 +214,33 @@ def test_argument_errors_raise_runtime_error(rt):
     out = rt.cluster_reconstruct(torch.randn(2, 4, device="cuda"), idx, None, False)
     assert rt.device_status() & 1 and not out[2].any()
     assert rt.device_status() == 0
+
+
+@pytest.mark.parametrize("n, bits, shape", [
+    (1, 4, "one"), (900, 4, "spread"), (1024, 16, "distinct"), (1500, 11, "spread"), (5000, 16, "distinct"),
+    (70000, 1, "spread"), (70000, 16, "two giants"), (70000, 12, "power"), (300000, 16, "power"),
+    (300000, 16, "two giants"), (1500000, 21, "distinct"), (1500000, 21, "power"), (9000, 0, "one")])
+def test_bucket_plan_of_the_device_equals_the_host_one(rt, n, bits, shape):
+    """An assignment's plan (statistics, lists and entries by kernels) against the plan the host cuts for the same
+    index: figures, degrees and every bit of a mean (the summation order is the plan's), over one row, rows
+    below, at and beyond a tile of rows, lengths beyond the histogram, and more than 2^20 buckets."""
+    gen = torch.Generator(device="cuda").manual_seed(n + bits)
+    if shape == "distinct":
+        codes = torch.randperm(n, device="cuda", generator=gen)
+    elif shape == "two giants":
+        codes = torch.randint(0, 2 ** bits, (n,), device="cuda", generator=gen)
+        codes[: n // 2] = 5
+        codes[n // 2: n - 3000] = 2 ** bits - 1
+    elif shape == "power":
+        codes = (torch.rand(n, device="cuda", generator=gen) ** 6 * 2 ** bits).long()
+    else:
+        codes = torch.randint(0, 2 ** bits, (n,), device="cuda", generator=gen) * (shape != "one")
+    codes = (codes % 2 ** bits).int()
+    workspace = rt.cluster_workspace(torch.empty(n, 1, device="cuda"), bits)
+    ids, counts, active = rt._assign_from_codes(codes, n, bits, workspace, codes.device)
+    mine, host = rt.index_plan(ids, active + 1), rt.SegmentPlan.from_index(ids, active + 1)
+    for name in ("rows", "nnz", "split", "long_rows", "chunks", "direct_units", "compact_rows", "source_rows",
+                 "degree_p50", "degree_p99", "degree_max"):
+        assert getattr(mine, name) == getattr(host, name), name
+    x = torch.randn(n, 12, device="cuda", generator=gen)
+    assert torch.equal(rt.cluster_mean(x, ids, counts, plan=mine), rt.cluster_mean(x, ids, counts, plan=host))
