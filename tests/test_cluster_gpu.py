@@ -216,6 +216,21 @@ def test_argument_errors_raise_runtime_error(rt):
     assert rt.device_status() == 0
 
 
+@pytest.mark.parametrize("groups", [1, 7, 255, 256, 257, 2049, 70001])
+def test_bias_gradient_sums(groups):
+    """Column sums of the group gradients around the row blocks of the two stages, against 64 bits: a sum is a
+    chain of at most 32 + 8 and then 35 + 8 additions here, each within half an ulp of the sum of magnitudes."""
+    from compressgnn_b200 import runtime as rt
+    gen = torch.Generator(device="cuda").manual_seed(groups)
+    index = torch.arange(groups, device="cuda")
+    for width in (1, 31, 33, 47, 128):
+        grad = torch.randn(groups, width, device="cuda", generator=gen)
+        d_reps, d_bias = rt.cluster_reconstruct_backward(grad, index, grad, groups, False, return_bias_grad=True)
+        assert torch.equal(d_reps, grad)
+        bound = 96 * 2.0 ** -24 * grad.double().abs().sum(0)
+        assert bool(((d_bias.double() - grad.double().sum(0)).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("n, bits, shape", [
     (1, 4, "one"), (900, 4, "spread"), (1024, 16, "distinct"), (1500, 11, "spread"), (5000, 16, "distinct"),
     (70000, 1, "spread"), (70000, 16, "two giants"), (70000, 12, "power"), (300000, 16, "power"),
