@@ -60,6 +60,37 @@ def test_spmm_widths(rt, dtype, width):
     assert_close_rel(got.cpu().numpy(), ref_acc, what=f"spmm accumulate width {width}")
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("dtype, widths", [(np.float32, (1, 2, 11, 12, 13, 27, 28, 29, 59, 60, 61, 123, 124, 125, 249, 602)),
+                                           (np.float64, (1, 6, 7, 13, 14, 15, 29, 30, 31, 61, 62, 63, 125, 126, 127, 253))])
+def test_rows_that_are_no_whole_vectors(rt, dtype, widths, shift):
+    """Around the edges of the column tiles, with both matrices starting ``shift`` elements past a 16-byte boundary
+    (so that widths of whole vectors take the same kernel), fresh and accumulated, and with what lies
+    around the source matrix not a number: nothing outside a row may enter its sum."""
+    def moved(a):
+        flat = torch.full((a.size + 2 * shift,), float("nan"), dtype=torch.from_numpy(a).dtype, device="cuda")
+        view = flat[shift:shift + a.size].view(a.shape)
+        view.copy_(torch.from_numpy(a))
+        return view
+
+    rng = np.random.default_rng(len(widths) + shift)
+    rows, src_rows = 300, 211
+    rowptr, col = random_csr(rng, rows, src_rows, 12, long_rows=[(7, 500), (123, 131), (299, 70)])
+    val = rng.standard_normal(col.size).astype(dtype)
+    args = cu(rowptr), cu(col), cu(val)
+    for width in widths:
+        mat = rng.standard_normal((src_rows, width)).astype(dtype)
+        mat[-1] = np.nan if shift else mat[-1]  # rows that are gathered from beside it stay finite
+        used = np.where(col == src_rows - 1, 0, col) if shift else col
+        src = moved(mat)
+        out = rt.spmm_func(args[0], cu(used), args[2], src, "rowbalance_rowcache", None)
+        assert_close_rel(out.cpu().numpy(), oracle.spmm(rowptr, used, val, mat), what=f"width {width} shift {shift}")
+        base = rng.standard_normal((rows, width)).astype(dtype)
+        got = rt.spmm_func(args[0], cu(used), args[2], src, "nnzbalance_parreduce", moved(base))
+        assert_close_rel(got.cpu().numpy(), oracle.spmm(rowptr, used, val, mat, out=base.copy()),
+                         what=f"accumulate, width {width} shift {shift}")
+
+
 def test_accuracy_against_fp64(rt):
     """The fp32 CUDA result is as close to the exact (fp64) product as the reference's own
     fp32 loop is: error no larger than twice the CPU oracle's, row by row in max norm."""
