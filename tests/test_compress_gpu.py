@@ -75,6 +75,18 @@ def test_web_graph_rows(rounds, frequency):
         assert expand(dv, de, node, n) == e[v[node]:v[node + 1]].tolist()
 
 
+def test_runs_of_the_left_to_right_step():
+    """Rows of one repeated symbol (every pair weighs the same, the whole row is one run), of two in turn, runs begun
+    behind a pair the first step took, and lengths around them, against the host's row-by-row walk."""
+    rng = np.random.default_rng(2)
+    rows = [[1] * k for k in range(1, 45)] + [[2, 3] * k for k in range(1, 20)] + [[4] * 3000]
+    rows += [[7, 8] * 2 + [1] * k + [7, 8] for k in range(12)]
+    rows += [rng.integers(0, 3, rng.integers(0, 40)).tolist() for _ in range(400)]
+    v, e = csr_of(rows)
+    for frequency in (3, 5, 40):
+        same(compress_graph_csr(v, e, frequency, backend='cuda'), compress_graph_csr(v, e, frequency, backend='cpu'))
+
+
 def test_argument_errors():
     v, e = csr_of([[0, 1], [1, 5]])
     with pytest.raises(RuntimeError):
