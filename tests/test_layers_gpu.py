@@ -427,3 +427,39 @@ def test_forward_mode_is_refused():
             Compressgnn_SPMM_Function.apply(data.edge_index, x)
         with pytest.raises(RuntimeError, match="forward-mode"):
             Compressgnn_Reconstruct()(reps, index)
+
+
+@pytest.mark.parametrize("width", [1, 16, 47, 130, 256])
+def test_chained_launches_of_a_pass(width):
+    """The launches of a pass overlap at their ends: whole passes against the same launches made one at a time, many
+    times over, with the stream busy before and after, and replayed from a captured graph."""
+    from compressgnn_b200 import runtime as rt
+    data = make_data(n=3000, width=width, max_depth=6)
+    data.to("cuda")
+    graph = data.edge_index
+    native, last = graph.propagation_plan().native, graph.propagation_plan().launches - 1
+    x = torch.randn(data.vertex_cnt, width, device="cuda")
+    rule = rt.empty_row_aligned(data.rule_cnt, x)
+    for backward in (False, True):
+        want = torch.empty_like(x)
+        for i in range(last + 1):
+            native.run(x, backward, want, rule, i, i)
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            native.run(x, backward)
+            side.synchronize()
+            recorded = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(recorded, stream=side):
+                replayed = native.run(x, backward)
+        torch.cuda.current_stream().wait_stream(side)
+        for _ in range(20):
+            y = x * 1.0  # a producer right before and a consumer right after the pass
+            got = native.run(y, backward)
+            y.zero_()
+            assert torch.equal(got, want)
+            replayed.zero_()
+            recorded.replay()
+            assert torch.equal(replayed, want)
+        del recorded
