@@ -737,8 +737,22 @@ __global__ void __launch_bounds__(CGNN_SEG_BULK_WARPS * 32) seg_bulk_kernel(cons
 #define CGNN_SEG_ASYNC_MAX_VECS 32   // widest row (in 16-byte vectors) handled as ONE tile by this engine
 #endif
 
-__device__ __forceinline__ void async_copy16(uint32_t dst_shared, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_shared), "l"(src) : "memory");
+template <int BYTES>
+__device__ __forceinline__ void async_copy(uint32_t dst_shared, const void *src) {
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_shared), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst_shared), "l"(src) : "memory");
+}
+template <typename V>
+__device__ __forceinline__ V shared_vec(uint32_t address) {
+    if constexpr (sizeof(V) == 16) {
+        float4 t;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(address));
+        return *reinterpret_cast<V *>(&t);
+    } else {
+        float2 t;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.x), "=f"(t.y) : "r"(address));
+        return *reinterpret_cast<V *>(&t);
+    }
 }
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // Steps (warp-wide copies per vector) of one stage: a stage never holds more than the 32 entries of a window.
@@ -760,19 +774,20 @@ __device__ __forceinline__ void async_wait() {
 template <typename T, int VW, int LPR, int VPL, bool PLAIN>
 __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
     using V = Vec<T, VW>;
-    static_assert(sizeof(T) * VW == 16, "cp.async staging moves 16-byte vectors");
+    constexpr int VB = (int)sizeof(T) * VW;   // bytes of a vector
+    static_assert(VB == 16 || VB == 8, "cp.async staging moves 16-byte or 8-byte vectors");
     static_assert(LPR == 32 || VPL == 1, "several vectors per lane only for full-warp rows");
     constexpr int G = 32 / LPR;               // entries per step (one warp-wide copy per vector)
     constexpr int K = async_steps(LPR), S = CGNN_SEG_ASYNC_S, RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     constexpr int KE = K * G;                 // entries per stage
     static_assert(32 % KE == 0, "a stage must not straddle two entry windows");
     constexpr int TILE = LPR * VPL * VW;      // columns of one tile
-    constexpr int SLOT = 32 * VPL * 16;       // bytes of one staged step
+    constexpr int SLOT = 32 * VPL * VB;       // bytes of one staged step
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(128) unsigned char async_smem[];
     const int lane = threadIdx.x;
     const int gl = lane & (LPR - 1), gk = lane / LPR;
-    const uint32_t ring = shared_addr(async_smem) + lane * 16;  // this lane's 16 bytes of slot 0, vector 0
+    const uint32_t ring = shared_addr(async_smem) + lane * VB;  // this lane's bytes of slot 0, vector 0
 
     chain_open(a);
     const int64_t unit = blockIdx.x;
@@ -852,7 +867,7 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
         const char *src = gbase + (int64_t)rj * row_bytes;  // one widening multiply-add
 #pragma unroll
         for (int p = 0; p < VPL; ++p)
-            if (colok[p]) async_copy16(slot + (uint32_t)(p * 512), src + p * 512);
+            if (colok[p]) async_copy<VB>(slot + (uint32_t)(p * 32 * VB), src + p * 32 * VB);
     };
     auto issue = [&](int b) {
         if (b < nb) {
@@ -909,11 +924,7 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 #pragma unroll
             for (int p = 0; p < VPL; ++p) {
                 if (colok[p]) {
-                    float4 t;
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                 : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w)
-                                 : "r"(stage + (uint32_t)(j * SLOT + p * 512)));
-                    x[j][p] = *reinterpret_cast<V *>(&t);
+                    x[j][p] = shared_vec<V>(stage + (uint32_t)(j * SLOT + p * 32 * VB));
                 }
             }
         }
@@ -998,48 +1009,44 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Rows that are no whole number of 16-byte vectors, or do not start on one (602 raw features, 47 class
-// scores): the same cp.async engine with one shift.  What bounded these rows in seg_kernel was instructions
-// and loads in flight -- one 4-byte load per element and entry.  Here a tile of a gathered row is copied by the
-// ALIGNED 16-byte vectors that cover it, wherever the row begins, LPR * NP of them; a tile is one vector
-// short of that (ragged_tile), so the cover always fits.  The last vector copies no byte past the tile's
-// end, and the first starts at most 15 bytes early, inside the aligned 16 bytes its first element lies in.  A lane
-// then reads elements gl, gl + LPR, ... (consecutive words across the lanes, no bank conflict) from the
-// row's offset into the cover, which it gets by shuffle from the lane that loaded the entry.  Lanes read
-// what other lanes copied, hence the two __syncwarp per stage.
-// Forward + backward of a propagation at 40,000 nodes x 602 columns: 539 -> 396 us.
+// Rows of fp32 that start on any 4-byte boundary (odd widths: 47 class scores, or a view that begins anywhere): the
+// same cp.async engine with one shift.  What bounded these rows in seg_kernel was instructions and loads in
+// flight -- one 4-byte load per element and entry.  Here a tile of a gathered row is copied by the ALIGNED
+// 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is one vector short of that
+// (ragged_tile), so the cover always fits.  The last vector copies no byte past the tile's end, and the first
+// starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then
+// reads elements gl, gl + LPR, ... (consecutive words across the lanes, no bank conflict) from the row's
+// offset into the cover, which it gets by shuffle from the lane that loaded the entry.  Lanes read what other lanes
+// copied, hence the two __syncwarp per stage.  Rows on 8-byte boundaries (even widths; any width in fp64)
+// take seg_async_kernel with 8-byte copies instead, which needs neither the shift nor the second lane.
+// Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 396 through the aligned cover, 320 with 8-byte
+// copies.  Segment sums of 7 columns (2,708 rows): 34 -> 10 us, of 47 (325 k rows): 116 -> 108.
 // ---------------------------------------------------------------------------------------
-template <typename T>
-__host__ __device__ constexpr int ragged_tile(int lpr, int np) {
-    return (lpr * np - 1) * (16 / (int)sizeof(T));
-}
+__host__ __device__ constexpr int ragged_tile(int lpr) { return (lpr - 1) * 4; }
 // 16 bytes into shared memory of which the first min(left, 16) are read, the others zero.
 __device__ __forceinline__ void async_copy16_upto(uint32_t dst_shared, const void *src, uintptr_t left) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_shared), "l"(src),
                  "r"((uint32_t)(left < 16 ? left : 16))
                  : "memory");
 }
-template <typename T>
-__device__ __forceinline__ T shared_load(uint32_t address) {
-    T t;
-    if constexpr (sizeof(T) == 4) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(address));
-    else asm volatile("ld.shared.f64 %0, [%1];" : "=d"(t) : "r"(address));
+__device__ __forceinline__ float shared_load(uint32_t address) {
+    float t;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(address));
     return t;
 }
 
-template <typename T, int LPR, int NP>
-__global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<T> a) {
+template <int LPR>
+__global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) {
+    using T = float;
     using V = Vec<T, 1>;
-    static_assert(LPR == 32 || NP == 1, "several vectors per lane only for full-warp rows");
     constexpr int VW = 1;
-    constexpr int NV = 16 / (int)sizeof(T);   // elements of a copied vector
-    constexpr int VPL = NV * NP;              // elements of a row per lane
+    constexpr int VPL = 4;                    // elements of a row per lane
     constexpr int G = 32 / LPR;               // entries per step (one warp-wide copy per vector)
     constexpr int K = async_steps(LPR), S = CGNN_SEG_ASYNC_S, RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     constexpr int KE = K * G;                 // entries per stage
     static_assert(32 % KE == 0, "a stage must not straddle two entry windows");
-    constexpr int TILE = ragged_tile<T>(LPR, NP);  // columns of one tile
-    constexpr int SLOT = 32 * NP * 16;        // bytes of one staged step
+    constexpr int TILE = ragged_tile(LPR);    // columns of one tile
+    constexpr int SLOT = 512;                 // bytes of one staged step
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(128) unsigned char async_smem[];
     const int lane = threadIdx.x;
@@ -1120,10 +1127,8 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<T> a) {
     auto copy_row = [&](uint32_t slot, int32_t rj) {
         const uintptr_t begin = reinterpret_cast<uintptr_t>(gbase + (int64_t)rj * row_bytes);
         const uintptr_t end = begin + tile_bytes;
-        uintptr_t at = (begin & ~(uintptr_t)15) + gl * 16;
-#pragma unroll
-        for (int p = 0; p < NP; ++p, at += 512)
-            if (at < end) async_copy16_upto(slot + (uint32_t)(p * 512), reinterpret_cast<const void *>(at), end - at);
+        const uintptr_t at = (begin & ~(uintptr_t)15) + gl * 16;
+        if (at < end) async_copy16_upto(slot, reinterpret_cast<const void *>(at), end - at);
     };
     auto issue = [&](int b) {
         if (b < nb) {
@@ -1187,7 +1192,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<T> a) {
                                  gl * (uint32_t)sizeof(T);
 #pragma unroll
             for (int p = 0; p < VPL; ++p)
-                if (colok[p]) x[j][p].v[0] = shared_load<T>(row + (uint32_t)(p * LPR * (int)sizeof(T)));
+                if (colok[p]) x[j][p].v[0] = shared_load(row + (uint32_t)(p * LPR * (int)sizeof(T)));
         }
         __syncwarp();  // every lane has read the stage
         if (cnt >= KE && ebase + KE <= row_end && ebase < row_end) {  // a full stage inside the current row
@@ -1272,7 +1277,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<T> a) {
 
 template <typename T, int VW, int LPR, int VPL, bool PLAIN>
 static int launch_async_as(const SegArgs<T> &a, cudaStream_t stream) {
-    constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 32 * VPL * 16;
+    constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 32 * VPL * VW * sizeof(T);
     constexpr int RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     static std::mutex mu;
     static uint64_t configured = 0;  // one bit per device: the kernel may use BYTES of shared memory
@@ -1301,32 +1306,40 @@ static int launch_async(const SegArgs<T> &a, cudaStream_t stream) {
                  : launch_async_as<T, VW, LPR, VPL, false>(a, stream);
 }
 
-template <typename T, int LPR, int NP>
-static int launch_ragged_as(const SegArgs<T> &a, cudaStream_t stream) {
-    constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 32 * NP * 16;
+template <int LPR>
+static int launch_ragged_as(const SegArgs<float> &a, cudaStream_t stream) {
+    constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 512;
     static_assert(BYTES <= 48 * 1024, "more than the default shared memory of a block");
     constexpr int RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     const int64_t gx = ceil_div(a.n_direct, RPU) + a.n_items;
-    const int64_t gy = ceil_div(a.width, (int64_t)ragged_tile<T>(LPR, NP));
+    const int64_t gy = ceil_div(a.width, (int64_t)ragged_tile(LPR));
     CGNN_REQUIRE(gx < (1ll << 31) && gy < 65536, "segment reduce: grid too large");
-    CGNN_CUDA(launch_chained(seg_ragged_kernel<T, LPR, NP>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
+    CGNN_CUDA(launch_chained(seg_ragged_kernel<LPR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
     return CGNN_OK;
 }
 
-// The fewest lanes whose tile holds the row; wider rows take tiles of 124 (fp32) or 126 (fp64) columns, never
-// more tiles than ticket_tiles() has words for.
+// Rows that are not 16-byte vectors throughout, without a mask row per entry: 8-byte copies where every row starts on an
+// 8-byte boundary, else the aligned cover.  The fewest lanes that hold the row; but with a mask row per group
+// the sums keep seg_kernel's order, that of one lane group, whatever the width: both mask modes of
+// reconstruct backward then give the same bits.  No more column tiles than ticket_tiles() has words for.
 template <typename T>
-static int launch_ragged(const SegArgs<T> &a, cudaStream_t stream) {
-    if (a.seg_mask == nullptr) {  // (with a mask row per group the sums keep seg_kernel's order, that of one lane group,
-                                  // whatever the width: both mask modes of reconstruct backward then give the same bits)
-        if (a.width <= ragged_tile<T>(4, 1)) return launch_ragged_as<T, 4, 1>(a, stream);
-        if (a.width <= ragged_tile<T>(8, 1)) return launch_ragged_as<T, 8, 1>(a, stream);
-        if (a.width <= ragged_tile<T>(16, 1)) return launch_ragged_as<T, 16, 1>(a, stream);
+static int launch_unaligned(const SegArgs<T> &a, bool aligned8, cudaStream_t stream) {
+    const bool one_group = a.seg_mask != nullptr;
+    constexpr int VW = 8 / (int)sizeof(T);
+    const int64_t vecs = a.width / VW;
+    if constexpr (sizeof(T) == 4) {
+        if (!aligned8) {
+            if (!one_group && a.width <= ragged_tile(4)) return launch_ragged_as<4>(a, stream);
+            if (!one_group && a.width <= ragged_tile(8)) return launch_ragged_as<8>(a, stream);
+            if (!one_group && a.width <= ragged_tile(16)) return launch_ragged_as<16>(a, stream);
+            return launch_ragged_as<32>(a, stream);
+        }
     }
-    if constexpr (sizeof(T) == 8) {
-        if (a.width > ragged_tile<T>(32, 1)) return launch_ragged_as<T, 32, 2>(a, stream);
-    }
-    return launch_ragged_as<T, 32, 1>(a, stream);
+    if (!one_group && vecs <= 4) return launch_async<T, VW, 4, 1>(a, stream);
+    if (!one_group && vecs <= 8) return launch_async<T, VW, 8, 1>(a, stream);
+    if (!one_group && vecs <= 16) return launch_async<T, VW, 16, 1>(a, stream);
+    if (vecs <= 32) return launch_async<T, VW, 32, 1>(a, stream);
+    return launch_async<T, VW, 32, 2>(a, stream);
 }
 
 template <typename T, int VW, int VPL, bool MASKED>
@@ -1466,7 +1479,11 @@ static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *s
         return launch_vw<T, VWMAX, false, false>(a, stream);
     }
     if (mask) return launch_vw<T, 1, true, false>(a, stream);
-    if (width * (int64_t)sizeof(T) < 0x7fffffffll) return launch_ragged<T>(a, stream);
+    if (width * (int64_t)sizeof(T) < 0x7fffffffll) {
+        auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
+        return launch_unaligned<T>(a, width * sizeof(T) % 8 == 0 && aligned8(src0) && aligned8(src1) && aligned8(seg_mask) &&
+                                          aligned8(out), stream);
+    }
     return launch_vw<T, 1, false, false>(a, stream);
 }
 
@@ -1495,7 +1512,8 @@ static int run(const cgnn_plan *p, int dtype, int64_t width, const void *val, co
 // ---------------------------------------------------------------------------------------
 // Column sums of a small [rows, width] matrix in two fixed-order stages (bias gradient): blocks of COLSUM_ROWS
 // rows, then the blocks' sums.  What bounds them is the length of the dependent chain, not bytes, so a block's
-// rows are shared among its warps and several loads are in flight: 36 us a call were two launches of 11 and 25 us, now 5 us each.
+// rows are shared among its warps and several loads are in flight: 36 us a call were two launches of 11 and 25 us, now 5 us
+// each.
 // ---------------------------------------------------------------------------------------
 constexpr int COLSUM_ROWS = 256;
 
