@@ -25,6 +25,8 @@
 #include <vector>
 #include <cub/cub.cuh>
 #include <cuda.h>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "cgnn_plan.h"
 
@@ -591,14 +593,27 @@ struct AssignLayout {
     size_t total;
 };
 
+// 1 where a bucket begins in the sorted codes.  The scan over these numbers the buckets; the flag is two cached reads,
+// so nothing is stored for it.  (Codes count modulo 2^bits, the bits the sort looks at: mask = 2^bits - 1.)
+struct HeadFlag {
+    const int32_t *sorted;
+    int32_t mask;
+    __host__ __device__ int32_t operator()(int32_t i) const {
+        return i == 0 || ((sorted[i] ^ sorted[i - 1]) & mask) != 0 ? 1 : 0;
+    }
+};
+using HeadIterator = thrust::transform_iterator<HeadFlag, thrust::counting_iterator<int32_t>, int32_t, int32_t>;
+
 static size_t cub_temp_bytes(int64_t n) {
     size_t sort_bytes = 0, scan_bytes = 0;
     cub::DoubleBuffer<int32_t> k(nullptr, nullptr), v(nullptr, nullptr);
     const int num = (int)std::max<int64_t>(n, 1);
     cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, k, v, num, 0, 32);
-    cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, (const int32_t *)nullptr, (int32_t *)nullptr, num);
+    size_t head_bytes = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, head_bytes, HeadIterator(thrust::counting_iterator<int32_t>(0), HeadFlag{nullptr, 0}),
+                                  (int32_t *)nullptr, num);
     cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const int32_t *)nullptr, (int32_t *)nullptr, num + 2);
-    return align_up(std::max(sort_bytes, scan_bytes) + 256, 256);
+    return align_up(std::max({sort_bytes, head_bytes, scan_bytes}) + 256, 256);
 }
 
 static AssignLayout assign_layout(void *base, int64_t n) {
@@ -618,31 +633,43 @@ static AssignLayout assign_layout(void *base, int64_t n) {
     return L;
 }
 
-__global__ void iota_kernel(int32_t *v, int64_t n) {
+// Row numbers for the sort, and with `codes` a copy of them (the sort consumes its keys).
+__global__ void sort_input_kernel(const int32_t *codes, int32_t *keys, int32_t *v, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)blockDim.x * gridDim.x)
+         i += (int64_t)blockDim.x * gridDim.x) {
         v[i] = (int32_t)i;
+        if (codes) keys[i] = codes[i];
+    }
 }
 
-__global__ void head_flags_kernel(const int32_t *sorted, int32_t *flags, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)blockDim.x * gridDim.x)
-        flags[i] = (i == 0 || sorted[i] != sorted[i - 1]) ? 1 : 0;
-}
-
-__global__ void scatter_ids_kernel(const int32_t *perm, const int32_t *cid, const int32_t *flags,
-                                   int64_t n, int64_t *ids, int32_t *segstart, int32_t *active) {
+// Segment starts, bucket count and what turns a row into its id: with `table` (2^bits words), the id of each code, from
+// which ids_from_codes_kernel writes the ids in row order; without, the ids themselves, scattered by the
+// permutation.  The table is taken when it has no more words than there are rows (it then fits the unused sort
+// buffer): 2.45 M rows, 16 bits, flags and ids were
+// 34 us of kernels and are 22; with the row numbers and the copy of the codes in one kernel a refresh went
+// 475 -> 453 us.
+__global__ void bucket_heads_kernel(const int32_t *sorted, const int32_t *perm, const int32_t *cid, int64_t n, int64_t *ids,
+                                    int32_t *table, int32_t mask, int32_t *segstart, int32_t *active) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)blockDim.x * gridDim.x) {
         const int32_t c = cid[i];
-        ids[perm[i]] = c;
-        if (flags[i]) segstart[c] = (int32_t)i;
+        if (!table) ids[perm[i]] = c;
+        if (i == 0 || cid[i - 1] != c) {
+            segstart[c] = (int32_t)i;
+            if (table) table[sorted[i] & mask] = c;
+        }
         if (i == 0) segstart[0] = 0;
         if (i == n - 1) {
             segstart[c + 1] = (int32_t)n;
             *active = c;
         }
     }
+}
+
+__global__ void ids_from_codes_kernel(const int32_t *codes, const int32_t *table, int32_t mask, int64_t n, int64_t *ids) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)blockDim.x * gridDim.x)
+        ids[i] = table[codes[i] & mask];
 }
 
 __global__ void counts_kernel(const int32_t *segstart, int64_t active, int32_t *counts) {
@@ -699,11 +726,11 @@ static HostSegments &host_segments() {
 
 static unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), 148 * 16)); }
 
-// Sort (key,row) pairs by the low `bits` bits of the key; leaves sorted keys in keys_out and
-// the permutation in vals[0].
-static int sort_pairs(AssignLayout &L, int64_t n, int bits, int32_t **sorted_keys,
+// Sort (key,row) pairs by the low `bits` bits of the key (`codes`, or what is already in keys[0]); leaves sorted
+// keys in keys_out and the permutation in vals[0].
+static int sort_pairs(AssignLayout &L, const int32_t *codes, int64_t n, int bits, int32_t **sorted_keys,
                       cudaStream_t stream) {
-    iota_kernel<<<grid_for(n), 256, 0, stream>>>(L.vals[0], n);
+    sort_input_kernel<<<grid_for(n), 256, 0, stream>>>(codes, L.keys[0], L.vals[0], n);
     CGNN_LAUNCH_CHECK();
     if (bits == 0) {
         *sorted_keys = L.keys[0];
@@ -776,19 +803,21 @@ int cgnn_cluster_assign(const int32_t *codes, int64_t n, int bits, void *workspa
     AssignLayout L = assign_layout(workspace, n);
     CGNN_REQUIRE(workspace_bytes >= L.total, "cluster_assign: workspace of %zu bytes needed, %zu given",
                  L.total, workspace_bytes);
-    CGNN_CUDA(cudaMemcpyAsync(L.keys[0], codes, sizeof(int32_t) * (size_t)n,
-                              cudaMemcpyDeviceToDevice, stream));
     int32_t *sorted = nullptr;
-    int rc = sort_pairs(L, n, bits, &sorted, stream);
+    int rc = sort_pairs(L, codes, n, bits, &sorted, stream);
     if (rc != CGNN_OK) return rc;
-    int32_t *flags = sorted == L.keys[0] ? L.keys[1] : L.keys[0];
-    head_flags_kernel<<<grid_for(n), 256, 0, stream>>>(sorted, flags, n);
-    CGNN_LAUNCH_CHECK();
+    const int32_t mask = (int32_t)(((int64_t)1 << bits) - 1);
+    int32_t *table = ((int64_t)1 << bits) > n ? nullptr : sorted == L.keys[0] ? L.keys[1] : L.keys[0];
     size_t bytes = L.temp_bytes;
-    CGNN_CUDA(cub::DeviceScan::InclusiveSum(L.temp, bytes, flags, L.cid, (int)n, stream));
-    scatter_ids_kernel<<<grid_for(n), 256, 0, stream>>>(L.vals[0], L.cid, flags, n, ids, L.segstart,
-                                                        L.active);
+    CGNN_CUDA(cub::DeviceScan::InclusiveSum(L.temp, bytes, HeadIterator(thrust::counting_iterator<int32_t>(0), HeadFlag{sorted, mask}),
+                                            L.cid, (int)n, stream));
+    bucket_heads_kernel<<<grid_for(n), 256, 0, stream>>>(sorted, L.vals[0], L.cid, n, ids, table, mask, L.segstart,
+                                                         L.active);
     CGNN_LAUNCH_CHECK();
+    if (table) {
+        ids_from_codes_kernel<<<grid_for(n), 256, 0, stream>>>(codes, table, mask, n, ids);
+        CGNN_LAUNCH_CHECK();
+    }
     // One synchronisation fetches `active`.  With it comes what the export step needs to build the
     // bucket plan without another round trip: when there are at most 2^22 buckets (PLAN_DEVICE_MAX_ROWS:
     // the usual bit counts), the row statistics of the plan, taken on the device and
@@ -897,7 +926,7 @@ int cgnn_plan_create_from_index(cgnn_plan **plan_out, const int64_t *index, int6
             int bits = 1;
             while (bits < 31 && ((int64_t)1 << bits) < groups) ++bits;
             int32_t *sorted = nullptr;
-            rc = sort_pairs(L, n, bits, &sorted, stream);
+            rc = sort_pairs(L, nullptr, n, bits, &sorted, stream);
             if (rc != CGNN_OK) break;
         }
         size_t bytes = L.temp_bytes;
