@@ -259,3 +259,29 @@ def test_bucket_plan_of_the_device_equals_the_host_one(rt, n, bits, shape):
         assert getattr(mine, name) == getattr(host, name), name
     x = torch.randn(n, 12, device="cuda", generator=gen)
     assert torch.equal(rt.cluster_mean(x, ids, counts, plan=mine), rt.cluster_mean(x, ids, counts, plan=host))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_expanded_rows_of_no_whole_vectors(rt, dtype):
+    """The row-block form of the reconstruction: widths whose vectors cross rows at every offset, on both sides of the
+    256 positions a block holds, row counts with every remainder; bit for bit the oracle's, dropped and kept
+    elements those of the whole-vector kernels (a mask is a function of the element's position)."""
+    rng = np.random.default_rng(11)
+    for width in (5, 6, 7, 9, 47, 127, 129, 254, 255, 257, 258, 602):
+        for n in (1, 2, 3, 5, 8, 1026, 4099):
+            idx = rng.integers(0, 9, n)
+            reps, bias = rng.standard_normal((9, width)).astype(dtype), rng.standard_normal(width).astype(dtype)
+            for relu in (False, True):
+                got = rt.cluster_reconstruct(cu(reps), cu(idx), cu(bias), relu)
+                np.testing.assert_array_equal(got.cpu().numpy(), oracle.reconstruct(reps, idx, bias, relu))
+            dropped = rt.cluster_reconstruct(cu(reps), cu(idx), cu(bias), True, 0.4, 77).flatten()
+            # the same element positions through rows of one 16-byte vector
+            flat = torch.nn.functional.pad(got.flatten(), (0, -got.numel() % 4)).view(-1, 4)
+            mask = rt.cluster_reconstruct(torch.ones_like(flat), torch.arange(flat.size(0), device="cuda"), None, True, 0.4, 77)
+            want = got.flatten() * (mask.flatten()[:got.numel()] != 0) * dtype(1.0 / 0.6)
+            np.testing.assert_allclose(dropped.cpu().numpy(), want.cpu().numpy(), rtol=1e-6)
+    bad = torch.tensor([0, 9, 2, -1, 3], device="cuda")
+    out = rt.cluster_reconstruct(cu(reps), bad, None, False)
+    assert not out[1].any() and not out[3].any() and torch.equal(out[4], cu(reps)[3])
+    with pytest.raises(RuntimeError):
+        rt.raise_on_device_status()
