@@ -59,6 +59,8 @@ SIGNATURES = {
                                                   ctypes.c_double, ctypes.c_uint64, _c_ptr, _c_ptr]),
     "cgnn_cluster_reconstruct_backward": (_c_int, [_c_ptr, _c_int, _c_i64, _c_ptr, _c_ptr, _c_int,
                                                    _c_ptr, _c_ptr, _c_ptr, _c_size, _c_ptr]),
+    "cgnn_matmul_tn_scratch_bytes": (_c_size, [_c_i64, _c_i64, _c_i64]),
+    "cgnn_matmul_tn": (_c_int, [_c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_size, _c_ptr]),
     "cgnn_sample_seed": (_c_int, [_c_ptr, _c_i64, _c_i64, _c_ptr, _c_ptr]),
     "cgnn_sample_count": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr]),
     "cgnn_sample_pick": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr, ctypes.c_uint32,

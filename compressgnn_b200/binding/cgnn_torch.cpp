@@ -309,6 +309,23 @@ std::pair<Tensor, Tensor> reconstruct_backward(const Tensor &grad, const Tensor 
     return {out, bias};
 }
 
+// a^T b for tall a [K, M] and b [K, N]: the weight gradient over the representatives.  The package's kernel splits K
+// over the GPU; it takes fp32 at full precision with up to a GPU of output tiles (64 x 128), beyond which the
+// library's tiles fill the GPU without a split, and leaves a caller who allowed TF32 products to the library.  (128 x 256 over
+// 64 k rows: 158 us there, 90 here; beyond 148 tiles neither side is measured and the library stays.)
+Tensor matmul_tn(const Tensor &a, const Tensor &b) {
+    const int64_t K = a.size(0), M = a.size(1), N = b.size(1);
+    const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
+    if (a.scalar_type() != at::kFloat || tiles > 148 || tiles == 0 || at::globalContext().allowTF32CuBLAS())
+        return at::mm(a.t(), b);
+    Tensor out = at::empty({M, N}, a.options());
+    const size_t bytes = cgnn_matmul_tn_scratch_bytes(K, M, N);
+    const Tensor scratch = at::empty({(int64_t)bytes}, a.options().dtype(at::kByte));
+    check(cgnn_matmul_tn(K, M, N, static_cast<const float *>(data(a)), static_cast<const float *>(data(b)),
+                         static_cast<float *>(data(out)), data(scratch), bytes, current_stream(a)));
+    return out;
+}
+
 // A fresh 63-bit key from torch's host generator (follows torch.manual_seed; no device synchronisation):
 // the draw of torch.randint(0, 2**63 - 1, (1,)).
 uint64_t dropout_key() {
@@ -507,7 +524,7 @@ struct TransformBackward : public Node {
                 r.first.mul_(1.0 / (1.0 - p));
                 r.second.mul_(1.0 / (1.0 - p));
             }
-            if (task_should_compute_output(1)) dw = at::mm(r.first.t(), reps);
+            if (task_should_compute_output(1)) dw = matmul_tn(r.first, reps);
             if (task_should_compute_output(0))
                 dx = mean_backward(at::mm(r.first, weight_.unpack()), index_.unpack(), counts_.unpack());
             if (task_should_compute_output(2)) db = r.second;
@@ -603,4 +620,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("reconstruct", &reconstruct_autograd, nogil());
     m.def("transform", &transform_autograd, nogil());
     m.def("assign", &assign, nogil());
+    m.def("matmul_tn", [](const Tensor &a, const Tensor &b) {
+        TORCH_CHECK(a.is_cuda() && a.device() == b.device() && a.scalar_type() == b.scalar_type() && a.dim() == 2 &&
+                        b.dim() == 2 && a.size(0) == b.size(0) && a.is_contiguous() && b.is_contiguous(),
+                    "Expected contiguous CUDA matrices with equal row counts");
+        const c10::cuda::OptionalCUDAGuard guard(a.device());
+        at::NoGradGuard no_grad;
+        return matmul_tn(a, b);
+    }, nogil());
 }

@@ -281,6 +281,14 @@ int cgnn_compressed_copy(const cgnn_compressed *c, int32_t *vlist_out, int32_t *
 void cgnn_compressed_destroy(cgnn_compressed *c);
 
 /* ---------------------------------------------------------------------------------------
+ * out[M, N] = a^T b for row-major fp32 a [K, M] and b [K, N] with K much larger than M and N (the weight
+ * gradient of a layer's Linear over its representatives).  K is split over the GPU; the partial products go
+ * to `scratch` (cgnn_matmul_tn_scratch_bytes, 0 when there is one split) and are added in a fixed order. */
+size_t cgnn_matmul_tn_scratch_bytes(int64_t K, int64_t M, int64_t N);
+int cgnn_matmul_tn(int64_t K, int64_t M, int64_t N, const float *a, const float *b, float *out,
+                   void *scratch, size_t scratch_bytes, cgnn_stream_t stream);
+
+/* ---------------------------------------------------------------------------------------
  * Neighbour sampling on the compressed graph, one hop at a time.
  * ref: neighbor_sample_sim_impl, src/sample/csrc/neighbor_sample.h:27-131 (a host function there, bound
  * as compressgnn_sample.neighbor_sample_cg_sim); get_neighbor / get_neighbor_list,

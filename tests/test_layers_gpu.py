@@ -429,6 +429,26 @@ def test_forward_mode_is_refused():
             Compressgnn_Reconstruct()(reps, index)
 
 
+@pytest.mark.parametrize("m, n", [(1, 1), (7, 64), (47, 128), (64, 128), (65, 129), (128, 256), (130, 36), (256, 602)])
+def test_weight_gradient_product(m, n):
+    """a^T b around the tiles, the stages and the splits of K, against 64 bits: a sum is a chain of at most
+    ceil(K / splits) fused multiply-adds and the chain over the splits, each within half an ulp of the magnitudes."""
+    from compressgnn_b200 import runtime as rt
+    assert not torch.backends.cuda.matmul.allow_tf32
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    for k in (1, 15, 16, 17, 63, 64, 127, 129, 2708, 30011):
+        a = torch.randn(k, m, device="cuda", generator=gen)
+        b = torch.randn(k, n, device="cuda", generator=gen)
+        got = rt.ops().matmul_tn(a, b)
+        exact = a.double().t() @ b.double()
+        splits = max(1, min(592 // (-(-m // 64) * -(-n // 128)), k // 64))
+        chain = -(-k // splits) + 16 + splits // 8 + 9
+        bound = chain * 2.0 ** -24 * (a.double().abs().t() @ b.double().abs())
+        assert bool(((got.double() - exact).abs() <= bound + 1e-30).all()), k
+        assert torch.equal(got, rt.ops().matmul_tn(a, b))
+    assert not rt.ops().matmul_tn(a[:0], b[:0]).any()
+
+
 @pytest.mark.parametrize("width", [1, 16, 47, 130, 256])
 def test_chained_launches_of_a_pass(width):
     """The launches of a pass overlap at their ends: whole passes against the same launches made one at a time, many
