@@ -74,6 +74,8 @@ SIGNATURES = {
     "cgnn_sample_hops_result": (_c_int, [_c_ptr, _c_i64, _c_int, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
                                          _c_ptr, _c_ptr, _c_ptr]),
     "cgnn_compress_csr_batch": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_int, _c_int, _c_ptr, _c_ptr]),
+    "cgnn_compress_workspace_bytes": (_c_size, [_c_i64, _c_i64, _c_int]),
+    "cgnn_compress_csr_batch_in": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_int, _c_int, _c_ptr, _c_size, _c_ptr, _c_ptr]),
     "cgnn_compressed_info": (_c_int, [_c_ptr, _c_ptr]),
     "cgnn_compressed_copy": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr]),
     "cgnn_compressed_destroy": (None, [_c_ptr]),

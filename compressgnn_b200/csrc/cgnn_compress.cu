@@ -19,14 +19,15 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
-#include <vector>
+#include <memory>
 
 #include "cgnn_common.cuh"
 
 struct cgnn_compressed {
-    int32_t *vlist = nullptr;  // device, rows + 1
-    int32_t *elist = nullptr;  // device, entries
+    const int32_t *vlist = nullptr;  // device, rows + 1
+    const int32_t *elist = nullptr;  // device, entries
     int64_t n = 0, rules = 0, entries = 0;
+    void *owned = nullptr;           // device block the arrays lie in, unless that is the caller's workspace
 };
 
 namespace cgnn {
@@ -40,41 +41,62 @@ static inline unsigned blocks_for(int64_t count) {
 #define GRID_STRIDE(i, count) \
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (count); i += (int64_t)blockDim.x * gridDim.x)
 
-// Device buffers of one compression: the work arrays are carved out of one allocation (sized by a dry
-// pass of the same requests), the rule pairs of each round are allocated as the rounds find them.
+// Device buffers of one compression, result included, carved out of one block (sized by a dry pass of the same requests):
+// the caller's workspace, or an allocation of this call.  What a call without a workspace pays for is
+// not the kernels but the driver mapping and unmapping 250 MB.  325 k-node graph, host arrays in
+// and out: 8.4 ms with an allocation per call and per round, 5.9 ms with a workspace.
 struct Arena {
-    std::vector<void *> held;
     char *block = nullptr;
-    size_t used = 0, capacity = 0;
+    size_t used = 0;
     bool sizing = true;
-    ~Arena() {
-        for (void *p : held) cudaFree(p);
-    }
     template <typename T>
     void carve(T **p, size_t count) {
         const size_t bytes = align_up(std::max<size_t>(count, 1) * sizeof(T), 256);
         *p = sizing ? nullptr : reinterpret_cast<T *>(block + used);
         used += bytes;
     }
-    cudaError_t commit() {  // end of the dry pass
-        capacity = used;
-        used = 0;
-        sizing = false;
-        void *raw = nullptr;
-        cudaError_t e = cudaMalloc(&raw, std::max<size_t>(capacity, 256));
-        if (e == cudaSuccess) held.push_back(raw);
-        block = reinterpret_cast<char *>(raw);
-        return e;
-    }
-    template <typename T>
-    cudaError_t get(T **p, size_t count) {
-        void *raw = nullptr;
-        cudaError_t e = cudaMalloc(&raw, std::max<size_t>(count, 1) * sizeof(T));
-        if (e == cudaSuccess) held.push_back(raw);
-        *p = reinterpret_cast<T *>(raw);
-        return e;
-    }
 };
+
+struct Buffers {
+    int32_t *rowptr[2], *sym[2], *row_of[2], *keep, *value, *slot, *run_count, *flag, *cand_count, *uses, *remap, *rule_pairs;
+    int32_t *final_vlist;
+    uint64_t *key, *key_sorted, *run_key, *cand_key, *weight;
+    uint8_t *take, *temp;
+    int32_t *scalars;  // 0: bad input, 1: runs, 2: candidates, 3: new total, 4: rules kept
+    size_t cand_cap, temp_bytes;
+};
+
+// Requests the buffers of a compression of `cap` symbols (rows only shrink); returns the bytes they take.
+static size_t carve_buffers(Arena &arena, Buffers &b, int64_t n, int64_t cap, int min_frequency) {
+    for (int i = 0; i < 2; ++i) {
+        arena.carve(&b.rowptr[i], (size_t)n + 1);
+        arena.carve(&b.sym[i], (size_t)cap);
+        arena.carve(&b.row_of[i], (size_t)cap);
+    }
+    b.cand_cap = (size_t)(cap / min_frequency + 1);  // at most one candidate per min_frequency pairs
+    for (int32_t **p : {&b.keep, &b.value, &b.slot, &b.run_count, &b.flag}) arena.carve(p, (size_t)cap);
+    for (uint64_t **p : {&b.key, &b.key_sorted, &b.run_key, &b.weight}) arena.carve(p, (size_t)cap);
+    arena.carve(&b.take, (size_t)cap);
+    arena.carve(&b.scalars, 8);
+    arena.carve(&b.cand_key, b.cand_cap);
+    for (int32_t **p : {&b.cand_count, &b.uses, &b.remap}) arena.carve(p, b.cand_cap);
+    // a kept rule is used, and every use takes a symbol away: at most `cap` rules, and symbols + rules <= cap
+    arena.carve(&b.rule_pairs, 2 * (size_t)cap);
+    arena.carve(&b.final_vlist, (size_t)n + (size_t)cap + 1);
+    size_t need = 0;
+    b.temp_bytes = 0;
+    const int cap32 = (int)std::max<int64_t>(cap, 1);
+    uint64_t *k = nullptr;
+    int32_t *w = nullptr;
+    cub::DeviceRadixSort::SortKeys(nullptr, need, k, k, cap32, 0, 64);
+    b.temp_bytes = std::max(b.temp_bytes, need);
+    cub::DeviceRunLengthEncode::Encode(nullptr, need, k, k, w, w, cap32);
+    b.temp_bytes = std::max(b.temp_bytes, need);
+    cub::DeviceScan::ExclusiveSum(nullptr, need, w, w, cap32);
+    b.temp_bytes = std::max(b.temp_bytes, need);
+    arena.carve(&b.temp, b.temp_bytes);
+    return arena.used;
+}
 
 __global__ void load_rows_kernel(const int64_t *vlist, const int64_t *elist, int64_t n, int64_t total, int32_t *rowptr,
                                  int32_t *sym, int *bad) {
@@ -164,8 +186,8 @@ __global__ void take_heavier_kernel(const uint64_t *key, const uint64_t *weight,
 // pair of the first step behind it.  Along a run of open positions the taken ones simply alternate, starting with
 // the first unless the pair before the run was taken; everything between two runs is settled already.  So the
 // thread of a run's first position walks the run (rows of the web graph: a few symbols), where one thread per
-// row used to walk whole rows, the longest of 10,000 symbols.  Five rounds on the 325 k-node graph took
-// 649 us that way.
+// row used to walk whole rows, the longest of 10,000 symbols.  Five rounds on the 325 k-node graph:
+// 649 -> 90 us.
 // take[]: bit 0 the first step, bit 1 this one; a run's bytes are written by its own thread and other threads
 // look at bit 0 only.
 __global__ void take_greedy_kernel(const uint64_t *key, const uint64_t *weight, int64_t total, uint8_t *take) {
@@ -266,8 +288,20 @@ using namespace cgnn;
 
 extern "C" {
 
+size_t cgnn_compress_workspace_bytes(int64_t n, int64_t entries, int min_frequency) {
+    if (n < 0 || entries < 0 || min_frequency < 3 || n + entries >= INT32_MAX) return 0;
+    Arena arena;
+    Buffers b;
+    return carve_buffers(arena, b, n, entries, min_frequency);
+}
+
 int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t n, int rounds, int min_frequency,
-                            cgnn_compressed **out, cgnn_stream_t stream_) {
+                            cgnn_compressed **out, cgnn_stream_t stream) {
+    return cgnn_compress_csr_batch_in(vlist, elist, n, rounds, min_frequency, nullptr, 0, out, stream);
+}
+
+int cgnn_compress_csr_batch_in(const int64_t *vlist, const int64_t *elist, int64_t n, int rounds, int min_frequency,
+                               void *workspace, size_t workspace_bytes, cgnn_compressed **out, cgnn_stream_t stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     CGNN_REQUIRE(out != nullptr, "compress_csr_batch: null result pointer");
     *out = nullptr;
@@ -282,46 +316,29 @@ int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t 
     const int64_t cap = total64;  // rows only shrink
 
     Arena arena;
-    int32_t *rowptr[2], *sym[2], *row_of[2], *keep, *value, *slot, *run_count, *flag, *cand_count, *uses, *remap;
-    uint64_t *key, *key_sorted, *run_key, *cand_key, *weight;
-    uint8_t *take, *temp;
-    int32_t *scalars;  // 0: bad input, 1: runs, 2: candidates, 3: new total, 4: rules kept
-    // candidate arrays: at most one candidate per min_frequency pairs
-    const size_t cand_cap = (size_t)(cap / min_frequency + 1);
-    size_t temp_bytes = 0, need = 0;
-    const int cap32 = (int)std::max<int64_t>(cap, 1);
-    for (int pass = 0; pass < 2; ++pass) {  // 0: sizes only, 1: pointers into the one allocation
-        for (int b = 0; b < 2; ++b) {
-            arena.carve(&rowptr[b], (size_t)n + 1);
-            arena.carve(&sym[b], (size_t)cap);
-            arena.carve(&row_of[b], (size_t)cap);
-        }
-        arena.carve(&keep, (size_t)cap);
-        arena.carve(&value, (size_t)cap);
-        arena.carve(&slot, (size_t)cap);
-        arena.carve(&run_count, (size_t)cap);
-        arena.carve(&flag, (size_t)cap);
-        arena.carve(&key, (size_t)cap);
-        arena.carve(&key_sorted, (size_t)cap);
-        arena.carve(&run_key, (size_t)cap);
-        arena.carve(&weight, (size_t)cap);
-        arena.carve(&take, (size_t)cap);
-        arena.carve(&scalars, 8);
-        arena.carve(&cand_key, cand_cap);
-        arena.carve(&cand_count, cand_cap);
-        arena.carve(&uses, cand_cap);
-        arena.carve(&remap, cand_cap);
-        if (pass == 0) {
-            cub::DeviceRadixSort::SortKeys(nullptr, need, key, key_sorted, cap32, 0, 64, stream);
-            temp_bytes = std::max(temp_bytes, need);
-            cub::DeviceRunLengthEncode::Encode(nullptr, need, key_sorted, run_key, run_count, scalars + 1, cap32, stream);
-            temp_bytes = std::max(temp_bytes, need);
-            cub::DeviceScan::ExclusiveSum(nullptr, need, flag, slot, cap32, stream);
-            temp_bytes = std::max(temp_bytes, need);
-        }
-        arena.carve(&temp, temp_bytes);
-        if (pass == 0) CGNN_CUDA(arena.commit());
+    Buffers buf;
+    const size_t bytes = carve_buffers(arena, buf, n, cap, min_frequency);
+    std::unique_ptr<cgnn_compressed, decltype(&cgnn_compressed_destroy)> res(new cgnn_compressed(), cgnn_compressed_destroy);
+    if (workspace == nullptr) {
+        CGNN_CUDA(cudaMalloc(&res->owned, bytes));
+        workspace = res->owned;
+    } else {
+        CGNN_REQUIRE(workspace_bytes >= bytes && (reinterpret_cast<uintptr_t>(workspace) & 255) == 0,
+                     "compress_csr_batch: workspace of %zu bytes on a 256-byte boundary needed, %zu given", bytes,
+                     workspace_bytes);
     }
+    arena.block = static_cast<char *>(workspace);
+    arena.used = 0;
+    arena.sizing = false;
+    carve_buffers(arena, buf, n, cap, min_frequency);
+    int32_t **rowptr = buf.rowptr, **sym = buf.sym, **row_of = buf.row_of, *keep = buf.keep, *value = buf.value;
+    int32_t *slot = buf.slot, *run_count = buf.run_count, *flag = buf.flag, *cand_count = buf.cand_count, *uses = buf.uses;
+    int32_t *remap = buf.remap, *scalars = buf.scalars;
+    uint64_t *key = buf.key, *key_sorted = buf.key_sorted, *run_key = buf.run_key, *cand_key = buf.cand_key;
+    uint64_t *weight = buf.weight;
+    uint8_t *take = buf.take, *temp = buf.temp;
+    const size_t cand_cap = buf.cand_cap, temp_bytes = buf.temp_bytes;
+    size_t need = 0;
     CGNN_CUDA(cudaMemsetAsync(scalars, 0, 8 * sizeof(int32_t), stream));
     int32_t *used = flag, *rank = slot;  // free again once the rows are compacted
 
@@ -337,7 +354,6 @@ int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t 
     row_of_kernel<<<blocks_for(n), THREADS, 0, stream>>>(rowptr[0], n, row_of[0]);
     CGNN_LAUNCH_CHECK();
 
-    std::vector<std::pair<int32_t *, int32_t>> rule_blocks;  // (device pairs, count) of every round
     int64_t total = cap, rules = 0;
     int cur = 0;
     for (int round = 0; round < rounds && total > 1; ++round) {
@@ -394,10 +410,8 @@ int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t 
         CGNN_LAUNCH_CHECK();
         need = temp_bytes;
         CGNN_CUDA(cub::DeviceScan::ExclusiveSum(temp, need, used, rank, candidates, stream));
-        int32_t *pairs = nullptr;
-        CGNN_CUDA(arena.get(&pairs, 2 * (size_t)candidates));
         keep_rules_kernel<<<blocks_for(candidates), THREADS, 0, stream>>>(cand_key, used, rank, candidates, shift, base,
-                                                                          remap, pairs, scalars + 4);
+                                                                          remap, buf.rule_pairs + 2 * rules, scalars + 4);
         CGNN_LAUNCH_CHECK();
         CGNN_CUDA(cudaMemcpyAsync(host_scalars, scalars, sizeof(host_scalars), cudaMemcpyDeviceToHost, stream));
         CGNN_CUDA(cudaStreamSynchronize(stream));
@@ -407,41 +421,42 @@ int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t 
             remap_kernel<<<blocks_for(total), THREADS, 0, stream>>>(sym[cur], total, base, remap);
             CGNN_LAUNCH_CHECK();
         }
-        rule_blocks.emplace_back(pairs, kept);
         rules += kept;
     }
 
     CGNN_REQUIRE(total + 2 * rules < INT32_MAX, "compressed arrays exceed int32 capacity");
-    auto *res = new cgnn_compressed();
     res->n = n;
     res->rules = rules;
     res->entries = total + 2 * rules;
-    cudaError_t e = cudaMalloc(&res->vlist, (size_t)(n + rules + 1) * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&res->elist, std::max<size_t>((size_t)res->entries, 1) * sizeof(int32_t));
-    if (e != cudaSuccess) {
-        cgnn_compressed_destroy(res);
-        set_error("compress_csr_batch: cudaMalloc of the result failed: %s", cudaGetErrorString(e));
-        return CGNN_ERR_CUDA;
-    }
     final_vlist_kernel<<<blocks_for(n + rules + 1), THREADS, 0, stream>>>(rowptr[cur], n, rules, (int32_t)total,
-                                                                          res->vlist);
-    cudaError_t launch = cudaGetLastError();
-    if (launch == cudaSuccess && total > 0)
-        launch = cudaMemcpyAsync(res->elist, sym[cur], (size_t)total * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream);
-    int64_t at = total;
-    for (const auto &block : rule_blocks) {
-        if (launch == cudaSuccess && block.second > 0)
-            launch = cudaMemcpyAsync(res->elist + at, block.first, 2 * (size_t)block.second * sizeof(int32_t),
-                                     cudaMemcpyDeviceToDevice, stream);
-        at += 2 * (int64_t)block.second;
+                                                                          buf.final_vlist);
+    CGNN_LAUNCH_CHECK();
+    // rows, then rule bodies: the pair keys are free by now and hold 2 * cap words
+    int32_t *elist_out = reinterpret_cast<int32_t *>(key);
+    if (total > 0)
+        CGNN_CUDA(cudaMemcpyAsync(elist_out, sym[cur], (size_t)total * sizeof(int32_t), cudaMemcpyDeviceToDevice, stream));
+    if (rules > 0)
+        CGNN_CUDA(cudaMemcpyAsync(elist_out + total, buf.rule_pairs, 2 * (size_t)rules * sizeof(int32_t),
+                                  cudaMemcpyDeviceToDevice, stream));
+    res->vlist = buf.final_vlist;
+    res->elist = elist_out;
+    if (res->owned) {  // the work arrays go, the result moves to an allocation of its own size
+        const size_t v_bytes = align_up((size_t)(n + rules + 1) * sizeof(int32_t), 256);
+        const size_t e_bytes = std::max<size_t>((size_t)res->entries, 1) * sizeof(int32_t);
+        void *exact = nullptr;
+        CGNN_CUDA(cudaMalloc(&exact, v_bytes + e_bytes));
+        std::swap(res->owned, exact);
+        std::unique_ptr<void, cudaError_t (*)(void *)> work(exact, cudaFree);
+        char *base = static_cast<char *>(res->owned);
+        CGNN_CUDA(cudaMemcpyAsync(base, res->vlist, (size_t)(n + rules + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice,
+                                  stream));
+        CGNN_CUDA(cudaMemcpyAsync(base + v_bytes, res->elist, (size_t)res->entries * sizeof(int32_t),
+                                  cudaMemcpyDeviceToDevice, stream));
+        CGNN_CUDA(cudaStreamSynchronize(stream));
+        res->vlist = reinterpret_cast<const int32_t *>(base);
+        res->elist = reinterpret_cast<const int32_t *>(base + v_bytes);
     }
-    if (launch == cudaSuccess) launch = cudaStreamSynchronize(stream);  // the arena is freed on return
-    if (launch != cudaSuccess) {
-        cgnn_compressed_destroy(res);
-        set_error("compress_csr_batch: assembling the result failed: %s", cudaGetErrorString(launch));
-        return CGNN_ERR_CUDA;
-    }
-    *out = res;
+    *out = res.release();
     return CGNN_OK;
 }
 
@@ -466,8 +481,7 @@ int cgnn_compressed_copy(const cgnn_compressed *c, int32_t *vlist_out, int32_t *
 
 void cgnn_compressed_destroy(cgnn_compressed *c) {
     if (!c) return;
-    cudaFree(c->vlist);
-    cudaFree(c->elist);
+    if (c->owned) cudaFree(c->owned);
     delete c;
 }
 

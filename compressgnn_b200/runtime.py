@@ -605,8 +605,13 @@ def compress_csr_batch(vlist, elist, rounds=12, min_pair_frequency=16):
     handle = ctypes.c_void_p(0)
     with on_device(device):
         stream = _stream_ptr(device)
-        check(lib().cgnn_compress_csr_batch(_ptr(vlist), _ptr(elist), vlist.numel() - 1, int(rounds),
-                                            int(min_pair_frequency), ctypes.byref(handle), stream))
+        # torch's allocator keeps the workspace's pages between calls, which cudaMalloc would map anew; without
+        # sizes that make sense the call below is the one that says so
+        n, frequency = vlist.numel() - 1, int(min_pair_frequency)
+        room = lib().cgnn_compress_workspace_bytes(n, elist.numel(), frequency)
+        workspace = torch.empty(room, dtype=torch.uint8, device=device)
+        check(lib().cgnn_compress_csr_batch_in(_ptr(vlist), _ptr(elist), n, int(rounds), frequency, _ptr(workspace), room,
+                                               ctypes.byref(handle), stream))
         try:
             info = (ctypes.c_int64 * 3)()
             check(lib().cgnn_compressed_info(handle, info))

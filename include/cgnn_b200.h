@@ -275,6 +275,12 @@ int cgnn_cluster_reconstruct_backward(const cgnn_plan *plan, int dtype, int64_t 
 typedef struct cgnn_compressed cgnn_compressed;
 int cgnn_compress_csr_batch(const int64_t *vlist, const int64_t *elist, int64_t n, int rounds,
                             int min_frequency, cgnn_compressed **out, cgnn_stream_t stream);
+/* The same with a caller's workspace (device, 256-byte aligned, cgnn_compress_workspace_bytes for the rows and
+ * the edges): nothing is allocated, and the result lies in the workspace until it has been copied out. */
+size_t cgnn_compress_workspace_bytes(int64_t n, int64_t entries, int min_frequency);
+int cgnn_compress_csr_batch_in(const int64_t *vlist, const int64_t *elist, int64_t n, int rounds,
+                               int min_frequency, void *workspace, size_t workspace_bytes,
+                               cgnn_compressed **out, cgnn_stream_t stream);
 int cgnn_compressed_info(const cgnn_compressed *c, int64_t info[3]);
 int cgnn_compressed_copy(const cgnn_compressed *c, int32_t *vlist_out, int32_t *elist_out,
                          cgnn_stream_t stream);

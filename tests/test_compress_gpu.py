@@ -87,6 +87,30 @@ def test_runs_of_the_left_to_right_step():
         same(compress_graph_csr(v, e, frequency, backend='cuda'), compress_graph_csr(v, e, frequency, backend='cpu'))
 
 
+def test_with_and_without_a_workspace():
+    """The entry point that allocates for itself and the one that is given a workspace."""
+    import ctypes
+    from compressgnn_b200 import runtime as rt
+    from compressgnn_b200._lib import check, lib
+    v, e = off.generate_copy_graph(2000, alpha=2.1, x_min=5.3, max_degree=500, copy_prob=0.7, window=64, candidates=8, seed=1)
+    dv, de = torch.from_numpy(v).cuda(), torch.from_numpy(e).cuda()
+    want = rt.compress_csr_batch(dv, de, 12, 4)
+    handle, info = ctypes.c_void_p(0), (ctypes.c_int64 * 3)()
+    check(lib().cgnn_compress_csr_batch(dv.data_ptr(), de.data_ptr(), v.size - 1, 12, 4, ctypes.byref(handle), 0))
+    check(lib().cgnn_compressed_info(handle, info))
+    assert list(info) == [want[2], want[3], want[1].numel()]
+    got = torch.empty_like(want[0]), torch.empty_like(want[1])
+    check(lib().cgnn_compressed_copy(handle, got[0].data_ptr(), got[1].data_ptr(), 0))
+    torch.cuda.synchronize()
+    lib().cgnn_compressed_destroy(handle)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    room = lib().cgnn_compress_workspace_bytes(v.size - 1, e.size, 4)
+    small = torch.empty(room, dtype=torch.uint8, device="cuda")
+    with pytest.raises(RuntimeError, match="workspace"):
+        check(lib().cgnn_compress_csr_batch_in(dv.data_ptr(), de.data_ptr(), v.size - 1, 12, 4, small.data_ptr(), room - 256,
+                                               ctypes.byref(handle), 0))
+
+
 def test_argument_errors():
     v, e = csr_of([[0, 1], [1, 5]])
     with pytest.raises(RuntimeError):
