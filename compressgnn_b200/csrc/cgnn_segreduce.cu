@@ -8,14 +8,17 @@
 //   * rows longer than `split` are cut into chunks (work units of their own); a chunk writes its
 //     partial sum to scratch, takes a ticket, and the chunk that draws the last ticket adds the
 //     partials in chunk order -- deterministic, no float atomics, and no unit ever waits for another;
-//   * three gather engines share that decomposition and produce the same bits:
+//   * the gather engines share that decomposition and its row order; on rows of more than 16 vectors they produce the
+//     same bits (narrower rows share a step among lane groups, whose sums meet in a fixed tree):
 //       seg_async_kernel  gathered rows staged through shared memory by 16-byte cp.async copies, one
 //                         warp-wide instruction per 512 bytes; rows narrower than 512 bytes bring
 //                         several entries per instruction.  The engine of every plain launch on
-//                         16-byte aligned rows (column tiles of 128 fp32 columns).
+//                         16-byte aligned rows (column tiles of 128 fp32 columns), and with 8-byte copies
+//                         of rows on 8-byte boundaries.
+//       seg_ragged_kernel the same for fp32 rows on 4-byte boundaries, by the aligned vectors that cover them.
 //       seg_bulk_kernel   rows staged by one bulk copy (cp.async.bulk + mbarrier) per row; kept for
 //                         the launches that also stage a mask row per entry or per output row.
-//       seg_kernel        register gathers; scalar rows, unaligned operands, two source matrices
+//       seg_kernel        register gathers; masked launches on unaligned or narrow rows, two source matrices
 //                         that are not a whole number of rows apart.
 #include <algorithm>
 #include <cmath>
