@@ -357,6 +357,7 @@ void check_bias(const Tensor &bias, int64_t width, const Tensor &like) {
                     "Invalid reconstruction bias");
 }
 
+// (Saved tensors are unpacked with .contiguous(): what a saved-tensor hook hands back may have other strides.)
 // The gradients of these nodes are final: differentiating them again raises.
 variable_list first_order(variable_list &&result, const variable_list &) {
     if (!at::GradMode::is_enabled()) return std::move(result);
@@ -386,7 +387,7 @@ struct MeanBackward : public Node {
             at::NoGradGuard no_grad;
             const Tensor grad = grads[0].contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
-            dx = mean_backward(grad, index_.unpack(), counts_.unpack());
+            dx = mean_backward(grad, index_.unpack().contiguous(), counts_.unpack().contiguous());
         }
         return first_order({dx}, grads);
     }
@@ -452,8 +453,8 @@ struct ReconstructBackward : public Node {
             at::NoGradGuard no_grad;
             const Tensor grad = grads[0].contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
-            const Tensor output = relu ? output_.unpack(shared_from_this()) : Tensor();
-            const PlanPtr segments = grad.numel() ? plan_for(plan, index_.unpack(), groups) : plan;
+            const Tensor output = relu ? output_.unpack(shared_from_this()).contiguous() : Tensor();
+            const PlanPtr segments = grad.numel() ? plan_for(plan, index_.unpack().contiguous(), groups) : plan;
             // Without dropout the rows of a group are identical and one mask row per group suffices; with it every
             // row has its own zeros (dropped or clamped alike): exact mask, sums rescaled.
             r = backward_or_zero(grad, output, groups, relu ? (p > 0.0 ? 1 : 2) : 0, has_bias, segments);
@@ -517,8 +518,8 @@ struct TransformBackward : public Node {
             at::NoGradGuard no_grad;
             const Tensor grad = grads[0].contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
-            const Tensor reps = reps_.unpack();
-            const Tensor output = relu ? output_.unpack(shared_from_this()) : Tensor();
+            const Tensor reps = reps_.unpack().contiguous();
+            const Tensor output = relu ? output_.unpack(shared_from_this()).contiguous() : Tensor();
             auto r = backward_or_zero(grad, output, reps.size(0), relu ? (p > 0.0 ? 1 : 2) : 0, true, plan);
             if (p > 0.0) {
                 r.first.mul_(1.0 / (1.0 - p));
@@ -526,7 +527,7 @@ struct TransformBackward : public Node {
             }
             if (task_should_compute_output(1)) dw = matmul_tn(r.first, reps);
             if (task_should_compute_output(0))
-                dx = mean_backward(at::mm(r.first, weight_.unpack()), index_.unpack(), counts_.unpack());
+                dx = mean_backward(at::mm(r.first, weight_.unpack()), index_.unpack().contiguous(), counts_.unpack().contiguous());
             if (task_should_compute_output(2)) db = r.second;
         }
         return first_order({dx, dw, db}, grads);

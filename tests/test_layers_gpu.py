@@ -483,3 +483,28 @@ def test_chained_launches_of_a_pass(width):
             recorded.replay()
             assert torch.equal(replayed, want)
         del recorded
+
+
+def test_saved_tensors_with_other_strides():
+    """Hooks that hand the saved tensors back with other strides change no gradient."""
+    from compressgnn_b200.model import GNNLayer
+    data = make_data(n=900, width=24)
+    data.to("cuda")
+    torch.manual_seed(0)
+    layer = GNNLayer(24, 12, 8, use_transformation=True, activation="relu").cuda()
+    x = torch.randn(data.vertex_cnt, 24, device="cuda", requires_grad=True)
+    grad = torch.randn(data.vertex_cnt, 12, device="cuda")
+
+    def gradients():
+        out = layer(x, data.edge_index)
+        return torch.autograd.grad(out, [x] + list(layer.parameters()), grad)
+
+    def strided(t):
+        wide = torch.empty(*t.shape, 2, dtype=t.dtype, device=t.device)
+        wide[..., 0] = t
+        return wide[..., 0]
+
+    want = gradients()
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, strided):
+        got = gradients()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
