@@ -50,7 +50,7 @@ class _Mean:
     def apply(x, index, counts):
         _require_cuda(x)
         plan = _native.index_plan(index, counts.numel()).native if x.numel() else None
-        return _native.ops().mean(x, index, counts, plan)
+        return _native.differentiable(_native.ops().mean, x, index, counts, plan)
 
 
 def _assign(input, planes, bits, workspace=None, process_group=None):

@@ -17,8 +17,8 @@ class _Reconstruct:
 
     @staticmethod
     def apply(src, index, bias, relu, dropout_p=0.0):
-        return _native.ops().reconstruct(src, index, bias, relu, dropout_p,
-                                         _native.known_index_plan(index, src.size(0)))
+        return _native.differentiable(_native.ops().reconstruct, src, index, bias, relu, dropout_p,
+                                      _native.known_index_plan(index, src.size(0)))
 
 
 class Compressgnn_Reconstruct(torch.nn.Module):

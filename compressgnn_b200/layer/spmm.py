@@ -110,7 +110,7 @@ class Compressgnn_SPMM_Function:
     @staticmethod
     def apply(graph, x_j):
         _require_cuda(x_j)
-        return graph.propagation_plan().native.apply(x_j, False)
+        return _native.differentiable(graph.propagation_plan().native.apply, x_j, False)
 
 
 class Compressgnn_SPMM(torch.nn.Module):

@@ -29,6 +29,36 @@ _METHODS = ("rowbalance_parreduce", "rowbalance_seqreduce", "rowbalance_rowcache
 INT_MAX = 2**31 - 1
 
 
+class _Traced(torch.autograd.Function):
+    """A native operator as ONE opaque node of a ``torch.jit.trace``, replayed by calling it again."""
+
+    @staticmethod
+    def forward(ctx, op, *args):
+        # (the allocations inside are recorded too, as dead code that the trace drops)
+        with torch.enable_grad():
+            inner = [a.detach().requires_grad_() if needed else a
+                     for a, needed in zip(args, ctx.needs_input_grad[1:])]
+            out = op(*inner)
+        ctx.inputs = inner
+        ctx.save_for_backward(out)
+        return out.detach()
+
+    @staticmethod
+    def backward(ctx, grad):
+        out, = ctx.saved_tensors
+        needed = ctx.needs_input_grad[1:]
+        found = iter(torch.autograd.grad(out, [a for a, n in zip(ctx.inputs, needed) if n], grad, retain_graph=True,
+                                         create_graph=torch.is_grad_enabled(), allow_unused=True))
+        return (None, *(next(found) if n else None for n in needed))
+
+
+def differentiable(op, *args):
+    """Call a differentiable operator of the native binding.  ``torch.jit.trace`` follows the dispatcher, which these
+    operators do not pass: all it would record of one is the allocation of its result, so a trace gets an
+    opaque node instead."""
+    return op(*args) if torch._C._get_tracing_state() is None else _Traced.apply(op, *args)
+
+
 def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() else ctypes.c_void_p(0)
 
@@ -242,7 +272,7 @@ def csr_plan(vlist, elist):
 
 def known_index_plan(index, groups):
     """The binding's plan of an assignment made here, or None for an index from elsewhere."""
-    plan = _index_plans.get((index,), (groups,))
+    plan = _index_plans.get((index,), (int(groups),))
     return None if plan is None else plan.native
 
 

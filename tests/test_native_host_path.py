@@ -1,0 +1,86 @@
+"""The layers' native host path (``binding/cgnn_torch.cpp``) where it meets torch: tracing, saved tensors, gradients of
+gradients, precision switches, streams, devices and graph capture."""
+import numpy as np
+import pytest
+import torch
+
+from compressgnn_b200 import runtime as rt
+
+
+# ---------------------------------------------------------------------------------------------
+# torch.jit.trace
+# ---------------------------------------------------------------------------------------------
+class _Scaled(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, factor):
+        ctx.factor = factor
+        out = torch.empty_like(x)
+        out.numpy()[...] = x.numpy() * factor  # as a native operator: written past the dispatcher
+        return out
+
+    @staticmethod
+    def backward(ctx, grad):
+        return grad * ctx.factor, None
+
+
+def _native_like(x, factor, _plan):
+    return _Scaled.apply(x, factor)
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_a_trace_calls_the_operator_again():
+    for grad in (False, True):
+        traced = torch.jit.trace(lambda x: rt.differentiable(_native_like, x, 3.0, None) + 1,
+                                 (torch.randn(4, 5, requires_grad=grad),))
+        x = torch.randn(4, 5, requires_grad=True)
+        out = traced(x)
+        torch.testing.assert_close(out, 3 * x + 1)
+        upstream = torch.randn(4, 5)
+        out.backward(upstream, retain_graph=True)
+        torch.testing.assert_close(x.grad, 3 * upstream)
+        out.backward(upstream)
+        torch.testing.assert_close(x.grad, 6 * upstream)
+        with pytest.raises(RuntimeError, match="second time"):
+            out.backward(upstream)
+
+
+class _Holding(torch.nn.Module):
+    def __init__(self, layer, graph):
+        super().__init__()
+        self.layer, self.graph = layer, graph
+
+    def forward(self, x):
+        return self.layer(x, self.graph)
+
+
+def _graph(width=8, n=600, **kw):
+    from test_layers_gpu import make_data
+    data = make_data(n=n, width=width, **kw)
+    data.to("cuda")
+    return data.edge_index
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore")
+def test_traced_layers_replay():
+    from compressgnn_b200.layer import Compressgnn_Reconstruct, Compressgnn_SPMM, _Mean
+    from compressgnn_b200.model import GNNLayer
+    graph = _graph()
+    nodes = graph.vertex_cnt
+    index = torch.randint(0, 7, (nodes,), device="cuda")
+    counts = torch.bincount(index, minlength=7).int()
+    spmm, reconstruct = Compressgnn_SPMM(), Compressgnn_Reconstruct()
+    layer = GNNLayer(8, 5, 4, use_transformation=True, activation="relu", refresh_interval=5).cuda()
+    layer.set_epoch(0)
+    layer(torch.randn(nodes, 8, device="cuda"), graph)  # the assignment that is kept
+    bias = torch.randn(8, device="cuda")
+    for f in (lambda x: 2 * spmm(graph, x), lambda x: reconstruct(_Mean.apply(x, index, counts), index, bias, "relu"),
+              _Holding(layer, graph)):
+        x = torch.randn(nodes, 8, device="cuda", requires_grad=True)
+        want = f(x)
+        traced = torch.jit.trace(f, (torch.randn(nodes, 8, device="cuda", requires_grad=True),))
+        torch.full((1 << 20,), float("nan"), device="cuda")  # what a fresh buffer would hold
+        got = traced(x)
+        assert torch.equal(got, want)
+        upstream = torch.randn_like(want)
+        assert torch.equal(torch.autograd.grad(got, x, upstream)[0], torch.autograd.grad(want, x, upstream)[0])
