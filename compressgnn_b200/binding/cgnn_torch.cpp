@@ -172,6 +172,7 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
     const std::vector<Tensor> &ordered(bool backward, const Tensor &x, int code, cgnn_stream_t stream) {
         auto &have = ordered_[backward][code];
         if (!have.empty()) return have;
+        std::vector<Tensor> arrays;  // kept when complete: a call that fails half way leaves nothing behind
         for (auto &launch : launches_[backward]) {
             Tensor dst = at::empty({launch.first->nnz}, x.options());
             if (launch.first->nnz) {
@@ -184,8 +185,9 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
                 TORCH_CHECK(given == launch.first->nnz, "values do not match the plan's entries");
                 check(cgnn_plan_permute_values(launch.first->get(), code, data(v0), data(v1), dst.data_ptr(), stream));
             }
-            have.push_back(dst);
+            arrays.push_back(dst);
         }
+        have = std::move(arrays);
         return have;
     }
 

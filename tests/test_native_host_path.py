@@ -84,3 +84,32 @@ def test_traced_layers_replay():
         assert torch.equal(got, want)
         upstream = torch.randn_like(want)
         assert torch.equal(torch.autograd.grad(got, x, upstream)[0], torch.autograd.grad(want, x, upstream)[0])
+
+
+# ---------------------------------------------------------------------------------------------
+# the propagation's launch tables
+# ---------------------------------------------------------------------------------------------
+def _tables(plan, graph):
+    """The launches of ``graph`` as the native propagation takes them: (forward, backward)."""
+    forward = [(plan.r2v.native, [graph.r2v_graph.value])] + \
+        [(p.native, [b.value]) for p, b in zip(plan.levels, graph.r2r_graph)] + \
+        [(plan.out.native, [graph.v2r_graph.value, graph.v2v_graph.value])]
+    backward = [(plan.v2r_t.native, [graph.v2r_graph.csc()[2]])] + \
+        [(p.native, [b.csc()[2]]) for p, b in reversed(list(zip(plan.levels_t, graph.r2r_graph)))] + \
+        [(plan.out_t.native, [graph.v2v_graph.csc()[2], graph.r2v_graph.csc()[2]])]
+    return forward, backward
+
+
+@pytest.mark.gpu
+def test_a_failed_first_pass_can_be_repeated():
+    """A value array that does not match its plan fails each call, not only the first."""
+    graph = _graph()
+    plan = graph.propagation_plan()
+    forward, backward = _tables(plan, graph)
+    forward[-1] = (forward[-1][0], [forward[-1][1][0], forward[-1][1][1][:-1].contiguous()])
+    native = rt.ops().Propagation(graph.vertex_cnt, graph.rule_cnt, forward, backward)
+    x = torch.randn(graph.vertex_cnt, 8, device="cuda")
+    for _ in range(3):
+        with pytest.raises(RuntimeError, match="values do not match"):
+            native.run(x, False)
+    assert torch.equal(native.run(x, True), plan.native.run(x, True))
