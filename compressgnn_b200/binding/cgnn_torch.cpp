@@ -546,7 +546,8 @@ Tensor transform_autograd(const Tensor &x_in, const Tensor &index, const Tensor 
     check_index(index, x_in);
     check_counts(counts, x_in);
     TORCH_CHECK(index.numel() == x_in.size(0), "Input/index length mismatch");
-    TORCH_CHECK(x_in.numel() == 0 || (plan && plan->rows == counts.numel() && plan->nnz == index.numel()),
+    // (without columns the mean needs no plan, but the backward sums gradients as wide as the layer's output)
+    TORCH_CHECK(x_in.size(0) == 0 || (plan && plan->rows == counts.numel() && plan->nnz == index.numel()),
                 "transform: plan does not match index/count");
     const Tensor bias = bias_in.has_value() ? *bias_in : Tensor();
     refuse_dual("the transformation", {x_in, weight, bias});

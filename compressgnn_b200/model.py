@@ -42,7 +42,7 @@ class GNNLayer(torch.nn.Module):
             kept = self.cluster.assignment(x)
             # cluster mean, the Linear on the representatives and the fused reconstruction as ONE autograd node
             # (ref: the three modules chained in model/compressgnn/gcn.py:27-34)
-            plan = _native.index_plan(kept.index, kept.counts.numel()).native if x.numel() else None
+            plan = _native.index_plan(kept.index, kept.counts.numel()).native if x.size(0) else None
             return _native.differentiable(_native.ops().transform, x, kept.index, kept.counts, plan, self.lin.weight,
                                           self.lin.bias, self.activation == "relu", float(dropout))
         if self.use_transformation:

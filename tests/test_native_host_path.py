@@ -87,6 +87,35 @@ def test_traced_layers_replay():
 
 
 # ---------------------------------------------------------------------------------------------
+# a layer's transformation
+# ---------------------------------------------------------------------------------------------
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore:Initializing zero-element")
+@pytest.mark.parametrize("nodes, activation", [(600, None), (600, "relu"), (0, "relu")])
+def test_features_without_columns(nodes, activation):
+    """[N, 0] features: the output is the bias, its gradient the column sums, the weight's gradient is empty."""
+    layer = _layer(0, 5, activation)
+    x = torch.randn(nodes, 0, device="cuda", requires_grad=True)
+    out = layer(x, None)
+    want = layer.lin.bias.detach().expand(nodes, 5)
+    want = want.relu() if activation else want
+    assert torch.equal(out, want)
+    upstream = torch.randn(nodes, 5, device="cuda")
+    out.backward(upstream)
+    masked = upstream * (want > 0) if activation else upstream
+    torch.testing.assert_close(layer.lin.bias.grad, masked.double().sum(0).float())
+    assert layer.lin.weight.grad.shape == (5, 0) and x.grad.shape == (nodes, 0)
+
+
+def _layer(width, out, activation=None):
+    """A GNNLayer whose propagation is the identity."""
+    from compressgnn_b200.model import GNNLayer
+    layer = GNNLayer(width, out, 4, use_transformation=True, activation=activation).cuda()
+    layer.P.forward = lambda x, **_: x
+    return layer
+
+
+# ---------------------------------------------------------------------------------------------
 # the propagation's launch tables
 # ---------------------------------------------------------------------------------------------
 def _tables(plan, graph):
