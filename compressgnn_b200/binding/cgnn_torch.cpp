@@ -315,10 +315,17 @@ std::pair<Tensor, Tensor> reconstruct_backward(const Tensor &grad, const Tensor 
 // over the GPU; it takes fp32 at full precision with up to a GPU of output tiles (64 x 128), beyond which the
 // library's tiles fill the GPU without a split, and leaves a caller who allowed TF32 products to the library.  (128 x 256 over
 // 64 k rows: 158 us there, 90 here; beyond 148 tiles neither side is measured and the library stays.)
+// The precision is asked for by the query that answers for all of torch's switches: the older one raises once the
+// newer switch has been used.
+bool full_precision_products() {
+    const auto precision = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);
+    return precision == at::Float32Precision::NONE || precision == at::Float32Precision::IEEE;
+}
+
 Tensor matmul_tn(const Tensor &a, const Tensor &b) {
     const int64_t K = a.size(0), M = a.size(1), N = b.size(1);
     const int64_t tiles = ((M + 63) / 64) * ((N + 127) / 128);
-    if (a.scalar_type() != at::kFloat || tiles > 148 || tiles == 0 || at::globalContext().allowTF32CuBLAS())
+    if (a.scalar_type() != at::kFloat || tiles > 148 || tiles == 0 || !full_precision_products())
         return at::mm(a.t(), b);
     Tensor out = at::empty({M, N}, a.options());
     const size_t bytes = cgnn_matmul_tn_scratch_bytes(K, M, N);

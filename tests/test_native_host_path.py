@@ -107,6 +107,42 @@ def test_features_without_columns(nodes, activation):
     assert layer.lin.weight.grad.shape == (5, 0) and x.grad.shape == (nodes, 0)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("switch", ["allow_tf32", "set_float32_matmul_precision", "matmul.fp32_precision", "fp32_precision",
+                                    "ieee"])
+def test_precision_switches(switch):
+    """Each of torch's ways to allow TF32 products sends the weight gradient to the library, none makes it raise."""
+    matmul = torch.backends.cuda.matmul
+    layer = _layer(24, 12)
+    x = torch.randn(600, 24, device="cuda")
+    a, b = torch.randn(3000, 48, device="cuda"), torch.randn(3000, 65, device="cuda")
+    layer(x, None).square().sum().backward()
+    want, full = layer.lin.weight.grad.clone(), rt.ops().matmul_tn(a, b)
+    layer.lin.weight.grad = None
+    try:
+        if switch == "allow_tf32":
+            matmul.allow_tf32 = True
+        elif switch == "set_float32_matmul_precision":
+            torch.set_float32_matmul_precision("high")
+        elif switch == "matmul.fp32_precision":
+            matmul.fp32_precision = "tf32"
+        elif switch == "fp32_precision":
+            torch.backends.fp32_precision = "tf32"
+        else:
+            matmul.fp32_precision = "ieee"
+        layer(x, None).square().sum().backward()
+        assert torch.equal(rt.ops().matmul_tn(a, b), full if switch == "ieee" else a.t() @ b)
+    finally:
+        torch.backends.fp32_precision = matmul.fp32_precision = "none"
+        torch.set_float32_matmul_precision("highest")
+        matmul.fp32_precision = "none"
+    assert not matmul.allow_tf32
+    # three products of operands rounded to 11 bits, against sums of some hundred terms
+    error = (layer.lin.weight.grad.double() - want.double()).norm() / want.double().norm()
+    assert error <= 4 * 2.0 ** -11
+    assert torch.equal(rt.ops().matmul_tn(a, b), full)
+
+
 def _layer(width, out, activation=None):
     """A GNNLayer whose propagation is the identity."""
     from compressgnn_b200.model import GNNLayer
