@@ -367,9 +367,10 @@ void check_bias(const Tensor &bias, int64_t width, const Tensor &like) {
 }
 
 // (Saved tensors are unpacked with .contiguous(): what a saved-tensor hook hands back may have other strides.)
-// The gradients of these nodes are final: differentiating them again raises.
-variable_list first_order(variable_list &&result, const variable_list &) {
-    if (!at::GradMode::is_enabled()) return std::move(result);
+// The gradients of these nodes are final: differentiating them again raises.  That takes an incoming gradient that
+// is differentiated itself; with a constant one the result is a constant.
+variable_list first_order(variable_list &&result, const variable_list &incoming) {
+    if (!torch::autograd::compute_requires_grad(incoming)) return std::move(result);
     variable_list wrapped;
     for (auto &t : result) {
         if (t.defined()) {

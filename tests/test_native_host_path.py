@@ -152,6 +152,43 @@ def _layer(width, out, activation=None):
 
 
 # ---------------------------------------------------------------------------------------------
+# gradients of gradients
+# ---------------------------------------------------------------------------------------------
+def _operators():
+    """(function of one differentiable matrix, its shape) of every first-order operator."""
+    from compressgnn_b200.layer import Compressgnn_Reconstruct, _Mean
+    index = torch.randint(0, 7, (60,), device="cuda")
+    counts = torch.bincount(index, minlength=7).int()
+    rt.index_plan(index, 7)  # the reconstruction's plan is known, as it is inside a layer
+    reconstruct, layer = Compressgnn_Reconstruct(), _layer(6, 4, "relu")
+    return [(lambda x: _Mean.apply(x, index, counts), (60, 6)),
+            (lambda x: reconstruct(x, index), (7, 6)),
+            (lambda x: reconstruct(x, index, activation="relu"), (7, 6)),
+            (lambda x: layer(x, None), (60, 6))]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", range(4))
+def test_gradients_of_first_order_operators(which):
+    """With create_graph: a gradient taken with a constant upstream gradient is a constant, one taken with a
+    differentiable upstream gradient refuses to be differentiated."""
+    f, shape = _operators()[which]
+    x = torch.randn(shape, device="cuda", requires_grad=True)
+    w = torch.randn(shape, device="cuda", requires_grad=True)
+    out = f(x)
+    (plain,) = torch.autograd.grad(out, x, torch.ones_like(out), retain_graph=True)
+    (grad,) = torch.autograd.grad(out, x, torch.ones_like(out), create_graph=True)
+    assert torch.equal(grad, plain) and not grad.requires_grad
+    (grad * w).sum().backward()
+    assert torch.equal(w.grad, grad)
+    upstream = torch.ones_like(out, requires_grad=True)
+    (grad,) = torch.autograd.grad(f(x), x, upstream, create_graph=True)
+    assert torch.equal(grad, plain)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        grad.sum().backward()
+
+
+# ---------------------------------------------------------------------------------------------
 # the propagation's launch tables
 # ---------------------------------------------------------------------------------------------
 def _tables(plan, graph):
