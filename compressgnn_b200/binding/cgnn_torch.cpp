@@ -464,7 +464,8 @@ struct ReconstructBackward : public Node {
             const Tensor grad = grads[0].contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
             const Tensor output = relu ? output_.unpack(shared_from_this()).contiguous() : Tensor();
-            const PlanPtr segments = grad.numel() ? plan_for(plan, index_.unpack().contiguous(), groups) : plan;
+            const Tensor index = index_.unpack().contiguous();
+            const PlanPtr segments = grad.numel() ? plan_for(plan, index, groups) : plan;
             // Without dropout the rows of a group are identical and one mask row per group suffices; with it every
             // row has its own zeros (dropped or clamped alike): exact mask, sums rescaled.
             r = backward_or_zero(grad, output, groups, relu ? (p > 0.0 ? 1 : 2) : 0, has_bias, segments);
@@ -528,7 +529,9 @@ struct TransformBackward : public Node {
             at::NoGradGuard no_grad;
             const Tensor grad = grads[0].contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
-            const Tensor reps = reps_.unpack().contiguous();
+            // all of them, needed or not: one that was modified in place since the forward pass is an error
+            const Tensor index = index_.unpack().contiguous(), counts = counts_.unpack().contiguous();
+            const Tensor reps = reps_.unpack().contiguous(), weight = weight_.unpack();
             const Tensor output = relu ? output_.unpack(shared_from_this()).contiguous() : Tensor();
             auto r = backward_or_zero(grad, output, reps.size(0), relu ? (p > 0.0 ? 1 : 2) : 0, true, plan);
             if (p > 0.0) {
@@ -537,7 +540,7 @@ struct TransformBackward : public Node {
             }
             if (task_should_compute_output(1)) dw = matmul_tn(r.first, reps);
             if (task_should_compute_output(0))
-                dx = mean_backward(at::mm(r.first, weight_.unpack()), index_.unpack().contiguous(), counts_.unpack().contiguous());
+                dx = mean_backward(at::mm(r.first, weight), index, counts);
             if (task_should_compute_output(2)) db = r.second;
         }
         return first_order({dx, dw, db}, grads);

@@ -188,6 +188,46 @@ def test_gradients_of_first_order_operators(which):
         grad.sum().backward()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", range(4))
+def test_a_second_backward_needs_the_graph_retained(which):
+    f, shape = _operators()[which]
+    out = f(torch.randn(shape, device="cuda", requires_grad=True))
+    out.sum().backward(retain_graph=True)
+    out.sum().backward()
+    with pytest.raises(RuntimeError, match="second time"):
+        out.sum().backward()
+
+
+@pytest.mark.gpu
+def test_saved_tensors_modified_in_place():
+    """Whatever a node saved, a change between forward and backward is refused, also of what this backward can do
+    without."""
+    from compressgnn_b200.layer import Compressgnn_Reconstruct, _Mean
+    index = torch.randint(0, 7, (60,), device="cuda")
+    counts = torch.bincount(index, minlength=7).int()
+    rt.index_plan(index, 7)
+    x = torch.randn(60, 6, device="cuda")
+    reps = torch.randn(7, 6, device="cuda")
+    for f, changed in ((lambda: _Mean.apply(x.clone().requires_grad_(), index, counts), counts),
+                       (lambda: Compressgnn_Reconstruct()(reps.clone().requires_grad_(), index), index)):
+        out = f()
+        changed += 0
+        with pytest.raises(RuntimeError, match="inplace"):
+            out.sum().backward()
+    for activation in (None, "relu"):
+        layer = _layer(6, 4, activation)
+        out = layer(x, None)  # takes no gradient itself: the weight is saved, and not needed
+        with torch.no_grad():
+            layer.lin.weight += 0
+        with pytest.raises(RuntimeError, match="inplace"):
+            out.sum().backward()
+        out = layer(x, None)
+        layer.cluster.vertex_index += 0
+        with pytest.raises(RuntimeError, match="inplace"):
+            out.sum().backward()
+
+
 # ---------------------------------------------------------------------------------------------
 # the propagation's launch tables
 # ---------------------------------------------------------------------------------------------
