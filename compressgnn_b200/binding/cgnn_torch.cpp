@@ -225,12 +225,15 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
     std::vector<std::unique_ptr<Table>> tables_;
 };
 
+// What arrives for an output whose consumer returned no gradient: zeros, as autograd functions get them.
+Tensor materialized(Node &node, const Tensor &grad) { return grad.defined() ? grad : node.input_metadata(0).zeros_like(); }
+
 struct PropagateBackward : public Node {
     std::shared_ptr<Propagation> graph;
     bool backward = false;  // direction of the pass this node differentiates
     variable_list apply(variable_list &&grads) override {
-        if (!grads[0].defined() || !task_should_compute_output(0)) return {Tensor()};
-        return {graph->apply(grads[0], !backward)};
+        if (!task_should_compute_output(0)) return {Tensor()};
+        return {graph->apply(materialized(*this, grads[0]), !backward)};
     }
     std::string name() const override { return "CompressgnnPropagateBackward"; }
 };
@@ -391,11 +394,11 @@ variable_list first_order(variable_list &&result, const variable_list &incoming)
 struct MeanBackward : public Node {
     SavedVariable index_, counts_;
     variable_list apply(variable_list &&grads) override {
-        if (!grads[0].defined() || !task_should_compute_output(0)) return {Tensor()};
+        if (!task_should_compute_output(0)) return {Tensor()};
         Tensor dx;
         {
             at::NoGradGuard no_grad;
-            const Tensor grad = grads[0].contiguous();
+            const Tensor grad = materialized(*this, grads[0]).contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
             dx = mean_backward(grad, index_.unpack().contiguous(), counts_.unpack().contiguous());
         }
@@ -457,11 +460,10 @@ struct ReconstructBackward : public Node {
     bool relu = false, has_bias = false;
     double p = 0.0;
     variable_list apply(variable_list &&grads) override {
-        if (!grads[0].defined()) return {Tensor(), Tensor()};
         std::pair<Tensor, Tensor> r;
         {
             at::NoGradGuard no_grad;
-            const Tensor grad = grads[0].contiguous();
+            const Tensor grad = materialized(*this, grads[0]).contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
             const Tensor output = relu ? output_.unpack(shared_from_this()).contiguous() : Tensor();
             const Tensor index = index_.unpack().contiguous();
@@ -523,11 +525,10 @@ struct TransformBackward : public Node {
     bool relu = false;
     double p = 0.0;
     variable_list apply(variable_list &&grads) override {
-        if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
         Tensor dx, dw, db;
         {
             at::NoGradGuard no_grad;
-            const Tensor grad = grads[0].contiguous();
+            const Tensor grad = materialized(*this, grads[0]).contiguous();
             const c10::cuda::OptionalCUDAGuard guard(grad.device());
             // all of them, needed or not: one that was modified in place since the forward pass is an error
             const Tensor index = index_.unpack().contiguous(), counts = counts_.unpack().contiguous();

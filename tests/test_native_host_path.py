@@ -228,6 +228,26 @@ def test_saved_tensors_modified_in_place():
             out.sum().backward()
 
 
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x.clone()
+
+    @staticmethod
+    def backward(ctx, grad):
+        return None
+
+
+@pytest.mark.gpu
+def test_no_gradient_from_the_consumer_is_a_zero_gradient():
+    from compressgnn_b200.layer import Compressgnn_SPMM
+    graph, spmm = _graph(), Compressgnn_SPMM()
+    for f, shape in _operators() + [(lambda x: spmm(graph, x), (graph.vertex_cnt, 8))]:
+        x = torch.randn(shape, device="cuda", requires_grad=True)
+        _NoGradient.apply(f(x)).sum().backward()
+        assert x.grad is not None and x.grad.shape == shape and not x.grad.any()
+
+
 # ---------------------------------------------------------------------------------------------
 # the propagation's launch tables
 # ---------------------------------------------------------------------------------------------
