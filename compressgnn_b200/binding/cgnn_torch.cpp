@@ -6,6 +6,7 @@
 // Python side of two autograd functions, the backward one behind a GIL hand-over); here a pass costs the
 // allocations and the launches.  Nothing below computes anything the C ABI does not.
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -49,6 +50,21 @@ void refuse_dual(const char *what, at::TensorList inputs) {
     for (const Tensor &t : inputs)
         TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(t), what,
                                     " does not support forward-mode automatic differentiation");
+}
+
+// Runs `fill`, which makes a buffer that launches on any stream will read from now on, and returns when the buffer is
+// complete.  While the current stream is captured the buffer is made on another one: the captured graph may be
+// replayed late, after other users of the buffer, or never.
+template <typename Fill>
+auto complete(int device, Fill &&fill) {
+    c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(device);
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+        stream = c10::cuda::getStreamFromPool(false, device);
+    const c10::cuda::CUDAStreamGuard guard(stream);
+    auto made = fill();
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    return made;
 }
 
 // Owner of a native plan and of its scratch: one zero-initialised buffer per (width, dtype, stream), since
@@ -169,25 +185,30 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
         std::vector<size_t> scratch_bytes;
     };
 
-    const std::vector<Tensor> &ordered(bool backward, const Tensor &x, int code, cgnn_stream_t stream) {
+    // The value arrays of one direction in plan order.  Every stream reads the same ones, so they are complete before
+    // the first launch that does.
+    const std::vector<Tensor> &ordered(bool backward, const Tensor &x, int code) {
         auto &have = ordered_[backward][code];
         if (!have.empty()) return have;
-        std::vector<Tensor> arrays;  // kept when complete: a call that fails half way leaves nothing behind
-        for (auto &launch : launches_[backward]) {
-            Tensor dst = at::empty({launch.first->nnz}, x.options());
-            if (launch.first->nnz) {
-                Tensor v0 = launch.second[0].to(x.scalar_type()).contiguous(), v1;
-                int64_t given = v0.numel();
-                if (launch.second.size() > 1) {
-                    v1 = launch.second[1].to(x.scalar_type()).contiguous();
-                    given += v1.numel();
+        have = complete(x.get_device(), [&] {
+            std::vector<Tensor> arrays;
+            for (auto &launch : launches_[backward]) {
+                Tensor dst = at::empty({launch.first->nnz}, x.options());
+                if (launch.first->nnz) {
+                    Tensor v0 = launch.second[0].to(x.scalar_type()).contiguous(), v1;
+                    int64_t given = v0.numel();
+                    if (launch.second.size() > 1) {
+                        v1 = launch.second[1].to(x.scalar_type()).contiguous();
+                        given += v1.numel();
+                    }
+                    TORCH_CHECK(given == launch.first->nnz, "values do not match the plan's entries");
+                    check(cgnn_plan_permute_values(launch.first->get(), code, data(v0), data(v1), dst.data_ptr(),
+                                                   current_stream(x)));
                 }
-                TORCH_CHECK(given == launch.first->nnz, "values do not match the plan's entries");
-                check(cgnn_plan_permute_values(launch.first->get(), code, data(v0), data(v1), dst.data_ptr(), stream));
+                arrays.push_back(dst);
             }
-            arrays.push_back(dst);
-        }
-        have = std::move(arrays);
+            return arrays;
+        });
         return have;
     }
 
@@ -202,12 +223,13 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
         t->width = width;
         t->code = code;
         t->stream = stream;
-        const auto &values = ordered(backward, x, code, stream);
+        const auto &values = ordered(backward, x, code);
         const auto &launches = launches_[backward];
         for (size_t i = 0; i < launches.size(); ++i) {
             auto s = launches[i].first->scratch(width, code, stream);
             t->plans.push_back(launches[i].first->get());
             t->values.push_back(data(values[i]));
+            values[i].record_stream(c10::cuda::getCurrentCUDAStream(x.get_device()));
             t->scratch.push_back(s.first);
             t->scratch_bytes.push_back(s.second);
         }

@@ -275,3 +275,28 @@ def test_a_failed_first_pass_can_be_repeated():
         with pytest.raises(RuntimeError, match="values do not match"):
             native.run(x, False)
     assert torch.equal(native.run(x, True), plan.native.run(x, True))
+
+
+@pytest.mark.gpu
+def test_first_passes_on_two_streams():
+    """The value arrays are shared: a pass on a second stream right after the first one, on a busy stream, reads them
+    complete."""
+    x = torch.randn(3000, 40, device="cuda")
+    busy = torch.randn(2048, 2048, device="cuda")
+    graph = _graph(n=3000)
+    plan = graph.propagation_plan()
+    want = plan.native.run(x, False), plan.native.run(x, True)
+    for _ in range(3):
+        native = rt.ops().Propagation(graph.vertex_cnt, graph.rule_cnt, *_tables(plan, graph))
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        got = []
+        for stream in (first, second):
+            with torch.cuda.stream(stream):
+                if stream is first:
+                    for _ in range(40):
+                        busy @ busy
+                got.append([native.run(x, backward) for backward in (False, True)])
+        torch.cuda.synchronize()
+        for pair in got:
+            assert torch.equal(pair[0], want[0]) and torch.equal(pair[1], want[1])
