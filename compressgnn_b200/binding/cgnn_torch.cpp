@@ -52,6 +52,9 @@ void refuse_dual(const char *what, at::TensorList inputs) {
                                     " does not support forward-mode automatic differentiation");
 }
 
+// Is the current stream of the current device being captured?
+bool capturing() { return c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
 // Runs `fill`, which makes a buffer that launches on any stream will read from now on, and returns when the buffer is
 // complete.  While the current stream is captured the buffer is made on another one: the captured graph may be
 // replayed late, after other users of the buffer, or never.
@@ -59,8 +62,7 @@ template <typename Fill>
 auto complete(int device, Fill &&fill) {
     c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(device);
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
-    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-        stream = c10::cuda::getStreamFromPool(false, device);
+    if (capturing()) stream = c10::cuda::getStreamFromPool(false, device);
     const c10::cuda::CUDAStreamGuard guard(stream);
     auto made = fill();
     C10_CUDA_CHECK(cudaStreamSynchronize(stream));
@@ -85,12 +87,15 @@ class Plan {
     intptr_t address() const { return reinterpret_cast<intptr_t>(plan_); }
 
     std::pair<void *, size_t> scratch(int64_t width, int code, cgnn_stream_t stream) {
-        std::lock_guard<std::mutex> guard(lock_);
+        std::lock_guard<std::mutex> held(lock_);
         for (const auto &s : scratch_)
             if (s.width == width && s.code == code && s.stream == stream) return {s.buffer.data_ptr(), s.buffer.numel()};
         const int64_t bytes = std::max<int64_t>((int64_t)cgnn_plan_scratch_bytes(plan_, width, code), 16);
-        scratch_.push_back({width, code, stream,
-                            at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device_))});
+        const c10::cuda::CUDAGuard guard(device_);
+        auto zeros = [&] { return at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device_)); };
+        const Tensor buffer = capturing() ? complete(device_, zeros) : zeros();
+        buffer.record_stream(c10::cuda::getCurrentCUDAStream(device_));
+        scratch_.push_back({width, code, stream, buffer});
         return {scratch_.back().buffer.data_ptr(), scratch_.back().buffer.numel()};
     }
     std::pair<intptr_t, size_t> scratch_py(int64_t width, int code, intptr_t stream) {

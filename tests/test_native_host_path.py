@@ -300,3 +300,36 @@ def test_first_passes_on_two_streams():
         torch.cuda.synchronize()
         for pair in got:
             assert torch.equal(pair[0], want[0]) and torch.equal(pair[1], want[1])
+
+
+@pytest.mark.gpu
+def test_first_pass_inside_a_capture():
+    """A first pass of a value type and width while a graph is captured: what the graph object keeps of it (values in
+    plan order, scratch) is complete without a replay."""
+    graph = _graph(n=3000)
+    plan = graph.propagation_plan()
+    x = torch.randn(3000, 40, device="cuda", dtype=torch.float64)
+    want = [plan.native.run(x, backward) for backward in (False, True)]
+    side = torch.cuda.Stream()
+    for replays in (0, 2):
+        graph._plan = None
+        plan = graph.propagation_plan()
+        native = plan.native
+        assert any(p.long_rows for p in [plan.out, plan.out_t])  # scratch is used
+        torch.cuda.synchronize()
+        recorded, again = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(recorded, stream=side):
+            outs = [native.run(x, backward) for backward in (False, True)]
+        with torch.cuda.stream(side):
+            for backward in (False, True):
+                assert torch.equal(native.run(x, backward), want[backward])
+        torch.cuda.synchronize()
+        with torch.cuda.graph(again, stream=side):
+            outs_again = [native.run(x, backward) for backward in (False, True)]
+        for _ in range(replays):
+            for graph_of, results in ((again, outs_again), (recorded, outs)):
+                for out in results:
+                    out.zero_()
+                graph_of.replay()
+                assert all(torch.equal(a, b) for a, b in zip(results, want))
+        del recorded, again, outs, outs_again
