@@ -194,20 +194,30 @@ class SegmentPlan:
 
     def values(self, val0, val1=None):
         """``val0`` (and ``val1`` of the second block) brought into the plan's entry order; the
-        result is cached for as long as the given tensors live and stay unmodified."""
+        result is cached for as long as the given tensors live and stay unmodified: one array per stream, on
+        which the copy precedes the launches that read it.  A captured graph reads what was there before the
+        capture; an array it fills itself is its own."""
         tensors = (val0,) if val1 is None else (val0, val1)
-        cached = self._values.get(tensors)
-        if cached is None:
-            _require(sum(t.numel() for t in tensors) == self.nnz, "values do not match the plan's entries")
-            cached = torch.empty(self.nnz, dtype=val0.dtype, device=self.device)
-            if self.nnz:
-                with on_device(self.device):
+        arrays = self._values.get(tensors)
+        if arrays is None:
+            arrays = {}
+        stream = _stream_ptr(self.device)
+        found = arrays.get(stream)
+        if found is None:
+            with on_device(self.device):
+                capturing = torch.cuda.is_current_stream_capturing()
+                if capturing and arrays:
+                    return next(iter(arrays.values()))
+                _require(sum(t.numel() for t in tensors) == self.nnz, "values do not match the plan's entries")
+                found = torch.empty(self.nnz, dtype=val0.dtype, device=self.device)
+                if self.nnz:
                     check(lib().cgnn_plan_permute_values(
                         self.handle, _dtype_code(val0, "values"), _ptr(val0.contiguous()),
-                        _ptr(val1.contiguous()) if val1 is not None else None, _ptr(cached),
-                        _stream_ptr(self.device)))
-            self._values.put(tensors, cached)
-        return cached
+                        _ptr(val1.contiguous()) if val1 is not None else None, _ptr(found), stream))
+            if not capturing:
+                arrays[stream] = found
+                self._values.put(tensors, arrays)
+        return found
 
     def scratch(self, width, dtype_code):
         """(pointer, bytes) of this plan's scratch for launches ``width`` columns wide on the

@@ -333,3 +333,44 @@ def test_first_pass_inside_a_capture():
                 graph_of.replay()
                 assert all(torch.equal(a, b) for a, b in zip(results, want))
         del recorded, again, outs, outs_again
+
+
+@pytest.mark.gpu
+def test_values_of_a_plan_are_ordered_per_stream():
+    """``spmm_func`` with values a busy stream has yet to bring into plan order, at once on a second stream, inside a
+    capture, and after a capture that was never replayed."""
+    rng = np.random.default_rng(0)
+    rows = rng.integers(0, 9, 2000)
+    vlist = torch.from_numpy(np.concatenate([[0], np.cumsum(rows)])).cuda()
+    elist = torch.from_numpy(rng.integers(0, 2000, rows.sum())).cuda()
+    mat = torch.randn(2000, 24, device="cuda")
+    busy = torch.randn(2048, 2048, device="cuda")
+
+    def product(value):
+        return rt.spmm_func(vlist, elist, value, mat, "rowbalance_rowcache", None)
+
+    for _ in range(3):
+        value = torch.randn(elist.numel(), device="cuda")
+        want = product(value.clone())
+        first, second, third = (torch.cuda.Stream() for _ in range(3))
+        torch.cuda.synchronize()
+        recorded = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(recorded, stream=third):
+            inside = product(value)
+        with torch.cuda.stream(first):
+            for _ in range(40):
+                busy @ busy
+            got = [product(value)]
+        with torch.cuda.stream(second):
+            got.append(product(value))
+        with torch.cuda.stream(third):
+            got.append(product(value))
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, want) for g in got)
+        again = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(again, stream=third):
+            twice = product(value)
+        inside.zero_(), twice.zero_()
+        again.replay(), recorded.replay()
+        assert torch.equal(inside, want) and torch.equal(twice, want)
+        del recorded, again
