@@ -85,6 +85,7 @@ class Plan {
 
     const cgnn_plan *get() const { return plan_; }
     intptr_t address() const { return reinterpret_cast<intptr_t>(plan_); }
+    int device() const { return device_; }
 
     std::pair<void *, size_t> scratch(int64_t width, int code, cgnn_stream_t stream) {
         std::lock_guard<std::mutex> held(lock_);
@@ -132,12 +133,19 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
         : vertices_(vertices), rules_(rules) {
         launches_[0] = std::move(forward);
         launches_[1] = std::move(backward);
-        for (auto &dir : launches_) TORCH_CHECK(dir.size() >= 2, "a pass has a rule launch and a vertex launch");
+        for (auto &dir : launches_) {
+            TORCH_CHECK(dir.size() >= 2, "a pass has a rule launch and a vertex launch");
+            for (auto &launch : dir)
+                TORCH_CHECK(launch.first && launch.first->device() == device(), "the plans must lie on one device");
+        }
     }
+    int device() const { return launches_[0].front().first->device(); }
 
     // Launches first .. last of one direction (last < 0: to the end) on the current stream.
     Tensor run(const Tensor &x_in, bool backward, const Tensor &out_in, const Tensor &rule_in, int first, int last) {
         TORCH_CHECK(x_in.is_cuda(), "compressgnn_b200 runs on CUDA tensors only (no CPU propagation path)");
+        TORCH_CHECK(x_in.get_device() == device(), "the feature matrix is on cuda:", (int)x_in.get_device(),
+                    " and the graph on cuda:", device());
         const Tensor x = x_in.contiguous();
         TORCH_CHECK(x.dim() == 2, "the feature matrix must have two dimensions");
         const c10::cuda::OptionalCUDAGuard guard(x.device());
@@ -145,7 +153,7 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
         Tensor out = out_in;
         if (!out.defined()) out = at::empty({vertices_, width}, x.options());
         else
-            TORCH_CHECK(out.dim() == 2 && out.size(0) == vertices_ && out.size(1) == width &&
+            TORCH_CHECK(out.device() == x.device() && out.dim() == 2 && out.size(0) == vertices_ && out.size(1) == width &&
                             out.scalar_type() == x.scalar_type() && out.is_contiguous(),
                         "out does not match the graph and the feature matrix");
         if (out.numel() == 0) return out;
@@ -154,8 +162,8 @@ class Propagation : public std::enable_shared_from_this<Propagation> {
         Tensor rule = rule_in;
         char *rule_ptr = nullptr;
         if (rule.defined()) {
-            TORCH_CHECK(rule.dim() == 2 && rule.size(0) == rules_ && rule.size(1) == width &&
-                            rule.scalar_type() == x.scalar_type(),
+            TORCH_CHECK(rule.device() == x.device() && rule.dim() == 2 && rule.size(0) == rules_ && rule.size(1) == width &&
+                            rule.scalar_type() == x.scalar_type() && rule.is_contiguous(),
                         "rule buffer does not match the graph and the feature matrix");
             rule_ptr = static_cast<char *>(data(rule));
         } else if (rules_ > 0) {

@@ -38,7 +38,8 @@ def _rule_buffer(graph, like, given):
     ``empty_row_aligned`` against ``like``) or a fresh one."""
     if given is None:
         return _native.empty_row_aligned(graph.rule_cnt, like)
-    if given.shape != (graph.rule_cnt, like.size(1)) or given.dtype != like.dtype:
+    if given.shape != (graph.rule_cnt, like.size(1)) or given.dtype != like.dtype or \
+            given.device != like.device or not given.is_contiguous():
         raise RuntimeError("rule buffer does not match the graph and the feature matrix")
     return given
 

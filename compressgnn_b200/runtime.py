@@ -125,8 +125,10 @@ class SegmentPlan:
     def __init__(self, native, device):
         """``native``: the plan's owner in the binding, or the address of a ``cgnn_plan`` to own."""
         device = torch.device(device)
+        if device.index is None:
+            device = torch.device(device.type, torch.cuda.current_device())
         if isinstance(native, int):
-            native = ops().Plan(native, device.index if device.index is not None else torch.cuda.current_device())
+            native = ops().Plan(native, device.index)
         self.native = native
         self.device = device
         self._values = _TensorKeyedCache(limit=8)
@@ -294,6 +296,12 @@ def index_plan(index, groups):
     return plan
 
 
+def _check_operands(plan, *tensors):
+    """Raw pointers follow: every matrix is dense and on the plan's device."""
+    for t in tensors:
+        _require(t.device == plan.device and t.is_contiguous(), "spmm: Expected contiguous matrices on the plan's device")
+
+
 # -----------------------------------------------------------------------------------------
 # spmm_func  (ref: src/runtime/csrc/sparse/spmm.cpp:11-23, cuda/spmm_gpu.cu:8-107)
 # -----------------------------------------------------------------------------------------
@@ -307,6 +315,7 @@ def spmm_with_plan(plan, value, mat, out=None, accumulate=False):
         accumulate = False
     if out.numel() == 0:
         return out
+    _check_operands(plan, mat, out)
     if plan.nnz == 0:
         return out if accumulate else out.zero_()
     _require(mat.size(0) >= plan.source_rows[0],
@@ -341,6 +350,7 @@ def spmm_pair_with_plan(plan, value0, mat0, value1, mat1, out=None, accumulate=F
         accumulate = False
     if out.numel() == 0:
         return out
+    _check_operands(plan, mat0, mat1, out)
     for which, mat in enumerate((mat0, mat1)):
         _require(mat.size(0) >= plan.source_rows[which],
                  f"spmm_pair: block {which} refers to row {plan.source_rows[which] - 1} but its matrix has "

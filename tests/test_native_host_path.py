@@ -374,3 +374,40 @@ def test_values_of_a_plan_are_ordered_per_stream():
         again.replay(), recorded.replay()
         assert torch.equal(inside, want) and torch.equal(twice, want)
         del recorded, again
+
+
+@pytest.mark.gpu
+def test_operands_of_a_pass_are_checked_on_the_host():
+    """A matrix on another device, or one that is no dense matrix, is refused before anything is launched.  (Plans said
+    to lie on a second GPU stand in for a graph there.)"""
+    import ctypes
+    from compressgnn_b200.layer import spmm
+
+    def plan_on(device):
+        handle, rowptr = ctypes.c_void_p(0), torch.zeros(5, dtype=torch.int64, device="cuda")
+        rt.check(rt.lib().cgnn_plan_create(ctypes.byref(handle), 4, 8, rowptr.data_ptr(), None, 0, None, None, 0, 0,
+                                           torch.cuda.current_stream().cuda_stream))
+        return rt.ops().Plan(handle.value, device), [torch.empty(0, device="cuda")]
+
+    graph = _graph()
+    x = torch.randn(graph.vertex_cnt, 8, device="cuda")
+    want = spmm._forward(graph, x)
+    wide = torch.empty(graph.rule_cnt, 16, device="cuda")
+    for bad in (torch.empty(graph.rule_cnt, 8), wide[:, :8], wide[:, ::2], torch.empty(8, graph.rule_cnt, device="cuda").t()):
+        with pytest.raises(RuntimeError, match="rule buffer does not match"):
+            spmm._forward(graph, x, rule_out=bad)
+        for detail in (dict(record=[]), dict(per_block=True)):
+            with pytest.raises(RuntimeError, match="rule buffer does not match"):
+                spmm._forward(graph, x, rule_out=bad, **detail)
+    for bad in (torch.empty(graph.vertex_cnt, 8), torch.empty(8, graph.vertex_cnt, device="cuda").t()):
+        with pytest.raises(RuntimeError, match="out does not match"):
+            spmm._forward(graph, x, out=bad)
+        with pytest.raises(RuntimeError, match="contiguous matrices on the plan's device"):
+            spmm._forward(graph, x, out=bad, per_block=True)
+    elsewhere = rt.ops().Propagation(graph.vertex_cnt, 4, [plan_on(1), plan_on(1)], [plan_on(1), plan_on(1)])
+    for call in (elsewhere.run, elsewhere.apply):
+        with pytest.raises(RuntimeError, match="on cuda:0 and the graph on cuda:1"):
+            call(x, False)
+    with pytest.raises(RuntimeError, match="one device"):
+        rt.ops().Propagation(graph.vertex_cnt, 4, [plan_on(0), plan_on(0)], [plan_on(0), plan_on(1)])
+    assert torch.equal(spmm._forward(graph, x), want)
