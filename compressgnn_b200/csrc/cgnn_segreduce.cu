@@ -167,6 +167,15 @@ __device__ __forceinline__ int32_t entry_row(const SegArgs<T> &a, int32_t c) {
     return (c & 0x7fffffff) + ((c >> 31) & a.delta_rows);
 }
 
+// Where a gathered row begins (`base`: row 0 of src0, at the caller's column).  FAR: the second matrix is no whole
+// number of rows away, or too many for an index; r is the entry as stored and its flag adds the distance.
+template <bool FAR, typename T>
+__device__ __forceinline__ const char *gathered_row(const SegArgs<T> &a, const char *base, int32_t r, int row_bytes) {
+    if constexpr (FAR) base += (int64_t)(r & 0x7fffffff) * row_bytes + (r < 0 ? a.delta_elems * (int64_t)sizeof(T) : 0);
+    else base += (int64_t)r * row_bytes;  // one widening multiply-add
+    return base;
+}
+
 // Load U gathered feature rows (entries j .. j+U of the current batch) into registers.
 // GENERIC: the second matrix is not row-aligned with the first; its entries (flag kept in
 // bit 31 of r) add an element remainder.
@@ -774,7 +783,7 @@ __device__ __forceinline__ void async_wait() {
 // Every group keeps a partial sum of the current row (its entries in ascending order) and a row is
 // finished by adding the groups' sums with a fixed shuffle tree -- the arrangement of
 // seg_narrow_kernel, fed from shared memory instead of registers.
-template <typename T, int VW, int LPR, int VPL, bool PLAIN>
+template <typename T, int VW, int LPR, int VPL, bool PLAIN, bool FAR>
 __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
     using V = Vec<T, VW>;
     constexpr int VB = (int)sizeof(T) * VW;   // bytes of a vector
@@ -862,12 +871,13 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
     const char *const gbase = reinterpret_cast<const char *>(a.src0 + colbase);  // this lane's first vector of source row 0
 
     // ---- issue side: source rows of a 32-entry window (lane l holds entry window*32 + l) --------------
+    auto row_of = [&](int32_t c) { return FAR ? c : entry_row(a, c); };
     int32_t o = 0, o_next = 0;
-    if (lane < n_ent) o = entry_row(a, a.entries[e_begin + lane]);
-    if (32 + lane < n_ent) o_next = entry_row(a, a.entries[e_begin + 32 + lane]);
+    if (lane < n_ent) o = row_of(a.entries[e_begin + lane]);
+    if (32 + lane < n_ent) o_next = row_of(a.entries[e_begin + 32 + lane]);
     int iwindow = 0;
     auto copy_row = [&](uint32_t slot, int32_t rj) {
-        const char *src = gbase + (int64_t)rj * row_bytes;  // one widening multiply-add
+        const char *src = gathered_row<FAR>(a, gbase, rj, row_bytes);
 #pragma unroll
         for (int p = 0; p < VPL; ++p)
             if (colok[p]) async_copy<VB>(slot + (uint32_t)(p * 32 * VB), src + p * 32 * VB);
@@ -879,7 +889,7 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
                 iwindow = first >> 5;
                 o = o_next;
                 const int nxt = (iwindow + 1) * 32 + lane;
-                if (nxt < n_ent) o_next = entry_row(a, a.entries[e_begin + nxt]);
+                if (nxt < n_ent) o_next = row_of(a.entries[e_begin + nxt]);
             }
             const int cnt = n_ent - first;  // >= 1
             const uint32_t stage = ring + (uint32_t)((b % S) * K) * SLOT;
@@ -1038,7 +1048,7 @@ __device__ __forceinline__ float shared_load(uint32_t address) {
     return t;
 }
 
-template <int LPR>
+template <int LPR, bool FAR>
 __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) {
     using T = float;
     using V = Vec<T, 1>;
@@ -1118,17 +1128,18 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     const char *const gbase = reinterpret_cast<const char *>(a.src0 + col0);  // the tile's first column of source row 0
 
     // ---- issue side: source rows of a 32-entry window (lane l holds entry window*32 + l) --------------
+    auto row_of = [&](int32_t c) { return FAR ? c : entry_row(a, c); };
     int32_t o = 0, o_next = 0;
-    if (lane < n_ent) o = entry_row(a, a.entries[e_begin + lane]);
-    if (32 + lane < n_ent) o_next = entry_row(a, a.entries[e_begin + 32 + lane]);
+    if (lane < n_ent) o = row_of(a.entries[e_begin + lane]);
+    if (32 + lane < n_ent) o_next = row_of(a.entries[e_begin + 32 + lane]);
     // where in its first aligned vector a row begins, in the order the entries are consumed
     auto lead_of = [&](int32_t rj) {
-        return (int)(reinterpret_cast<uintptr_t>(gbase + (int64_t)rj * row_bytes) & 15);
+        return (int)(reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, gbase, rj, row_bytes)) & 15);
     };
     int lead = lead_of(o), lead_next = lead_of(o_next);
     int iwindow = 0;
     auto copy_row = [&](uint32_t slot, int32_t rj) {
-        const uintptr_t begin = reinterpret_cast<uintptr_t>(gbase + (int64_t)rj * row_bytes);
+        const uintptr_t begin = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, gbase, rj, row_bytes));
         const uintptr_t end = begin + tile_bytes;
         const uintptr_t at = (begin & ~(uintptr_t)15) + gl * 16;
         if (at < end) async_copy16_upto(slot, reinterpret_cast<const void *>(at), end - at);
@@ -1140,7 +1151,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
                 iwindow = first >> 5;
                 o = o_next;
                 const int nxt = (iwindow + 1) * 32 + lane;
-                if (nxt < n_ent) o_next = entry_row(a, a.entries[e_begin + nxt]);
+                if (nxt < n_ent) o_next = row_of(a.entries[e_begin + nxt]);
             }
             const int cnt = n_ent - first;  // >= 1
             const uint32_t stage = ring + (uint32_t)((b % S) * K) * SLOT + lane * 16;
@@ -1177,7 +1188,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
             lead = lead_next;
             const int nxt = (cwindow + 1) * 32 + lane;
             if (nxt < n_ent) {
-                lead_next = lead_of(entry_row(a, a.entries[e_begin + nxt]));
+                lead_next = lead_of(row_of(a.entries[e_begin + nxt]));
                 if (a.val) v_next = a.val[e_begin + nxt];
             }
         }
@@ -1278,7 +1289,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     finish_row<T, VW, LPR, VPL>(a, lr.x, lr.w, acc, colbase, colok);
 }
 
-template <typename T, int VW, int LPR, int VPL, bool PLAIN>
+template <typename T, int VW, int LPR, int VPL, bool PLAIN, bool FAR>
 static int launch_async_as(const SegArgs<T> &a, cudaStream_t stream) {
     constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 32 * VPL * VW * sizeof(T);
     constexpr int RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
@@ -1289,7 +1300,7 @@ static int launch_async_as(const SegArgs<T> &a, cudaStream_t stream) {
     {
         std::lock_guard<std::mutex> lock(mu);
         if (device >= 64 || !(configured >> device & 1)) {
-            CGNN_CUDA(cudaFuncSetAttribute(seg_async_kernel<T, VW, LPR, VPL, PLAIN>,
+            CGNN_CUDA(cudaFuncSetAttribute(seg_async_kernel<T, VW, LPR, VPL, PLAIN, FAR>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BYTES));
             if (device < 64) configured |= 1ull << device;
         }
@@ -1297,19 +1308,20 @@ static int launch_async_as(const SegArgs<T> &a, cudaStream_t stream) {
     const int64_t gx = ceil_div(a.n_direct, RPU) + a.n_items;
     const int64_t gy = ceil_div(a.width, (int64_t)LPR * VPL * VW);
     CGNN_REQUIRE(gx < (1ll << 31) && gy < 65536, "segment reduce: grid too large");
-    CGNN_CUDA(launch_chained(seg_async_kernel<T, VW, LPR, VPL, PLAIN>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
+    CGNN_CUDA(launch_chained(seg_async_kernel<T, VW, LPR, VPL, PLAIN, FAR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
     return CGNN_OK;
 }
 
-template <typename T, int VW, int LPR, int VPL>
+template <typename T, int VW, int LPR, int VPL, bool FAR = false>
 static int launch_async(const SegArgs<T> &a, cudaStream_t stream) {
+    if constexpr (FAR) return launch_async_as<T, VW, LPR, VPL, false, true>(a, stream);
     const bool plain = !a.accumulate && a.div_counts == nullptr && a.seg_mask == nullptr &&
                        a.width % (LPR * VPL * VW) == 0;
-    return plain ? launch_async_as<T, VW, LPR, VPL, true>(a, stream)
-                 : launch_async_as<T, VW, LPR, VPL, false>(a, stream);
+    return plain ? launch_async_as<T, VW, LPR, VPL, true, false>(a, stream)
+                 : launch_async_as<T, VW, LPR, VPL, false, false>(a, stream);
 }
 
-template <int LPR>
+template <int LPR, bool FAR>
 static int launch_ragged_as(const SegArgs<float> &a, cudaStream_t stream) {
     constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 512;
     static_assert(BYTES <= 48 * 1024, "more than the default shared memory of a block");
@@ -1317,30 +1329,38 @@ static int launch_ragged_as(const SegArgs<float> &a, cudaStream_t stream) {
     const int64_t gx = ceil_div(a.n_direct, RPU) + a.n_items;
     const int64_t gy = ceil_div(a.width, (int64_t)ragged_tile(LPR));
     CGNN_REQUIRE(gx < (1ll << 31) && gy < 65536, "segment reduce: grid too large");
-    CGNN_CUDA(launch_chained(seg_ragged_kernel<LPR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
+    CGNN_CUDA(launch_chained(seg_ragged_kernel<LPR, FAR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
     return CGNN_OK;
 }
+
+template <typename T, int VW, bool MASKED, bool GENERIC>
+static int launch_vw(const SegArgs<T> &a, cudaStream_t stream);
 
 // Rows that are not 16-byte vectors throughout, without a mask row per entry: 8-byte copies where every row starts on an
 // 8-byte boundary, else the aligned cover.  The fewest lanes that hold the row; but with a mask row per group
 // the sums keep seg_kernel's order, that of one lane group, whatever the width: both mask modes of
 // reconstruct backward then give the same bits.  No more column tiles than ticket_tiles() has words for.
-template <typename T>
+// FAR (see gathered_row): the same lane groups and so the same sums, since where two buffers happen to lie must not
+// show in the bits; rows of a whole warp have seg_kernel's order in any engine and go there.
+template <typename T, bool FAR>
 static int launch_unaligned(const SegArgs<T> &a, bool aligned8, cudaStream_t stream) {
     const bool one_group = a.seg_mask != nullptr;
     constexpr int VW = 8 / (int)sizeof(T);
     const int64_t vecs = a.width / VW;
     if constexpr (sizeof(T) == 4) {
-        if (!aligned8) {
-            if (!one_group && a.width <= ragged_tile(4)) return launch_ragged_as<4>(a, stream);
-            if (!one_group && a.width <= ragged_tile(8)) return launch_ragged_as<8>(a, stream);
-            if (!one_group && a.width <= ragged_tile(16)) return launch_ragged_as<16>(a, stream);
-            return launch_ragged_as<32>(a, stream);
+        if (!aligned8 && !one_group) {
+            if (a.width <= ragged_tile(4)) return launch_ragged_as<4, FAR>(a, stream);
+            if (a.width <= ragged_tile(8)) return launch_ragged_as<8, FAR>(a, stream);
+            if (a.width <= ragged_tile(16)) return launch_ragged_as<16, FAR>(a, stream);
         }
+        if (!aligned8 && !FAR) return launch_ragged_as<32, false>(a, stream);
     }
-    if (!one_group && vecs <= 4) return launch_async<T, VW, 4, 1>(a, stream);
-    if (!one_group && vecs <= 8) return launch_async<T, VW, 8, 1>(a, stream);
-    if (!one_group && vecs <= 16) return launch_async<T, VW, 16, 1>(a, stream);
+    if ((sizeof(T) == 8 || aligned8) && !one_group) {
+        if (vecs <= 4) return launch_async<T, VW, 4, 1, FAR>(a, stream);
+        if (vecs <= 8) return launch_async<T, VW, 8, 1, FAR>(a, stream);
+        if (vecs <= 16) return launch_async<T, VW, 16, 1, FAR>(a, stream);
+    }
+    if constexpr (FAR) return launch_vw<T, 1, false, true>(a, stream);
     if (vecs <= 32) return launch_async<T, VW, 32, 1>(a, stream);
     return launch_async<T, VW, 32, 2>(a, stream);
 }
@@ -1386,12 +1406,12 @@ template <typename T, int VW, bool MASKED, bool GENERIC>
 static int launch_vw(const SegArgs<T> &a, cudaStream_t stream) {
     const int64_t vecs = a.width / VW;
 #if CGNN_SEG_ASYNC
-    if constexpr (sizeof(T) * VW == 16 && !MASKED && !GENERIC) {
+    if constexpr (sizeof(T) * VW == 16 && !MASKED) {
         if (a.seg_mask == nullptr && a.width * (int64_t)sizeof(T) < 0x7fffffffll) {
-            if (vecs <= 4) return launch_async<T, VW, 4, 1>(a, stream);
-            if (vecs <= 8) return launch_async<T, VW, 8, 1>(a, stream);
-            if (vecs <= 16) return launch_async<T, VW, 16, 1>(a, stream);
-            if (vecs >= CGNN_SEG_BULK_MIN_VECS) {
+            if (vecs <= 4) return launch_async<T, VW, 4, 1, GENERIC>(a, stream);
+            if (vecs <= 8) return launch_async<T, VW, 8, 1, GENERIC>(a, stream);
+            if (vecs <= 16) return launch_async<T, VW, 16, 1, GENERIC>(a, stream);
+            if (!GENERIC && vecs >= CGNN_SEG_BULK_MIN_VECS) {
                 if (vecs <= 32 || vecs > CGNN_SEG_ASYNC_MAX_VECS) return launch_async<T, VW, 32, 1>(a, stream);
                 if (vecs <= 64) return launch_async<T, VW, 32, 2>(a, stream);
             }
@@ -1473,20 +1493,18 @@ static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *s
     if (!accumulate && p->compact)
         CGNN_CUDA(cudaMemsetAsync(out, 0, (size_t)p->rows * (size_t)width * sizeof(T), stream));
     if (p->n_direct + p->n_items == 0) return CGNN_OK;
-    if (!row_aligned) {  // two sources that are not a whole number of rows apart
+    auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
+    const bool half = width * sizeof(T) % 8 == 0 && aligned8(src0) && aligned8(src1) && aligned8(seg_mask) && aligned8(out);
+    if (!row_aligned) {  // two sources that are not a whole number of rows apart (never with a mask)
         if (vec) return launch_vw<T, VWMAX, false, true>(a, stream);
-        return launch_vw<T, 1, false, true>(a, stream);
+        return launch_unaligned<T, true>(a, half, stream);
     }
     if (vec) {
         if (mask) return launch_vw<T, VWMAX, true, false>(a, stream);
         return launch_vw<T, VWMAX, false, false>(a, stream);
     }
     if (mask) return launch_vw<T, 1, true, false>(a, stream);
-    if (width * (int64_t)sizeof(T) < 0x7fffffffll) {
-        auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
-        return launch_unaligned<T>(a, width * sizeof(T) % 8 == 0 && aligned8(src0) && aligned8(src1) && aligned8(seg_mask) &&
-                                          aligned8(out), stream);
-    }
+    if (width * (int64_t)sizeof(T) < 0x7fffffffll) return launch_unaligned<T, false>(a, half, stream);
     return launch_vw<T, 1, false, false>(a, stream);
 }
 

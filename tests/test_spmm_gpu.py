@@ -285,3 +285,38 @@ def test_offsets_beyond_32_bits(rt):
     assert torch.equal(y, x.index_select(0, idx))
     del x
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_where_the_second_matrix_lies_does_not_show(rt, dtype):
+    """The fused pass with its two matrices a whole number of rows apart, a fraction of a row more, and beyond 2^30
+    rows (an index cannot hold that distance): the same bits."""
+    rng = np.random.default_rng(33)
+    rows, n0, n1 = 900, 300, 700
+    rp0, c0 = random_csr(rng, rows, n0, 4, long_rows=[(3, 200)])
+    rp1, c1 = random_csr(rng, rows, n1, 7, long_rows=[(3, 90), (500, 300)])
+    plan = rt.SegmentPlan.from_csr(cu(rp0), cu(c0), cu(rp1), cu(c1))
+    v0, v1 = (torch.from_numpy(rng.standard_normal(c.size)).to("cuda", dtype) for c in (c0, c1))
+    size = torch.empty((), dtype=dtype).element_size()
+    for width in (1, 2, 3, 4, 5, 6, 8, 10, 12, 13, 16, 24, 28, 32, 47, 60, 61, 64, 96, 130):
+        whole = width * size % 16 == 0, width * size % 8 == 0
+        fraction = (16 if whole[0] else 8 if whole[1] else 4) // size  # elements; keeps the alignment of the rows
+        reach = 2 ** 30 + 2 ** 20 if width * size <= 16 else 0      # 17 GB at most
+        buf = torch.empty((reach + n0 + n1 + 16) * width, dtype=dtype, device="cuda")
+        m0, m1 = (torch.from_numpy(rng.standard_normal((n, width))).to("cuda", dtype) for n in (n0, n1))
+
+        def run(at0, at1):
+            a, b = buf[at0:at0 + n0 * width].view(n0, width), buf[at1:at1 + n1 * width].view(n1, width)
+            a.copy_(m0), b.copy_(m1)
+            return rt.spmm_pair_with_plan(plan, v0, a, v1, b)
+
+        want = run(0, (n0 + 4) * width)
+        ref = oracle.spmm(rp1, c1, v1.cpu().numpy(), m1.cpu().numpy(),
+                          out=oracle.spmm(rp0, c0, v0.cpu().numpy(), m0.cpu().numpy()))
+        assert_close_rel(want.cpu().numpy(), ref, what=f"width {width}")
+        assert torch.equal(run((n1 + 4) * width, 0), want), width
+        if fraction % width:
+            assert torch.equal(run(0, (n0 + 4) * width + fraction), want), (width, "fraction of a row")
+        if reach:
+            assert torch.equal(run(0, (n0 + reach) * width), want), (width, "far")
+        del buf
