@@ -1353,14 +1353,17 @@ static int launch_unaligned(const SegArgs<T> &a, bool aligned8, cudaStream_t str
             if (a.width <= ragged_tile(8)) return launch_ragged_as<8, FAR>(a, stream);
             if (a.width <= ragged_tile(16)) return launch_ragged_as<16, FAR>(a, stream);
         }
-        if (!aligned8 && !FAR) return launch_ragged_as<32, false>(a, stream);
     }
     if ((sizeof(T) == 8 || aligned8) && !one_group) {
         if (vecs <= 4) return launch_async<T, VW, 4, 1, FAR>(a, stream);
         if (vecs <= 8) return launch_async<T, VW, 8, 1, FAR>(a, stream);
         if (vecs <= 16) return launch_async<T, VW, 16, 1, FAR>(a, stream);
     }
-    if constexpr (FAR) return launch_vw<T, 1, false, true>(a, stream);
+    // seg_kernel's column tiles are the widest (256): it also takes what would be more tiles here than a grid has rows
+    constexpr int64_t TILE = sizeof(T) == 4 ? ragged_tile(32) : 64;
+    if (FAR || a.width > 65535 * TILE) return launch_vw<T, 1, false, FAR>(a, stream);
+    if constexpr (sizeof(T) == 4)
+        if (!aligned8) return launch_ragged_as<32, false>(a, stream);
     if (vecs <= 32) return launch_async<T, VW, 32, 1>(a, stream);
     return launch_async<T, VW, 32, 2>(a, stream);
 }

@@ -320,3 +320,22 @@ def test_where_the_second_matrix_lies_does_not_show(rt, dtype):
         if reach:
             assert torch.equal(run(0, (n0 + reach) * width), want), (width, "far")
         del buf
+
+
+@pytest.mark.parametrize("dtype, tile", [(torch.float32, 124), (torch.float32, 128), (torch.float64, 64)])
+def test_rows_of_more_column_tiles_than_a_grid_has_rows(rt, dtype, tile):
+    """Widths at which the staged engines for rows of no whole vectors (tiles of 124, 128 and 64 columns) run out of
+    grid rows."""
+    for width in (65535 * tile - (1 if tile == 64 else 2), 65535 * tile + (1 if tile != 128 else 2)):
+        rp, col = np.array([0, 2, 2, 75]), np.concatenate([[1, 0], np.arange(73) % 2])
+        val = np.random.default_rng(1).standard_normal(75)
+        mat = torch.randn(2, width, device="cuda", dtype=dtype)
+        weights = torch.zeros(3, 2, dtype=torch.float64)
+        weights.index_put_((torch.from_numpy(np.repeat(np.arange(3), np.diff(rp))), torch.from_numpy(col)),
+                           torch.from_numpy(val), accumulate=True)
+        got = rt.spmm_func(cu(rp), cu(col), cu(val).to(dtype), mat, "rowbalance_rowcache", None)
+        for row in range(3):
+            want = (weights[row].cuda()[:, None] * mat.double()).sum(0)
+            # a chain of 73 fused multiply-adds, half an ulp of the magnitudes each, and the rounding of the values
+            bound = 80 * torch.finfo(dtype).eps * float(np.abs(val).sum()) * float(mat.abs().max())
+            assert float((got[row].double() - want).abs().max()) <= bound
