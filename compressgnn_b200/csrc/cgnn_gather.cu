@@ -293,9 +293,10 @@ __global__ void __launch_bounds__(EXPAND_BLOCK_THREADS) expand_block_kernel(cons
     // rows of up to 256 elements: several row blocks side by side; wider ones: all threads on one
     const int slot = width <= EXPAND_BLOCK_THREADS ? (int)(threadIdx.x / width) : 0;
     if (slot < blocks_at_once) {
-        for (int64_t j = threadIdx.x - slot * width; j < width; j += EXPAND_BLOCK_THREADS) {
+        const int64_t at = (int64_t)blockIdx.y * EXPAND_BLOCK_THREADS + threadIdx.x - slot * width;
+        for (int64_t j = at; j < width; j += EXPAND_BLOCK_THREADS * (int64_t)gridDim.y) {
             const int r0 = (int)(j * VW / width);              // row of the block the vector begins in
-            const int c0 = (int)(j * VW - r0 * width);         // and its first column there
+            const int64_t c0 = j * VW - r0 * width;            // and its first column there
             const int here = (int)min((int64_t)VW, width - c0);  // elements before that row ends
             T bias[VW];
 #pragma unroll
@@ -344,14 +345,14 @@ __global__ void __launch_bounds__(EXPAND_BLOCK_THREADS) expand_block_kernel(cons
         }
     }
     // the rows behind the last whole block (fewer than VW)
-    if (blockIdx.x == 0) {
-        for (int64_t e = blocks * VW * width + threadIdx.x; e < a.n * width; e += EXPAND_BLOCK_THREADS) {
-            const int64_t r = e / width;
-            Vec<T, 1> y;
-            y.v[0] = expand_element(a, r, e - r * width);
-            if (a.drop_threshold) drop_vector<T, 1>(y, e, a.drop_threshold, a.keep_scale, a.seed);
-            a.out[e] = y.v[0];
-        }
+    const int64_t block = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, all = (int64_t)gridDim.x * gridDim.y;
+    for (int64_t e = (blocks * VW * width) + block * EXPAND_BLOCK_THREADS + threadIdx.x; e < a.n * width;
+         e += all * EXPAND_BLOCK_THREADS) {
+        const int64_t r = e / width;
+        Vec<T, 1> y;
+        y.v[0] = expand_element(a, r, e - r * width);
+        if (a.drop_threshold) drop_vector<T, 1>(y, e, a.drop_threshold, a.keep_scale, a.seed);
+        a.out[e] = y.v[0];
     }
 }
 
@@ -376,8 +377,12 @@ static int expand_typed(const ExpandArgs<T> &a, cudaStream_t stream) {
     }
     if (a.div_counts == nullptr && aligned16(a.out) && a.width > 4) {
         const int at_once = (int)std::max<int64_t>(1, EXPAND_BLOCK_THREADS / a.width);
-        const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n / VWMAX, at_once), 148 * 6));  // 3 fit an SM
-        expand_block_kernel<T><<<(unsigned)grid, EXPAND_BLOCK_THREADS, 0, stream>>>(a, at_once);
+        constexpr int64_t most = 148 * 6;  // 3 fit an SM
+        const int64_t gx = std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n / VWMAX, at_once), most));
+        // few and wide rows: what is missing of `most` shares the columns (100 rows x 10,007: 47 -> 8 us; 3 x 100,003,
+        // all behind the last whole block: 465 -> 6)
+        const int64_t gy = std::min<int64_t>(ceil_div(a.width, EXPAND_BLOCK_THREADS), most / gx);
+        expand_block_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), EXPAND_BLOCK_THREADS, 0, stream>>>(a, at_once);
         CGNN_LAUNCH_CHECK();
         return CGNN_OK;
     }

@@ -285,3 +285,18 @@ def test_expanded_rows_of_no_whole_vectors(rt, dtype):
     assert not out[1].any() and not out[3].any() and torch.equal(out[4], cu(reps)[3])
     with pytest.raises(RuntimeError):
         rt.raise_on_device_status()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_expanded_rows_few_and_wide(rt, dtype):
+    """Few rows whose columns are shared among the blocks, and rows behind the last whole block of rows: bit for bit
+    the oracle's."""
+    rng = np.random.default_rng(12)
+    for width in (511, 513, 10007, 227329):  # 888 slices of 256 positions and one more
+        for n in (1, 2, 3, 5, 9, 103):
+            if n * width > 3_000_000:
+                continue
+            idx = rng.integers(0, 4, n)
+            reps, bias = rng.standard_normal((4, width)).astype(dtype), rng.standard_normal(width).astype(dtype)
+            got = rt.cluster_reconstruct(cu(reps), cu(idx), cu(bias), True)
+            np.testing.assert_array_equal(got.cpu().numpy(), oracle.reconstruct(reps, idx, bias, True))
