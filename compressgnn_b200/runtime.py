@@ -643,6 +643,12 @@ _STATUS_BITS = ((1, "an index outside its table was skipped"),
                 (4, "a CSR array held a negative or over-wide index"))
 
 
+# Most bytes the compressor leaves in torch's cache: 47 M edges' worth.  (3 M edges: 2.6 ms with the pages kept, 4.0 mapped
+# anew; 23 M: 13.4 and 32.  Beyond the bound the memory matters more: the library's own allocations, which a graph's
+# plans are made with, cannot use what torch keeps.)
+KEPT_WORKSPACE = 4 << 30
+
+
 def compress_csr_batch(vlist, elist, rounds=12, min_pair_frequency=16):
     """Grammar compression of a CSR graph on the GPU (``cgnn_compress_csr_batch``): ``vlist`` /
     ``elist`` are int64 CUDA tensors; returns ``(vlist int32, elist int32, vertices, rules)`` as CUDA
@@ -655,10 +661,12 @@ def compress_csr_batch(vlist, elist, rounds=12, min_pair_frequency=16):
     handle = ctypes.c_void_p(0)
     with on_device(device):
         stream = _stream_ptr(device)
-        # torch's allocator keeps the workspace's pages between calls, which cudaMalloc would map anew; without
-        # sizes that make sense the call below is the one that says so
+        # Up to KEPT_WORKSPACE the workspace is torch's, whose allocator keeps the pages between calls where cudaMalloc
+        # would map them anew; a larger one the library allocates, and gives back to the driver on return.  (With
+        # sizes that make no sense the call below is the one that says so.)
         n, frequency = vlist.numel() - 1, int(min_pair_frequency)
         room = lib().cgnn_compress_workspace_bytes(n, elist.numel(), frequency)
+        room = room if room <= KEPT_WORKSPACE else 0
         workspace = torch.empty(room, dtype=torch.uint8, device=device)
         check(lib().cgnn_compress_csr_batch_in(_ptr(vlist), _ptr(elist), n, int(rounds), frequency, _ptr(workspace), room,
                                                ctypes.byref(handle), stream))

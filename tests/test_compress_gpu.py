@@ -111,6 +111,22 @@ def test_with_and_without_a_workspace():
                                                ctypes.byref(handle), 0))
 
 
+def test_a_large_workspace_goes_back_to_the_driver(monkeypatch):
+    """Beyond the bound nothing of the work stays in torch's cache, and the arrays are the same."""
+    from compressgnn_b200 import runtime as rt
+    v, e = off.generate_copy_graph(20000, alpha=2.1, x_min=5.3, max_degree=500, copy_prob=0.7, window=64, candidates=8, seed=1)
+    dv, de = torch.from_numpy(v).cuda(), torch.from_numpy(e).cuda()
+    room = rt.lib().cgnn_compress_workspace_bytes(v.size - 1, e.size, 4)
+    want = rt.compress_csr_batch(dv, de, 12, 4)
+    torch.cuda.empty_cache()
+    monkeypatch.setattr(rt, "KEPT_WORKSPACE", room - 1)
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.max_memory_reserved()
+    got = rt.compress_csr_batch(dv, de, 12, 4)
+    assert torch.cuda.max_memory_reserved() - before < room // 2  # the result only
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and got[2:] == want[2:]
+
+
 def test_argument_errors():
     v, e = csr_of([[0, 1], [1, 5]])
     with pytest.raises(RuntimeError):
