@@ -46,10 +46,12 @@ def _compress_on_device(vlist, elist, rounds, frequency):
     # the host array (2.3 ms at 3.4 M edges) are needed only to name the error, or for edges behind the last row.
     if vlist.size < 1 or vlist[-1] != elist.size:
         require_int32_range()
+    if vlist.size > 1 and vlist[-1] > elist.size:
+        raise RuntimeError(runtime._BAD_ROW_POINTERS)
     # Runtime failures (out of memory included) propagate; nothing falls back to the host.
     try:
-        v, e, n, r = runtime.compress_csr_batch(torch.from_numpy(vlist).cuda(), torch.from_numpy(elist).cuda(),
-                                                rounds=rounds, min_pair_frequency=frequency)
+        v, e, n, r = runtime._compress_rows(torch.from_numpy(vlist).cuda(), torch.from_numpy(elist).cuda(), rounds,
+                                            frequency)
     except RuntimeError:
         require_int32_range()
         raise

@@ -138,6 +138,8 @@ def compress_csr_batch(vlist, elist, threads=4, rounds=12, min_pair_frequency=16
     vlist, elist = _i64(vlist), _i64(elist)
     if vlist.size < 1 or (elist.size and (elist.max() > np.iinfo(np.int32).max or elist.min() < 0)):
         raise ValueError("CSR value exceeds int32 range")
+    if vlist.size > 1 and vlist[-1] > elist.size:
+        raise ValueError("CSR row pointers exceed the edge count")
     frequency, threads, rounds = (operator.index(min_pair_frequency), operator.index(threads),
                                   operator.index(rounds))
     with _Result() as res:

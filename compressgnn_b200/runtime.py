@@ -656,7 +656,16 @@ def compress_csr_batch(vlist, elist, rounds=12, min_pair_frequency=16):
     _require(vlist.is_cuda and elist.is_cuda and vlist.device == elist.device, "compress_csr_batch needs CUDA tensors")
     _require(vlist.dtype == torch.int64 and elist.dtype == torch.int64 and vlist.dim() == 1 and elist.dim() == 1 and
              vlist.numel() >= 1, "compress_csr_batch needs one-dimensional int64 arrays")
-    vlist, elist = vlist.contiguous(), elist.contiguous()
+    _require(vlist.numel() == 1 or int(vlist[-1]) <= elist.numel(), _BAD_ROW_POINTERS)
+    return _compress_rows(vlist.contiguous(), elist.contiguous(), rounds, min_pair_frequency)
+
+
+_BAD_ROW_POINTERS = "compress_csr_batch: row pointers must ascend from 0 to the edge count"
+
+
+def _compress_rows(vlist, elist, rounds, min_pair_frequency):
+    """``compress_csr_batch`` of contiguous arrays whose last row pointer is known not to lie beyond the edges (the
+    library sees the pointers only)."""
     device = vlist.device
     handle = ctypes.c_void_p(0)
     with on_device(device):

@@ -127,6 +127,19 @@ def test_a_large_workspace_goes_back_to_the_driver(monkeypatch):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and got[2:] == want[2:]
 
 
+def test_row_pointers_beyond_the_edges_are_refused():
+    """Nothing is read behind the edge array, by however little the last row pointer passes its end."""
+    from compressgnn_b200 import runtime as rt
+    for beyond in (1, 2, 300):
+        vlist, elist = np.array([0, 2, 2 + beyond], np.int64), np.array([0, 1], np.int64)
+        with pytest.raises(RuntimeError, match="row pointers"):
+            compress_graph_csr(vlist, elist, 3, backend='cuda')
+        with pytest.raises(RuntimeError, match="row pointers"):
+            rt.compress_csr_batch(torch.from_numpy(vlist).cuda(), torch.from_numpy(elist).cuda())
+    with pytest.raises(RuntimeError, match="row pointers"):
+        rt.compress_csr_batch(torch.tensor([0, 1], device="cuda"), torch.empty(0, dtype=torch.int64, device="cuda"))
+
+
 def test_argument_errors():
     v, e = csr_of([[0, 1], [1, 5]])
     with pytest.raises(RuntimeError):

@@ -197,3 +197,10 @@ def test_helpers_match_the_compiled_reference_when_present():
                             theirs[2][1], [l[0] for l in lt], [l[1] for l in lt])
         np.testing.assert_array_equal(dm[0], dt[0])
         np.testing.assert_array_equal(dm[1], dt[1])
+
+
+def test_compressor_refuses_row_pointers_beyond_the_edges():
+    from compressgnn_b200.loader import compress_graph_csr
+    for beyond in (1, 2, 300):
+        with pytest.raises(ValueError, match="row pointers"):
+            compress_graph_csr(np.array([0, 2, 2 + beyond]), np.array([0, 1]), 3, backend="cpu")
