@@ -1,10 +1,10 @@
 // Native host path of the layers: the operators of include/cgnn_b200.h called on torch tensors, with
 // their autograd nodes, in C++.
 //
-// What bounds it is host time: a small propagation's six kernels take 26 us on the device while the
-// interpreter needed 130 us to issue them (argument checks, ctypes conversions, torch.empty calls and the
-// Python side of two autograd functions, the backward one behind a GIL hand-over); here a pass costs the
-// allocations and the launches.  Nothing below computes anything the C ABI does not.
+// What bounds it is host time: a small propagation's six kernels take 26 us on the device.  Issued from Python it
+// takes 135 us (argument checks, ctypes conversions, torch.empty calls and two autograd functions, the backward one
+// behind a GIL hand-over), from here 62: the allocations and the launches.  Nothing below computes anything
+// the C ABI does not.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>

@@ -1,4 +1,4 @@
-"""In-tree build of the native libraries (no JIT cache, no torch headers).
+"""In-tree build of the native libraries (no JIT cache; torch headers for the binding only).
 
 ``libcgnn_b200.so``   -- the sm_100a CUDA kernels behind the C ABI of ``include/cgnn_b200.h``
                          (``csrc/*.cu``, compiled by nvcc, one object per file, in parallel).

@@ -43,8 +43,8 @@ static inline unsigned blocks_for(int64_t count) {
 
 // Device buffers of one compression, result included, carved out of one block (sized by a dry pass of the same requests):
 // the caller's workspace, or an allocation of this call.  What a call without a workspace pays for is
-// not the kernels but the driver mapping and unmapping 250 MB.  325 k-node graph, host arrays in
-// and out: 8.4 ms with an allocation per call and per round, 5.9 ms with a workspace.
+// not the kernels but the driver mapping and unmapping 280 MB.  325 k-node graph, device arrays in and out: 4.0 ms
+// without a workspace, 2.6 with one.
 struct Arena {
     char *block = nullptr;
     size_t used = 0;
@@ -185,9 +185,8 @@ __global__ void take_heavier_kernel(const uint64_t *key, const uint64_t *weight,
 // That rule is a chain, but a short one: a position is OPEN when it is a candidate the first step left, with no
 // pair of the first step behind it.  Along a run of open positions the taken ones simply alternate, starting with
 // the first unless the pair before the run was taken; everything between two runs is settled already.  So the
-// thread of a run's first position walks the run (rows of the web graph: a few symbols), where one thread per
-// row used to walk whole rows, the longest of 10,000 symbols.  Five rounds on the 325 k-node graph:
-// 649 -> 90 us.
+// thread of a run's first position walks the run (rows of the web graph: a few symbols); one thread to a row would
+// walk whole rows, the longest of 10,000 symbols.  Five rounds on the 325 k-node graph: 90 us, by rows 649.
 // take[]: bit 0 the first step, bit 1 this one; a run's bytes are written by its own thread and other threads
 // look at bit 0 only.
 __global__ void take_greedy_kernel(const uint64_t *key, const uint64_t *weight, int64_t total, uint8_t *take) {

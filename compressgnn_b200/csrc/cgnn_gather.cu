@@ -271,8 +271,8 @@ static int launch_expand(const ExpandArgs<T> &a, cudaStream_t stream) {
 // 16-byte vector) are exactly `width` aligned vectors, so the output is written as blocks of VW rows in whole
 // aligned vectors, a vector taking its elements from up to two node rows.  What bounds it is instructions, not
 // the bytes stored: a thread keeps ONE vector position of the block -- its row, column and bias values are computed
-// once, where a flat walk over the output divided 64-bit positions and looked up four indices per
-// vector -- and has EXPAND_BLOCK_U blocks in flight.  325 k rows x 47: 36 -> 29 us.
+// once, where a flat walk over the output divides 64-bit positions and looks up four indices per
+// vector -- and has EXPAND_BLOCK_U blocks in flight.  325 k rows x 47: 27 us, by the flat walk 36.
 constexpr int EXPAND_BLOCK_THREADS = 256, EXPAND_BLOCK_U = 4;
 
 template <typename T>
@@ -379,8 +379,8 @@ static int expand_typed(const ExpandArgs<T> &a, cudaStream_t stream) {
         const int at_once = (int)std::max<int64_t>(1, EXPAND_BLOCK_THREADS / a.width);
         constexpr int64_t most = 148 * 6;  // 3 fit an SM
         const int64_t gx = std::max<int64_t>(1, std::min<int64_t>(ceil_div(a.n / VWMAX, at_once), most));
-        // few and wide rows: what is missing of `most` shares the columns (100 rows x 10,007: 47 -> 8 us; 3 x 100,003,
-        // all behind the last whole block: 465 -> 6)
+        // few and wide rows: what is missing of `most` shares the columns (100 rows x 10,007: 8 us, and 47 with one slice;
+        // 3 x 100,003, all behind the last whole block: 6 and 465)
         const int64_t gy = std::min<int64_t>(ceil_div(a.width, EXPAND_BLOCK_THREADS), most / gx);
         expand_block_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), EXPAND_BLOCK_THREADS, 0, stream>>>(a, at_once);
         CGNN_LAUNCH_CHECK();

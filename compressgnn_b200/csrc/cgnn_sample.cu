@@ -217,10 +217,9 @@ __global__ void seed_kernel(const int64_t *samples, int64_t count, int64_t n, in
 // ---------------------------------------------------------------------------------------
 // All hops of a batch without a host round trip (cgnn_sample_hops).
 //
-// What bounds a batch is latency: 60 k edges are a few microseconds of traffic, but hop by hop the host had to
-// learn two sizes per hop (edges, new vertices) before it could allocate and go on, the picks were
-// one thread's chain of dependent index reads, and ~15 small launches stood between them.  Here
-// frontier node i of a hop owns `stride` = min(fan-out, largest degree) pick slots, so the buffers are
+// What bounds a batch is latency: 60 k edges are a few microseconds of traffic, but hop by hop the host learns two
+// sizes per hop (edges, new vertices) before it can allocate and go on, a pick is one thread's
+// chain of dependent index reads, and ~15 small launches stand between them.  Here frontier node i of a hop owns `stride` = min(fan-out, largest degree) pick slots, so the buffers are
 // sized by a bound the host knows beforehand and the true sizes stay on the device:
 //   * a slot's position counts over the whole batch (seeds first, then hop after hop), and first[v] keeps
 //     the smallest position that named vertex v -- earlier hops have smaller positions, so one
@@ -229,8 +228,8 @@ __global__ void seed_kernel(const int64_t *samples, int64_t count, int64_t n, in
 //     totals of the hop before it; its value at first[v] IS the local id of v;
 //   * a warp picks for one node: the children of up to 32 rules are listed per step, and the lookups of Floyd's
 //     draws run side by side.
-// A batch of 1024 seeds with fan-outs 25 and 10 on the 325 k-node graph: 505 -> 131 us; the two pick kernels were 150 us of
-// it.  Going hop by hop stays for batches whose slots would exceed MAX_POSITIONS.
+// A batch of 1024 seeds with fan-outs 25 and 10 on the 325 k-node graph: 131 us, hop by hop 505 (150 of them in the two
+// pick kernels).  Going hop by hop stays for batches whose slots would exceed MAX_POSITIONS.
 // ---------------------------------------------------------------------------------------
 constexpr int32_t EMPTY_SLOT = -1;  // picked[]: no pick here
 constexpr int32_t BAD_VERTEX = -2;  // picked[]: an edge to a vertex outside the graph (reported; local id 0)

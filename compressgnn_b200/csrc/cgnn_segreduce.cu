@@ -18,8 +18,8 @@
 //       seg_ragged_kernel the same for fp32 rows on 4-byte boundaries, by the aligned vectors that cover them.
 //       seg_bulk_kernel   rows staged by one bulk copy (cp.async.bulk + mbarrier) per row; kept for
 //                         the launches that also stage a mask row per entry or per output row.
-//       seg_kernel        register gathers; masked launches on unaligned or narrow rows, two source matrices
-//                         that are not a whole number of rows apart.
+//       seg_kernel        register gathers; masked launches on unaligned or narrow rows, wide rows of two source
+//                         matrices that are no whole number of rows apart, widths beyond the others' grids.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -132,8 +132,9 @@ struct SegArgs {
 // stream serialization: once every block of the launch before it has started (chain_open), its blocks
 // are scheduled as that one's finish, read the plan -- which was complete before the pass began -- and
 // wait (chain_wait) until the launch before has completed and its writes are visible.  A launch whose follower
-// is not ours opens nothing.  Forward + backward at 2,708 nodes x 16:
-// 65.1 -> 61.5 us; 40,000 x 128 in fp64: 120.5 -> 108.7; forward at 325 k x 64: 107.8 -> 102.9.
+// is not ours opens nothing.  Without and with the overlap: forward + backward at 2,708 nodes x 16
+// 65.1 and 61.5 us; 40,000 x 128 in fp64 120.5 and 108.7; forward at 325 k x 64 107.8 and 102.9; no difference beyond
+// noise at 325 k x 256.
 enum { CHAIN_FOLLOWS = 1, CHAIN_LEADS = 2 };
 template <typename T>
 __device__ __forceinline__ void chain_open(const SegArgs<T> &a) {
@@ -1023,8 +1024,8 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 
 // ---------------------------------------------------------------------------------------
 // Rows of fp32 that start on any 4-byte boundary (odd widths: 47 class scores, or a view that begins anywhere): the
-// same cp.async engine with one shift.  What bounded these rows in seg_kernel was instructions and loads in
-// flight -- one 4-byte load per element and entry.  Here a tile of a gathered row is copied by the ALIGNED
+// same cp.async engine with one shift.  seg_kernel is bound by instructions and loads in flight on such rows -- one
+// 4-byte load per element and entry.  Here a tile of a gathered row is copied by the ALIGNED
 // 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is one vector short of that
 // (ragged_tile), so the cover always fits.  The last vector copies no byte past the tile's end, and the first
 // starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then
@@ -1033,7 +1034,7 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 // copied, hence the two __syncwarp per stage.  Rows on 8-byte boundaries (even widths; any width in fp64)
 // take seg_async_kernel with 8-byte copies instead, which needs neither the shift nor the second lane.
 // Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 396 through the aligned cover, 320 with 8-byte
-// copies.  Segment sums of 7 columns (2,708 rows): 34 -> 10 us, of 47 (325 k rows): 116 -> 108.
+// copies.  Segment sums of 7 columns (2,708 rows): 34 us in seg_kernel, 10 here; of 47 (325 k rows): 116 and 108.
 // ---------------------------------------------------------------------------------------
 __host__ __device__ constexpr int ragged_tile(int lpr) { return (lpr - 1) * 4; }
 // 16 bytes into shared memory of which the first min(left, 16) are read, the others zero.
@@ -1536,8 +1537,9 @@ static int run(const cgnn_plan *p, int dtype, int64_t width, const void *val, co
 // ---------------------------------------------------------------------------------------
 // Column sums of a small [rows, width] matrix in two fixed-order stages (bias gradient): blocks of COLSUM_ROWS
 // rows, then the blocks' sums.  What bounds them is the length of the dependent chain, not bytes, so a block's
-// rows are shared among its warps and several loads are in flight: 36 us a call were two launches of 11 and 25 us, now 5 us
-// each.
+// rows are shared among its warps and several loads are in flight: 32 rows to a warp in the first stage, rows / 2048 in
+// the second (some 30 at 65 k rows, 8192 at the most rows a grid takes, 16.8 M).  65 k rows x 47: two launches of 5 us
+// (11 and 25 us with one thread to a column and 64 rows).
 // ---------------------------------------------------------------------------------------
 constexpr int COLSUM_ROWS = 256;
 
@@ -1800,13 +1802,11 @@ int plan_build(cgnn_plan *p, const int32_t *const rowptr[2], const int32_t *cons
 // ---------------------------------------------------------------------------------------
 // Plan construction on the device (see cgnn_plan.h): the decisions of plan_build.
 //
-// What bounds it is the number of SMs at work and the longest serial stretch.  One CTA used to take the
-// statistics, one CTA the five prefix sums (34 and 59 us at 60 k rows, 121 us when the row pointers did
-// not fit its shared memory), and one warp copied a row's entries, however long (348 us when a few buckets
-// hold most of 325 k nodes).  Now the statistics are one pass over the whole GPU into a row-length histogram
-// that the last block to finish evaluates, the prefix sums go tile by tile (partial sums first), and
-// the entries are copied one per thread.  An assignment refresh of 2.45 M x 128 rows, 16 bits: 134 -> 35 us
-// of kernels, 546 -> 475 us in all; the 348 us copy is 5 us.
+// What bounds it is the number of SMs at work and the longest serial stretch.  So the statistics are one pass over
+// the whole GPU into a row-length histogram that the last block to finish evaluates, the prefix sums go
+// tile by tile (partial sums first), and the entries are copied one per thread, not one row per warp: a few
+// buckets may hold most of the rows (325 k nodes in such buckets: 5 us, and 348 row by row).  The kernels
+// for a refresh of 2.45 M x 128 rows, 16 bits: 35 us; with one CTA for the statistics and one for the sums, 134.
 // ---------------------------------------------------------------------------------------
 constexpr int PLAN_CTA = 1024;
 constexpr int PLAN_HIST_CAP = 4096;  // lengths of PLAN_HIST_CAP and more share the last bin
