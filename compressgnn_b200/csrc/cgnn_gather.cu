@@ -269,8 +269,8 @@ static int launch_expand(const ExpandArgs<T> &a, cudaStream_t stream) {
 
 // Rows whose byte length is no multiple of 16 (47 class scores: 188 bytes): VW consecutive rows (VW elements to a
 // 16-byte vector) are exactly `width` aligned vectors, so the output is written as blocks of VW rows in whole
-// aligned vectors, a vector taking its elements from up to two node rows.  What bounds it is instructions, not
-// the bytes stored: a thread keeps ONE vector position of the block -- its row, column and bias values are computed
+// aligned vectors, a vector taking its elements from up to two node rows.  What bounds it is instructions and the
+// latency of the index and table reads, not the bytes (issue slots 58 % busy, DRAM 8 %): a thread keeps ONE vector position of the block -- its row, column and bias values are computed
 // once, where a flat walk over the output divides 64-bit positions and looks up four indices per
 // vector -- and has EXPAND_BLOCK_U blocks in flight.  325 k rows x 47: 27 us, by the flat walk 36.
 constexpr int EXPAND_BLOCK_THREADS = 256, EXPAND_BLOCK_U = 4;
