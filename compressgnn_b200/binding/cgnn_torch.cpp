@@ -95,6 +95,7 @@ class Plan {
         const c10::cuda::CUDAGuard guard(device_);
         auto zeros = [&] { return at::zeros({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device_)); };
         const Tensor buffer = capturing() ? complete(device_, zeros) : zeros();
+        TORCH_CHECK(buffer.data_ptr() != nullptr, "the operators of compressgnn_b200 need tensors with memory, not fake ones");
         buffer.record_stream(c10::cuda::getCurrentCUDAStream(device_));
         scratch_.push_back({width, code, stream, buffer});
         return {scratch_.back().buffer.data_ptr(), scratch_.back().buffer.numel()};

@@ -411,3 +411,27 @@ def test_operands_of_a_pass_are_checked_on_the_host():
     with pytest.raises(RuntimeError, match="one device"):
         rt.ops().Propagation(graph.vertex_cnt, 4, [plan_on(0), plan_on(0)], [plan_on(0), plan_on(1)])
     assert torch.equal(spmm._forward(graph, x), want)
+
+
+@pytest.mark.gpu
+def test_fake_tensors_leave_nothing_behind():
+    """A pass under a fake tensor mode is refused, and what it asked for is not kept for real ones."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    graph = _graph(n=3000)
+    native = graph.propagation_plan().native
+    x = torch.randn(3000, 40, device="cuda")
+    native.run(torch.randn(3000, 8, device="cuda"), False)  # the value arrays are known, the scratch of 40 columns is not
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        with pytest.raises(RuntimeError):
+            native.run(x, False)
+        with pytest.raises(RuntimeError):
+            native.run(torch.empty(3000, 40, device="cuda"), False)
+    per_launch = torch.empty_like(x)
+    rule = rt.empty_row_aligned(graph.rule_cnt, x)
+    for i in range(graph.propagation_plan().launches):
+        native.run(x, False, per_launch, rule, i, i)
+    assert torch.equal(native.run(x, False), per_launch)
+    from conftest import assert_close_rel
+    from oracle import oracle
+    from test_layers_gpu import oracle_blocks
+    assert_close_rel(per_launch.cpu().numpy(), oracle.propagate_forward(oracle_blocks(graph), x.cpu().numpy()))
