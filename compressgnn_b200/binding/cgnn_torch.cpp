@@ -652,11 +652,11 @@ std::tuple<Tensor, Tensor, int64_t, PlanPtr> assign(const Tensor &x, const Tenso
 namespace py = pybind11;
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    using nogil = py::call_guard<py::gil_scoped_release>;
     py::class_<Plan, PlanPtr>(m, "Plan")
         .def(py::init<intptr_t, int>())
         .def_property_readonly("handle", &Plan::address)
-        .def("scratch", &Plan::scratch_py);
-    using nogil = py::call_guard<py::gil_scoped_release>;
+        .def("scratch", &Plan::scratch_py, nogil());
     py::class_<Propagation, std::shared_ptr<Propagation>>(m, "Propagation")
         .def(py::init<int64_t, int64_t, std::vector<Propagation::Launch>, std::vector<Propagation::Launch>>())
         .def("apply", &Propagation::apply, nogil())
