@@ -675,7 +675,10 @@ def _compress_rows(vlist, elist, rounds, min_pair_frequency):
         # sizes that make no sense the call below is the one that says so.)
         n, frequency = vlist.numel() - 1, int(min_pair_frequency)
         room = lib().cgnn_compress_workspace_bytes(n, elist.numel(), frequency)
-        room = room if room <= KEPT_WORKSPACE else 0
+        if room > KEPT_WORKSPACE:
+            if torch.cuda.mem_get_info(device)[0] < room + room // 4:
+                torch.cuda.empty_cache()  # what torch keeps for later stands in the library's way
+            room = 0
         workspace = torch.empty(room, dtype=torch.uint8, device=device)
         check(lib().cgnn_compress_csr_batch_in(_ptr(vlist), _ptr(elist), n, int(rounds), frequency, _ptr(workspace), room,
                                                ctypes.byref(handle), stream))
