@@ -14,8 +14,8 @@
 //                         warp-wide instruction per 512 bytes; rows narrower than 512 bytes bring
 //                         several entries per instruction.  The engine of every plain launch on
 //                         16-byte aligned rows (column tiles of 128 fp32 columns), and with 8-byte copies
-//                         of rows on 8-byte boundaries.
-//       seg_ragged_kernel the same for fp32 rows on 4-byte boundaries, by the aligned vectors that cover them.
+//                         of other fp64 rows.
+//       seg_ragged_kernel the same for fp32 rows on 8- or 4-byte boundaries, by the aligned vectors that cover them.
 //       seg_bulk_kernel   rows staged by one bulk copy (cp.async.bulk + mbarrier) per row; kept for
 //                         the launches that also stage a mask row per entry or per output row.
 //       seg_kernel        register gathers; masked launches on unaligned or narrow rows, wide rows of two source
@@ -1023,43 +1023,47 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Rows of fp32 that start on any 4-byte boundary (odd widths: 47 class scores, or a view that begins anywhere): the
-// same cp.async engine with one shift.  seg_kernel is bound by instructions and loads in flight on such rows -- one
-// 4-byte load per element and entry.  Here a tile of a gathered row is copied by the ALIGNED
-// 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is one vector short of that
-// (ragged_tile), so the cover always fits.  The last vector copies no byte past the tile's end, and the first
-// starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then
-// reads elements gl, gl + LPR, ... (consecutive words across the lanes, no bank conflict) from the row's
-// offset into the cover, which it gets by shuffle from the lane that loaded the entry.  Lanes read what other lanes
-// copied, hence the two __syncwarp per stage.  Rows on 8-byte boundaries (even widths; any width in fp64)
-// take seg_async_kernel with 8-byte copies instead, which needs neither the shift nor the second lane.
-// Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 396 through the aligned cover, 320 with 8-byte
-// copies.  Segment sums of 7 columns (2,708 rows): 34 us in seg_kernel, 10 here; of 47 (325 k rows): 116 and 108.
+// Rows of fp32 that start on any 4-byte boundary (widths that are no multiple of four, or a view that begins anywhere):
+// the same cp.async engine with one shift.  seg_kernel is bound by instructions and loads in flight on such rows, and
+// 8-byte copies of rows on 8-byte boundaries by twice the copies.  Here a tile of a gathered row is copied by the ALIGNED
+// 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is short of that by the worst lead
+// (ragged_tile), so the cover always fits.  Where the row goes on behind the tile the whole cover is copied (each vector
+// holds bytes of the row); in the row's last tile nothing past its end is, and the first vector
+// starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then reads units of
+// UNIT bytes -- 8 where every row begins on an 8-byte boundary, else 4 -- gl, gl + LPR, ... (consecutive words across the
+// lanes, no bank conflict) from the row's offset into the cover, which it gets by shuffle from the lane that
+// loaded the entry.  Lanes read what other lanes copied, hence the two __syncwarp per stage.
+// Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 320 with 8-byte copies, 295 here (the
+// aligned engine at 604 columns takes the same number of tiles).  Segment sums of 7 columns (2,708 rows): 34 us in
+// seg_kernel, 10 here.
 // ---------------------------------------------------------------------------------------
-__host__ __device__ constexpr int ragged_tile(int lpr) { return (lpr - 1) * 4; }
+// Columns that LPR aligned vectors hold wherever a row begins: all but the unit's worst lead.
+__host__ __device__ constexpr int ragged_tile(int lpr, int unit) { return (lpr * 16 - (16 - unit)) / 4; }
 // 16 bytes into shared memory of which the first min(left, 16) are read, the others zero.
-__device__ __forceinline__ void async_copy16_upto(uint32_t dst_shared, const void *src, uintptr_t left) {
+__device__ __forceinline__ void async_copy16_upto(uint32_t dst_shared, const void *src, int left) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_shared), "l"(src),
-                 "r"((uint32_t)(left < 16 ? left : 16))
+                 "r"(left < 16 ? left : 16)
                  : "memory");
 }
-__device__ __forceinline__ float shared_load(uint32_t address) {
-    float t;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t) : "r"(address));
+template <int UNIT>
+__device__ __forceinline__ Vec<float, UNIT / 4> shared_unit(uint32_t address) {
+    Vec<float, UNIT / 4> t;
+    if constexpr (UNIT == 8) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t.v[0]), "=f"(t.v[1]) : "r"(address));
+    else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(t.v[0]) : "r"(address));
     return t;
 }
 
-template <int LPR, bool FAR>
+template <int UNIT, int LPR, bool FAR>
 __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) {
     using T = float;
-    using V = Vec<T, 1>;
-    constexpr int VW = 1;
-    constexpr int VPL = 4;                    // elements of a row per lane
+    constexpr int VW = UNIT / 4;              // elements read at a time: what every row begin is a multiple of
+    constexpr int VPL = 16 / UNIT;            // units of a row per lane
+    using V = Vec<T, VW>;
     constexpr int G = 32 / LPR;               // entries per step (one warp-wide copy per vector)
     constexpr int K = async_steps(LPR), S = CGNN_SEG_ASYNC_S, RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     constexpr int KE = K * G;                 // entries per stage
     static_assert(32 % KE == 0, "a stage must not straddle two entry windows");
-    constexpr int TILE = ragged_tile(LPR);    // columns of one tile
+    constexpr int TILE = ragged_tile(LPR, UNIT);  // columns of one tile
     constexpr int SLOT = 512;                 // bytes of one staged step
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(128) unsigned char async_smem[];
@@ -1072,13 +1076,14 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     const int64_t width = a.width;
     const int row_bytes = (int)(width * (int64_t)sizeof(T));  // < 2^31: checked by the launcher
     const int64_t col0 = (int64_t)blockIdx.y * TILE;
-    const int64_t colbase = col0 + gl;
+    const int64_t colbase = col0 + gl * VW;
+    const bool inner = col0 + TILE < width;   // rows go on behind the tile: its whole cover may be read
     const int tile_bytes = (int)min((int64_t)TILE, width - col0) * (int)sizeof(T);
     bool colok[VPL];
     V acc[VPL];
 #pragma unroll
     for (int p = 0; p < VPL; ++p) {
-        colok[p] = gl + p * LPR < TILE && colbase + p * LPR < width;
+        colok[p] = (gl + p * LPR) * VW < TILE && colbase + p * (LPR * VW) < width;
         acc[p] = vec_zero<T, VW>();
     }
     const int64_t direct_units = (a.n_direct + RPU - 1) / RPU;
@@ -1106,7 +1111,10 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
 #pragma unroll
             for (int m = LPR; m < 32; m <<= 1) {
 #pragma unroll
-                for (int p = 0; p < VPL; ++p) acc[p].v[0] += __shfl_xor_sync(FULL, acc[p].v[0], m);
+                for (int p = 0; p < VPL; ++p) {
+#pragma unroll
+                    for (int i = 0; i < VW; ++i) acc[p].v[i] += __shfl_xor_sync(FULL, acc[p].v[i], m);
+                }
             }
         }
     };
@@ -1127,6 +1135,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     const int n_ent = e_end - e_begin;
     const int nb = (n_ent + KE - 1) / KE;
     const char *const gbase = reinterpret_cast<const char *>(a.src0 + col0);  // the tile's first column of source row 0
+    const char *const lbase = gbase + gl * 16;
 
     // ---- issue side: source rows of a 32-entry window (lane l holds entry window*32 + l) --------------
     auto row_of = [&](int32_t c) { return FAR ? c : entry_row(a, c); };
@@ -1139,11 +1148,15 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     };
     int lead = lead_of(o), lead_next = lead_of(o_next);
     int iwindow = 0;
-    auto copy_row = [&](uint32_t slot, int32_t rj) {
-        const uintptr_t begin = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, gbase, rj, row_bytes));
-        const uintptr_t end = begin + tile_bytes;
-        const uintptr_t at = (begin & ~(uintptr_t)15) + gl * 16;
-        if (at < end) async_copy16_upto(slot, reinterpret_cast<const void *>(at), end - at);
+    // Vector gl of the aligned cover: the lane's 16 bytes do not change what the row's begin is modulo 16.
+    auto copy_inner = [&](uint32_t slot, int32_t rj) {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, lbase, rj, row_bytes)) & ~(uintptr_t)15;
+        async_copy<16>(slot, reinterpret_cast<const void *>(at));
+    };
+    auto copy_last = [&](uint32_t slot, int32_t rj) {  // nothing past the row's end
+        const uintptr_t row = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, lbase, rj, row_bytes));
+        const int left = tile_bytes - gl * 16 + (int)(row & 15);
+        if (left > 0) async_copy16_upto(slot, reinterpret_cast<const void *>(row & ~(uintptr_t)15), left);
     };
     auto issue = [&](int b) {
         if (b < nb) {
@@ -1157,14 +1170,17 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
             const int cnt = n_ent - first;  // >= 1
             const uint32_t stage = ring + (uint32_t)((b % S) * K) * SLOT + lane * 16;
             const int pos = (first & 31) + gk;
-            if (cnt >= KE) {
+            if (cnt >= KE && inner) {
 #pragma unroll
-                for (int j = 0; j < K; ++j) copy_row(stage + (uint32_t)(j * SLOT), __shfl_sync(FULL, o, pos + j * G));
+                for (int j = 0; j < K; ++j) copy_inner(stage + (uint32_t)(j * SLOT), __shfl_sync(FULL, o, pos + j * G));
             } else {
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
                     const int32_t rj = __shfl_sync(FULL, o, (pos + j * G) & 31);
-                    if (j * G + gk < cnt) copy_row(stage + (uint32_t)(j * SLOT), rj);
+                    if (j * G + gk < cnt) {
+                        if (inner) copy_inner(stage + (uint32_t)(j * SLOT), rj);
+                        else copy_last(stage + (uint32_t)(j * SLOT), rj);
+                    }
                 }
             }
         }
@@ -1204,10 +1220,10 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
         for (int j = 0; j < K; ++j) {
             // element gl + p * LPR of the row sits at that offset from the row's own first byte
             const uint32_t row = stage + (uint32_t)(j * SLOT + gk * (LPR * 16)) + __shfl_sync(FULL, lead, (pos + j * G) & 31) +
-                                 gl * (uint32_t)sizeof(T);
+                                 gl * (uint32_t)UNIT;
 #pragma unroll
             for (int p = 0; p < VPL; ++p)
-                if (colok[p]) x[j][p].v[0] = shared_load(row + (uint32_t)(p * LPR * (int)sizeof(T)));
+                if (colok[p]) x[j][p] = shared_unit<UNIT>(row + (uint32_t)(p * LPR * UNIT));
         }
         __syncwarp();  // every lane has read the stage
         if (cnt >= KE && ebase + KE <= row_end && ebase < row_end) {  // a full stage inside the current row
@@ -1322,51 +1338,56 @@ static int launch_async(const SegArgs<T> &a, cudaStream_t stream) {
                  : launch_async_as<T, VW, LPR, VPL, false, false>(a, stream);
 }
 
-template <int LPR, bool FAR>
-static int launch_ragged_as(const SegArgs<float> &a, cudaStream_t stream) {
+template <int UNIT, int LPR, bool FAR>
+static int launch_ragged(const SegArgs<float> &a, cudaStream_t stream) {
     constexpr size_t BYTES = (size_t)CGNN_SEG_ASYNC_S * async_steps(LPR) * 512;
     static_assert(BYTES <= 48 * 1024, "more than the default shared memory of a block");
     constexpr int RPU = LPR == 32 ? CGNN_SEG_ASYNC_RPU : CGNN_SEG_NARROW_RPU;
     const int64_t gx = ceil_div(a.n_direct, RPU) + a.n_items;
-    const int64_t gy = ceil_div(a.width, (int64_t)ragged_tile(LPR));
+    const int64_t gy = ceil_div(a.width, (int64_t)ragged_tile(LPR, UNIT));
     CGNN_REQUIRE(gx < (1ll << 31) && gy < 65536, "segment reduce: grid too large");
-    CGNN_CUDA(launch_chained(seg_ragged_kernel<LPR, FAR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
+    CGNN_CUDA(launch_chained(seg_ragged_kernel<UNIT, LPR, FAR>, dim3((unsigned)gx, (unsigned)gy), BYTES, a, stream));
     return CGNN_OK;
 }
 
 template <typename T, int VW, bool MASKED, bool GENERIC>
 static int launch_vw(const SegArgs<T> &a, cudaStream_t stream);
 
-// Rows that are not 16-byte vectors throughout, without a mask row per entry: 8-byte copies where every row starts on an
-// 8-byte boundary, else the aligned cover.  The fewest lanes that hold the row; but with a mask row per group
+// fp32 rows by their aligned cover: the fewest lanes that hold the row.  No more column tiles than
+// ticket_tiles() has words for.  One lane group (`one_group`, see launch_unaligned) is a whole warp.
+template <int UNIT, bool FAR>
+static int launch_cover(const SegArgs<float> &a, bool one_group, cudaStream_t stream) {
+    if (!one_group) {
+        if (a.width <= ragged_tile(4, UNIT)) return launch_ragged<UNIT, 4, FAR>(a, stream);
+        if (a.width <= ragged_tile(8, UNIT)) return launch_ragged<UNIT, 8, FAR>(a, stream);
+        if (a.width <= ragged_tile(16, UNIT)) return launch_ragged<UNIT, 16, FAR>(a, stream);
+    }
+    // seg_kernel's column tiles are the widest (256): it also takes what would be more tiles here than a grid has rows
+    if (FAR || a.width > (int64_t)65535 * ragged_tile(32, UNIT)) return launch_vw<float, 1, false, FAR>(a, stream);
+    return launch_ragged<UNIT, 32, false>(a, stream);
+}
+
+// Rows that are not 16-byte vectors throughout, without a mask row per entry: fp32 by the aligned cover, read back in the
+// largest units every row begins on, and fp64 with 8-byte copies.  With a mask row per group
 // the sums keep seg_kernel's order, that of one lane group, whatever the width: both mask modes of
-// reconstruct backward then give the same bits.  No more column tiles than ticket_tiles() has words for.
+// reconstruct backward then give the same bits.
 // FAR (see gathered_row): the same lane groups and so the same sums, since where two buffers happen to lie must not
 // show in the bits; rows of a whole warp have seg_kernel's order in any engine and go there.
 template <typename T, bool FAR>
 static int launch_unaligned(const SegArgs<T> &a, bool aligned8, cudaStream_t stream) {
     const bool one_group = a.seg_mask != nullptr;
-    constexpr int VW = 8 / (int)sizeof(T);
-    const int64_t vecs = a.width / VW;
     if constexpr (sizeof(T) == 4) {
-        if (!aligned8 && !one_group) {
-            if (a.width <= ragged_tile(4)) return launch_ragged_as<4, FAR>(a, stream);
-            if (a.width <= ragged_tile(8)) return launch_ragged_as<8, FAR>(a, stream);
-            if (a.width <= ragged_tile(16)) return launch_ragged_as<16, FAR>(a, stream);
+        return aligned8 ? launch_cover<8, FAR>(a, one_group, stream) : launch_cover<4, FAR>(a, one_group, stream);
+    } else {
+        if (!one_group) {
+            if (a.width <= 4) return launch_async<T, 1, 4, 1, FAR>(a, stream);
+            if (a.width <= 8) return launch_async<T, 1, 8, 1, FAR>(a, stream);
+            if (a.width <= 16) return launch_async<T, 1, 16, 1, FAR>(a, stream);
         }
+        if (FAR || a.width > (int64_t)65535 * 64) return launch_vw<T, 1, false, FAR>(a, stream);
+        if (a.width <= 32) return launch_async<T, 1, 32, 1>(a, stream);
+        return launch_async<T, 1, 32, 2>(a, stream);
     }
-    if ((sizeof(T) == 8 || aligned8) && !one_group) {
-        if (vecs <= 4) return launch_async<T, VW, 4, 1, FAR>(a, stream);
-        if (vecs <= 8) return launch_async<T, VW, 8, 1, FAR>(a, stream);
-        if (vecs <= 16) return launch_async<T, VW, 16, 1, FAR>(a, stream);
-    }
-    // seg_kernel's column tiles are the widest (256): it also takes what would be more tiles here than a grid has rows
-    constexpr int64_t TILE = sizeof(T) == 4 ? ragged_tile(32) : 64;
-    if (FAR || a.width > 65535 * TILE) return launch_vw<T, 1, false, FAR>(a, stream);
-    if constexpr (sizeof(T) == 4)
-        if (!aligned8) return launch_ragged_as<32, false>(a, stream);
-    if (vecs <= 32) return launch_async<T, VW, 32, 1>(a, stream);
-    return launch_async<T, VW, 32, 2>(a, stream);
 }
 
 template <typename T, int VW, int VPL, bool MASKED>

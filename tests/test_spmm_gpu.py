@@ -91,6 +91,15 @@ def test_rows_that_are_no_whole_vectors(rt, dtype, widths, shift):
                          what=f"accumulate, width {width} shift {shift}")
 
 
+@pytest.mark.parametrize("shift", [0, 1, 2])
+@pytest.mark.parametrize("widths", [(2, 6, 10, 14, 18, 22, 26, 30, 34, 58, 62, 66, 122, 126, 130, 250, 252, 254, 378),
+                                    (8, 12, 16, 28, 32, 60, 64, 124, 128, 13, 14, 29, 30, 61, 62, 125, 126, 127, 250)])
+def test_rows_by_their_aligned_cover(rt, widths, shift):
+    """Edges of the tiles whose rows begin on 8-byte boundaries (14, 30, 62, 126 columns) and on 4-byte ones (13, 29, 61,
+    125), the matrices themselves beginning 0, 4 and 8 bytes past a 16-byte boundary."""
+    test_rows_that_are_no_whole_vectors(rt, np.float32, widths, shift)
+
+
 def test_accuracy_against_fp64(rt):
     """The fp32 CUDA result is as close to the exact (fp64) product as the reference's own
     fp32 loop is: error no larger than twice the CPU oracle's, row by row in max norm."""
