@@ -274,6 +274,68 @@ __device__ __forceinline__ void finish_row(const SegArgs<T> &a, int32_t row, int
     }
 }
 
+// Rows of more chunks than this ("hubs") are added up by a launch of their own (hub_rows_kernel).  A bucket of an
+// assignment may hold a large part of all rows (48 k of 325 k: 379 chunks), and one warp that adds so many
+// partial rows one after the other is a chain longer than the launch; up to 16 it is hidden by the launch's other
+// work, and a second launch (2 us) is not.
+constexpr int HUB_CHUNKS = 16;
+
+// The hub rows: block x looks at every gridDim.x-th long row, a lane per column of a 32-column tile, eight warps that
+// add every eighth partial row with eight loads in flight, the warps' sums in warp order.  The same order whichever
+// engine made the partial sums.  What bounds it is the latency of n_chunks / 64 dependent batches of loads.
+// Bucket mean of 325 k rows x 128 with buckets of 48 k, 21 k and 13 k: 146 us in one launch, 37 + 14 in two; 47
+// columns of reconstruct backward 108 and 25 + 12.
+constexpr int HUB_WARPS = 8;
+constexpr int HUB_UNROLL = 8;
+template <typename T>
+__global__ void __launch_bounds__(HUB_WARPS * 32) hub_rows_kernel(const SegArgs<T> a, int n_long) {
+    __shared__ int hubs[HUB_WARPS * 32];
+    __shared__ int n_hubs;
+    __shared__ T sums[HUB_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t base = blockIdx.x; base < n_long; base += (int64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x == 0) n_hubs = 0;
+        __syncthreads();
+        const int64_t mine = base + (int64_t)threadIdx.x * gridDim.x;
+        if (mine < n_long && a.longs[mine].z > HUB_CHUNKS) hubs[atomicAdd(&n_hubs, 1)] = (int)mine;
+        __syncthreads();
+        // (the list's order is not the same in two blocks: a block does its column tile of all of them)
+        const int found = n_hubs;
+        for (int h = 0; h < found; ++h) {
+            const int4 lr = a.longs[hubs[h]];
+            // a grid has at most 65,535 rows: wider matrices take several turns
+            for (int64_t tile = blockIdx.y; tile * 32 < a.width; tile += gridDim.y) {
+                const int64_t col = tile * 32 + lane;
+                const bool colok[1] = {col < a.width};
+                const T *part = a.partial + (int64_t)lr.y * a.width + col;
+                T s = T(0);
+                if (colok[0]) {
+                    int c = warp;
+                    for (; c + (HUB_UNROLL - 1) * HUB_WARPS < lr.z; c += HUB_UNROLL * HUB_WARPS) {
+                        T v[HUB_UNROLL];
+#pragma unroll
+                        for (int u = 0; u < HUB_UNROLL; ++u) v[u] = part[(int64_t)(c + u * HUB_WARPS) * a.width];
+#pragma unroll
+                        for (int u = 0; u < HUB_UNROLL; ++u) s += v[u];
+                    }
+                    for (; c < lr.z; c += HUB_WARPS) s += part[(int64_t)c * a.width];
+                }
+                sums[warp][lane] = s;
+                __syncthreads();
+                if (warp == 0) {
+                    Vec<T, 1> acc[1];
+                    acc[0].v[0] = s;
+#pragma unroll
+                    for (int w = 1; w < HUB_WARPS; ++w) acc[0].v[0] += sums[w][lane];
+                    finish_row<T, 1, 32, 1>(a, lr.x, lr.w, acc, col, colok);
+                }
+                __syncthreads();
+            }
+        }
+        __syncthreads();  // the list is read to its end before it is made anew
+    }
+}
+
 // One work unit per group of LPR lanes: a few consecutive rows of the direct list (one
 // contiguous entry range), or one chunk of a long row.
 template <typename T, int VW, int LPR, int VPL, bool MASKED, bool GENERIC>
@@ -391,6 +453,7 @@ __global__ void __launch_bounds__(CGNN_SEG_THREADS, CGNN_SEG_MINBLOCKS) seg_kern
 #pragma unroll
     for (int p = 0; p < VPL; ++p)
         if (colok[p]) vec_store<T, VW>(part + p * (LPR * VW), acc[p]);
+    if (lr.z > HUB_CHUNKS) return;  // hub_rows_kernel adds them up
     __threadfence();
     __syncwarp(gmask);
     int *tk = a.tickets + (int64_t)item.x * gridDim.y + blockIdx.y;
@@ -695,6 +758,7 @@ __global__ void __launch_bounds__(CGNN_SEG_BULK_WARPS * 32) seg_bulk_kernel(cons
 #pragma unroll
     for (int p = 0; p < VPL; ++p)
         if (colok[p]) vec_store<T, VW>(part + p * (LPR * VW), acc[p]);
+    if (lr.z > HUB_CHUNKS) return;  // hub_rows_kernel adds them up
     __threadfence();
     __syncwarp();
     int *tk = a.tickets + (int64_t)item.x * gridDim.y + blockIdx.y;
@@ -997,6 +1061,7 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 #pragma unroll
     for (int p = 0; p < VPL; ++p)
         if (colok[p]) vec_store<T, VW>(part + p * (LPR * VW), acc[p]);
+    if (lr.z > HUB_CHUNKS) return;  // hub_rows_kernel adds them up
     __threadfence();
     __syncwarp(gmask);
     int *tk = a.tickets + (int64_t)item.x * gridDim.y + blockIdx.y;
@@ -1281,6 +1346,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
 #pragma unroll
     for (int p = 0; p < VPL; ++p)
         if (colok[p]) vec_store<T, VW>(part + p * (LPR * VW), acc[p]);
+    if (lr.z > HUB_CHUNKS) return;  // hub_rows_kernel adds them up
     __threadfence();
     __syncwarp(gmask);
     int *tk = a.tickets + (int64_t)item.x * gridDim.y + blockIdx.y;
@@ -1472,6 +1538,27 @@ static size_t zero_prefix_bytes(const cgnn_plan *p, int64_t width) {
     return align_up((size_t)p->n_long * (size_t)ticket_tiles(width) * sizeof(int), 256);
 }
 
+// The engine for these operands (vec: rows of whole 16-byte vectors on 16-byte boundaries).
+template <typename T>
+static int launch_engine(const SegArgs<T> &a, bool vec, bool row_aligned, cudaStream_t stream) {
+    constexpr int VWMAX = 16 / (int)sizeof(T);
+    const T *src1 = a.src0 + a.delta_elems;
+    auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
+    const bool half = a.width * sizeof(T) % 8 == 0 && aligned8(a.src0) && aligned8(src1) && aligned8(a.seg_mask) &&
+                      aligned8(a.out);
+    if (!row_aligned) {  // two sources that are not a whole number of rows apart (never with a mask)
+        if (vec) return launch_vw<T, VWMAX, false, true>(a, stream);
+        return launch_unaligned<T, true>(a, half, stream);
+    }
+    if (vec) {
+        if (a.mask_src) return launch_vw<T, VWMAX, true, false>(a, stream);
+        return launch_vw<T, VWMAX, false, false>(a, stream);
+    }
+    if (a.mask_src) return launch_vw<T, 1, true, false>(a, stream);
+    if (a.width * (int64_t)sizeof(T) < 0x7fffffffll) return launch_unaligned<T, false>(a, half, stream);
+    return launch_vw<T, 1, false, false>(a, stream);
+}
+
 template <typename T>
 static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *src0, const T *src1,
                      const T *mask, const T *seg_mask, const int32_t *div_counts, T *out,
@@ -1518,19 +1605,12 @@ static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *s
     if (!accumulate && p->compact)
         CGNN_CUDA(cudaMemsetAsync(out, 0, (size_t)p->rows * (size_t)width * sizeof(T), stream));
     if (p->n_direct + p->n_items == 0) return CGNN_OK;
-    auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; };
-    const bool half = width * sizeof(T) % 8 == 0 && aligned8(src0) && aligned8(src1) && aligned8(seg_mask) && aligned8(out);
-    if (!row_aligned) {  // two sources that are not a whole number of rows apart (never with a mask)
-        if (vec) return launch_vw<T, VWMAX, false, true>(a, stream);
-        return launch_unaligned<T, true>(a, half, stream);
-    }
-    if (vec) {
-        if (mask) return launch_vw<T, VWMAX, true, false>(a, stream);
-        return launch_vw<T, VWMAX, false, false>(a, stream);
-    }
-    if (mask) return launch_vw<T, 1, true, false>(a, stream);
-    if (width * (int64_t)sizeof(T) < 0x7fffffffll) return launch_unaligned<T, false>(a, half, stream);
-    return launch_vw<T, 1, false, false>(a, stream);
+    const int rc = launch_engine<T>(a, vec, row_aligned, stream);
+    if (rc != CGNN_OK || p->degree_max <= (int64_t)HUB_CHUNKS * p->split) return rc;
+    const dim3 grid((unsigned)std::min<int64_t>(p->n_long, 148), (unsigned)std::min<int64_t>(ceil_div(width, 32), 65535));
+    hub_rows_kernel<T><<<grid, HUB_WARPS * 32, 0, stream>>>(a, (int)p->n_long);
+    CGNN_LAUNCH_CHECK();
+    return CGNN_OK;
 }
 
 static int run(const cgnn_plan *p, int dtype, int64_t width, const void *val, const void *src0,

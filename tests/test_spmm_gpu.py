@@ -100,6 +100,33 @@ def test_rows_by_their_aligned_cover(rt, widths, shift):
     test_rows_that_are_no_whole_vectors(rt, np.float32, widths, shift)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_rows_of_many_chunks(rt, dtype):
+    """Rows of up to 16 chunks are added up where their last chunk is made, longer ones by a launch of their own: around
+    that line and around whole batches of its loads (64 chunks)."""
+    rng = np.random.default_rng(8)
+    lengths = [3, 64 * 15, 64 * 16, 64 * 16 + 1, 5, 64 * 63 + 9, 64 * 64, 64 * 65, 20000] + [4] * 1000  # short: chunks of 64
+    rp = np.concatenate([[0], np.cumsum(lengths)])
+    col = rng.integers(0, 300, rp[-1])
+    val = rng.standard_normal(col.size)
+    weights = torch.zeros(len(lengths), 300, dtype=torch.float64)
+    weights.index_put_((torch.from_numpy(np.repeat(np.arange(len(lengths)), lengths)), torch.from_numpy(col)),
+                       torch.from_numpy(val).to(dtype).double(), accumulate=True)
+    for width in (1, 7, 16, 30, 47, 64, 66, 130, 256):
+        mat = torch.randn(300, width, device="cuda", dtype=dtype)
+        base = torch.randn(len(lengths), width, device="cuda", dtype=dtype)
+        args = cu(rp), cu(col), cu(val).to(dtype), mat
+        got = [rt.spmm_func(*args, "rowbalance_rowcache", None) for _ in range(2)]
+        assert torch.equal(*got)
+        want = weights.cuda() @ mat.double()
+        # any order of a row's additions: half an ulp of the magnitudes for each of them
+        magnitude = torch.from_numpy(np.add.reduceat(np.abs(val), rp[:-1])).cuda()[:, None] * mat.abs().max()
+        bound = torch.tensor(lengths, device="cuda")[:, None] * 0.5 * torch.finfo(dtype).eps * magnitude
+        assert bool(((got[0].double() - want).abs() <= bound).all()), width
+        added = rt.spmm_func(*args, "nnzbalance_parreduce", base.clone())
+        assert torch.equal(added, base + got[0]), width
+
+
 def test_accuracy_against_fp64(rt):
     """The fp32 CUDA result is as close to the exact (fp64) product as the reference's own
     fp32 loop is: error no larger than twice the CPU oracle's, row by row in max norm."""
