@@ -176,3 +176,25 @@ def test_loader_builds_the_same_graph_with_either_back_end():
                     pieces[backend] = [part for blk in g.blocks() for part in blk.csr()]
             assert len(pieces['cpu']) == len(pieces['cuda'])
             assert all(torch.equal(a, b) for a, b in zip(pieces['cpu'], pieces['cuda']))
+
+
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32])
+def test_staged_copies(dtype, monkeypatch):
+    """Arrays of less than a stage, whole stages, one element more or less, and enough parts to use each stage again; then
+    from several threads at once, each with a stream of its own."""
+    from concurrent.futures import ThreadPoolExecutor
+    from compressgnn_b200.loader import compression_backend as backend
+    monkeypatch.setattr(backend, "STAGE_BYTES", 1 << 16)
+    step = (1 << 16) // torch.empty((), dtype=dtype).element_size()
+
+    def both_ways(size):
+        host = torch.randint(-2**31, 2**31 - 1, (size,), dtype=dtype)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            there = backend._to_device(host)
+            back = backend._to_host(there)
+        return there.is_cuda and torch.equal(back, host)
+
+    sizes = [0, 1, step - 1, step, step + 1, 2 * step, 2 * step + 1, 7 * step - 1, 8 * step]
+    assert all(both_ways(size) for size in sizes)
+    with ThreadPoolExecutor(4) as pool:
+        assert all(pool.map(both_ways, sizes * 4))
