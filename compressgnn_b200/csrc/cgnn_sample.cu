@@ -23,9 +23,6 @@
 // graphs both orders below are the reference's, on deeper ones they are what its comments describe.
 #include <algorithm>
 #include <vector>
-#include <cub/cub.cuh>
-#include <thrust/iterator/counting_iterator.h>
-#include <thrust/iterator/transform_iterator.h>
 
 #include "cgnn_common.cuh"
 
@@ -224,24 +221,49 @@ __global__ void seed_kernel(const int64_t *samples, int64_t count, int64_t n, in
 //   * a slot's position counts over the whole batch (seeds first, then hop after hop), and first[v] keeps
 //     the smallest position that named vertex v -- earlier hops have smaller positions, so one
 //     table serves seeds and all hops and nothing is committed in between;
-//   * ONE scan per hop over the slots counts edges (high word) and new vertices (low word), started from the
-//     totals of the hop before it; its value at first[v] IS the local id of v;
+//   * edges and new vertices are numbered in two small launches: blocks of TILE slots number their own and leave their
+//     totals (hops_count_kernel), and the launch that writes the edges adds up the totals before each block, in
+//     shared memory, every block for itself (hops_relabel_kernel); the number at first[v] IS the local id of v;
 //   * a warp picks for one node: the children of up to 32 rules are listed per step, and the lookups of Floyd's
 //     draws run side by side.
-// A batch of 1024 seeds with fan-outs 25 and 10 on the 325 k-node graph: 131 us, hop by hop 505 (150 of them in the two
-// pick kernels).  Going hop by hop stays for batches whose slots would exceed MAX_POSITIONS.
+//   * a launch is scheduled while the one before it ends (hops_launch).
+// A batch of 1024 seeds with fan-outs 25 and 10 on the 325 k-node graph: 119 us; 131 with a library scan over the slots
+// in place of the numbering (three launches a hop where two do now, and none of them overlapping), hop by hop 505.  Going
+// hop by hop stays for batches whose slots would exceed MAX_POSITIONS.
 // ---------------------------------------------------------------------------------------
 constexpr int32_t EMPTY_SLOT = -1;  // picked[]: no pick here
 constexpr int32_t BAD_VERTEX = -2;  // picked[]: an edge to a vertex outside the graph (reported; local id 0)
 constexpr int64_t MAX_POSITIONS = 8 << 20;  // see cgnn_sample_hops_bytes
 
+// The launches of a batch follow one another at once: each opens the next one's scheduling when it starts and touches
+// memory only after the one before it is complete (hops_follow).
+__device__ __forceinline__ void hops_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void hops_follow() {
+    hops_open();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+static cudaError_t hops_launch(void (*kernel)(Params...), unsigned grid, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(THREADS);
+    config.stream = stream;
+    cudaLaunchAttribute follows = {};
+    follows.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    follows.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &follows;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // counts[h], h = 0 .. hops + 1: (edges << 32 | samples) before hop h - 1 has run; counts[0] = 0, counts[1] = the seeds
 __global__ void hops_begin_kernel(const int64_t *seeds, int64_t batch, int64_t n, int64_t *samples, int32_t *first,
-                                  uint64_t *prefix, uint64_t *counts) {
+                                  int32_t *ids, uint64_t *counts) {
+    hops_open();
     GRID_STRIDE(i, batch) {
         const int64_t v = seeds[i];
         samples[i] = v;
-        prefix[i] = (uint64_t)i;
+        ids[i] = (int32_t)i;
         if (v >= 0 && v < n) atomicMin(&first[v], (int32_t)i);  // a repeated seed keeps its first position
         else atomicOr(&g_sample_status, STATUS_BAD_INDEX);
         if (i == 0) {
@@ -295,6 +317,7 @@ __global__ void __launch_bounds__(THREADS) hops_pick_kernel(const GraphView g, c
                                                             int32_t *first) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (THREADS / 32);
+    hops_follow();
     const int64_t begin = (uint32_t)counts[0], end = (uint32_t)counts[1];
     for (int64_t i = (int64_t)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); i < nodes; i += warps) {
         int32_t *slots = picked + i * stride, *list = queue + i * stride;
@@ -371,31 +394,107 @@ __global__ void __launch_bounds__(THREADS) hops_pick_kernel(const GraphView g, c
     }
 }
 
-// What slot p of the hop adds to the totals: one edge (high word), one vertex (low word) if it is the first to name it.
-struct SlotCount {
+// The slots of a hop: an edge in each that is not empty, a new vertex in the first that names it.
+struct HopSlots {
     const int32_t *picked, *first;
-    int32_t base;
-    __device__ uint64_t operator()(int32_t p) const {
-        const int32_t v = picked[p];
-        if (v == EMPTY_SLOT) return 0;
-        return (1ull << 32) | (v >= 0 && first[v] == base + p ? 1ull : 0ull);
-    }
+    int64_t slots;
+    int32_t base;  // position of slot 0
+    __device__ bool is_new(int64_t p, int32_t v) const { return v >= 0 && first[v] == base + (int32_t)p; }
 };
-using SlotIterator = thrust::transform_iterator<SlotCount, thrust::counting_iterator<int32_t>, uint64_t, uint64_t>;
 
-__global__ void hops_relabel_kernel(SlotCount slot, int64_t slots, int32_t stride, const uint64_t *prefix, uint64_t *counts,
-                                    int32_t *rows, int32_t *cols, int64_t *samples) {
+constexpr int TILE_ROUNDS = 16;
+constexpr int TILE = THREADS * TILE_ROUNDS;  // slots a block numbers: 2048, so that two counts fit a word
+constexpr int MAX_TILES = (int)(MAX_POSITIONS / TILE);
+constexpr int TILES_PER_THREAD = MAX_TILES / THREADS;
+static_assert(MAX_TILES % THREADS == 0 && TILE < 1 << 15, "tiles are shared out evenly; counts are 16 bits each");
+
+// local[p] = edges before slot p in its tile (low half), new vertices before it (high half); totals[] of the tiles alike.
+__global__ void __launch_bounds__(THREADS) hops_count_kernel(const HopSlots hop, uint32_t *local, uint32_t *totals) {
+    constexpr int WARPS = THREADS / 32, CELLS = TILE_ROUNDS * WARPS;
+    static_assert(CELLS == 64, "a warp scans two cells a lane");
+    __shared__ uint32_t cells[CELLS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t tile0 = (int64_t)blockIdx.x * TILE;
+    hops_follow();
+    int32_t v[TILE_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        const int64_t p = tile0 + r * THREADS + threadIdx.x;
+        v[r] = p < hop.slots ? hop.picked[p] : EMPTY_SLOT;
+    }
+    uint32_t edges[TILE_ROUNDS], fresh[TILE_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        const int64_t p = tile0 + r * THREADS + threadIdx.x;
+        edges[r] = __ballot_sync(0xffffffffu, v[r] != EMPTY_SLOT);
+        fresh[r] = __ballot_sync(0xffffffffu, hop.is_new(p, v[r]));
+        if (lane == 0) cells[r * WARPS + warp] = (uint32_t)__popc(edges[r]) | (uint32_t)__popc(fresh[r]) << 16;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t low = cells[2 * lane], high = cells[2 * lane + 1];
+        int32_t sum;
+        const uint32_t before = (uint32_t)warp_exclusive((int32_t)(low + high), lane, &sum);
+        cells[2 * lane] = before;
+        cells[2 * lane + 1] = before + low;
+        if (lane == 0) totals[blockIdx.x] = (uint32_t)sum;
+    }
+    __syncthreads();
+    const uint32_t below = (1u << lane) - 1;
+#pragma unroll
+    for (int r = 0; r < TILE_ROUNDS; ++r) {
+        const int64_t p = tile0 + r * THREADS + threadIdx.x;
+        if (p < hop.slots)
+            local[p] = cells[r * WARPS + warp] + ((uint32_t)__popc(edges[r] & below) | (uint32_t)__popc(fresh[r] & below) << 16);
+    }
+}
+
+// Writes the hop's edges, its new vertices and their ids, and the totals after it.
+__global__ void __launch_bounds__(THREADS) hops_relabel_kernel(const HopSlots hop, int32_t stride, const uint32_t *local,
+                                                               const uint32_t *totals, int32_t tiles, uint64_t *counts,
+                                                               int32_t *ids, int32_t *rows, int32_t *cols,
+                                                               int64_t *samples) {
+    __shared__ uint64_t bases[MAX_TILES];  // (edges << 32 | samples) before each tile
+    __shared__ uint64_t warp_sums[THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    hops_follow();
+    auto widened = [](uint32_t c) { return (uint64_t)(c & 0xffffu) << 32 | (c >> 16); };
     const int32_t begin = (int32_t)(uint32_t)counts[0];
-    GRID_STRIDE(p, slots) {
-        const int32_t v = slot.picked[p];
-        const uint64_t here = prefix[slot.base + p], adds = slot((int32_t)p);
+    const int per_thread = (tiles + THREADS - 1) / THREADS;  // <= TILES_PER_THREAD
+    const int t0 = threadIdx.x * per_thread;
+    uint64_t sum = 0;
+    for (int t = t0; t < min(t0 + per_thread, tiles); ++t) sum += widened(totals[t]);
+    uint64_t upto = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t x = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += x;
+    }
+    if (lane == 31) warp_sums[warp] = upto;
+    __syncthreads();
+    uint64_t before = counts[1] + upto - sum;
+    for (int w = 0; w < warp; ++w) before += warp_sums[w];
+    for (int t = t0; t < min(t0 + per_thread, tiles); ++t) {
+        bases[t] = before;
+        before += widened(totals[t]);
+    }
+    if (blockIdx.x == 0 && t0 < tiles && t0 + per_thread >= tiles) counts[2] = before;  // the thread of the last tile
+    __syncthreads();
+    GRID_STRIDE(p, hop.slots) {
+        const int32_t v = hop.picked[p];
+        const uint64_t here = bases[p / TILE] + widened(local[p]);
+        ids[hop.base + p] = (int32_t)(uint32_t)here;  // what later hops find at first[v]
         if (v != EMPTY_SLOT) {
             const uint32_t edge = (uint32_t)(here >> 32);
             rows[edge] = begin + (int32_t)((uint32_t)p / (uint32_t)stride);
-            cols[edge] = v >= 0 ? (int32_t)(uint32_t)prefix[slot.first[v]] : 0;
-            if (adds & 1) samples[(uint32_t)here] = v;
+            int32_t id = 0;
+            if (v >= 0) {
+                const int32_t q = hop.first[v] - hop.base;
+                id = q < 0 ? ids[hop.base + q] : (int32_t)((uint32_t)bases[q / TILE] + (local[q] >> 16));
+                if (q == (int32_t)p) samples[(uint32_t)here] = v;
+            }
+            cols[edge] = id;
         }
-        if (p == slots - 1) counts[2] = here + adds;
     }
 }
 
@@ -414,16 +513,16 @@ __global__ void hops_finish_kernel(const int64_t *samples, const int32_t *rows, 
     }
 }
 
-// Slots of every hop and the layout of the workspace (the scan's scratch comes last).
+// Slots of every hop and the layout of the workspace.
 struct HopsLayout {
     std::vector<int64_t> nodes, stride;  // per hop: bound of the frontier, slots per node
     int64_t slots = 0, room = 0;         // all slots; bound of the samples
-    size_t counts = 0, samples = 0, prefix = 0, picked = 0, rows = 0, cols = 0, temp = 0, temp_bytes = 0, total = 0;
+    size_t counts = 0, samples = 0, ids = 0, picked = 0, rows = 0, cols = 0, local = 0, totals = 0, total = 0;
     bool fits = false;
 };
 
 static HopsLayout hops_layout(const cgnn_sample_graph *g, int64_t batch, int hops, const int64_t *fanouts,
-                              int64_t largest_degree, bool with_temp = true) {
+                              int64_t largest_degree) {
     HopsLayout L;
     if (batch > MAX_POSITIONS || g->vertices >= INT32_MAX || g->rules >= INT32_MAX || largest_degree >= INT32_MAX) return L;
     int64_t frontier = batch, most = 0;
@@ -440,10 +539,6 @@ static HopsLayout hops_layout(const cgnn_sample_graph *g, int64_t batch, int hop
         frontier = std::min(slots, g->vertices);
     }
     L.room = batch + std::min(L.slots, g->vertices);
-    if (most > 0 && with_temp)
-        cub::DeviceScan::ExclusiveScan(nullptr, L.temp_bytes, SlotIterator(thrust::counting_iterator<int32_t>(0), SlotCount{}),
-                                       (uint64_t *)nullptr, ::cuda::std::plus<>{},
-                                       cub::FutureValue<uint64_t>((uint64_t *)nullptr), (int)most);
     size_t used = 0;
     auto span = [&](size_t bytes) {
         const size_t at = used;
@@ -452,11 +547,12 @@ static HopsLayout hops_layout(const cgnn_sample_graph *g, int64_t batch, int hop
     };
     L.counts = span(((size_t)hops + 2) * 8);
     L.samples = span((size_t)L.room * 8);
-    L.prefix = span((size_t)(batch + L.slots) * 8);
+    L.ids = span((size_t)(batch + L.slots) * 4);
     L.picked = span((size_t)L.slots * 4);
     L.rows = span((size_t)L.slots * 4);
     L.cols = span((size_t)L.slots * 4);
-    L.temp = span(L.temp_bytes);
+    L.local = span((size_t)most * 4);
+    L.totals = span((size_t)ceil_div(most, TILE) * 4);
     L.total = used;
     L.fits = true;
     return L;
@@ -560,31 +656,30 @@ int cgnn_sample_hops(const cgnn_sample_graph *graph, const int64_t *seeds, int64
     CGNN_REQUIRE(L.fits && workspace_bytes >= L.total, "sample_hops: the workspace does not fit this batch");
     CGNN_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "sample_hops: workspace must be 256-byte aligned");
     char *base = reinterpret_cast<char *>(workspace);
-    uint64_t *counts = reinterpret_cast<uint64_t *>(base + L.counts), *prefix = reinterpret_cast<uint64_t *>(base + L.prefix);
+    uint64_t *counts = reinterpret_cast<uint64_t *>(base + L.counts);
+    int32_t *ids = reinterpret_cast<int32_t *>(base + L.ids);
+    uint32_t *local = reinterpret_cast<uint32_t *>(base + L.local), *totals = reinterpret_cast<uint32_t *>(base + L.totals);
     int64_t *samples = reinterpret_cast<int64_t *>(base + L.samples);
     int32_t *picked = reinterpret_cast<int32_t *>(base + L.picked), *rows = reinterpret_cast<int32_t *>(base + L.rows);
     int32_t *cols = reinterpret_cast<int32_t *>(base + L.cols);
     const GraphView view = view_of(graph);
-    hops_begin_kernel<<<blocks_for(batch), THREADS, 0, stream>>>(seeds, batch, graph->vertices, samples, first, prefix, counts);
+    hops_begin_kernel<<<blocks_for(batch), THREADS, 0, stream>>>(seeds, batch, graph->vertices, samples, first, ids, counts);
     CGNN_LAUNCH_CHECK();
     int64_t done = 0;  // slots of the hops before this one
     const int run = (int)L.nodes.size();
     for (int h = 0; h < run; ++h) {
         const int64_t nodes = L.nodes[h], stride = L.stride[h], slots = nodes * stride;
-        const SlotCount slot{picked + done, first, (int32_t)(batch + done)};
+        const HopSlots hop{picked + done, first, slots, (int32_t)(batch + done)};
+        const int32_t tiles = (int32_t)ceil_div(slots, TILE);
         // the rule lists use the slots' own part of `rows`: edges are written below it (edges <= slots so far)
         const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(nodes, THREADS / 32), 148 * 64);
-        hops_pick_kernel<<<grid, THREADS, 0, stream>>>(view, samples, counts + h, nodes, (int32_t)stride, fanouts[h],
-                                                       (uint32_t)h, seed, slot.base, picked + done, rows + done, first);
-        CGNN_LAUNCH_CHECK();
-        size_t temp_bytes = L.temp_bytes;
-        CGNN_CUDA(cub::DeviceScan::ExclusiveScan(base + L.temp, temp_bytes,
-                                                 SlotIterator(thrust::counting_iterator<int32_t>(0), slot),
-                                                 prefix + slot.base, ::cuda::std::plus<>{},
-                                                 cub::FutureValue<uint64_t>(counts + h + 1), (int)slots, stream));
-        hops_relabel_kernel<<<blocks_for(slots), THREADS, 0, stream>>>(slot, slots, (int32_t)stride, prefix, counts + h, rows,
-                                                                       cols, samples);
-        CGNN_LAUNCH_CHECK();
+        CGNN_CUDA(hops_launch(hops_pick_kernel, grid, stream, view, samples, counts + h, nodes, (int32_t)stride, fanouts[h],
+                              (uint32_t)h, seed, hop.base, picked + done, rows + done, first));
+        CGNN_CUDA(hops_launch(hops_count_kernel, (unsigned)tiles, stream, hop, local, totals));
+        // every block adds up all totals: no more blocks than run at once
+        const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(slots, THREADS), 148 * 6);
+        CGNN_CUDA(hops_launch(hops_relabel_kernel, blocks, stream, hop, (int32_t)stride, local, totals, tiles, counts + h, ids,
+                              rows, cols, samples));
         done += slots;
     }
     uint64_t last = 0;
@@ -599,7 +694,7 @@ int cgnn_sample_hops_result(const cgnn_sample_graph *graph, int64_t batch, int h
                             int64_t largest_degree, const int64_t sizes[2], int32_t *first, const void *workspace,
                             int64_t *samples_out, int64_t *rows_out, int64_t *cols_out, cgnn_stream_t stream) {
     CGNN_REQUIRE(graph && first && workspace && sizes && batch > 0, "sample_hops_result: null argument");
-    const HopsLayout L = hops_layout(graph, batch, hops, fanouts, largest_degree, false);
+    const HopsLayout L = hops_layout(graph, batch, hops, fanouts, largest_degree);
     CGNN_REQUIRE(L.fits && sizes[0] >= 0 && sizes[0] <= L.room && sizes[1] >= 0 && sizes[1] <= L.slots &&
                      samples_out != nullptr && (sizes[1] == 0 || (rows_out != nullptr && cols_out != nullptr)),
                  "sample_hops_result: the sizes do not fit this batch");

@@ -114,6 +114,19 @@ def test_all_hops_at_once_equal_hop_by_hop(fanouts):
     rt.raise_on_device_status()
 
 
+@pytest.mark.parametrize("batch, fanouts", [(2047, [1]), (2048, [1, 1]), (2049, [1, 2]), (1024, [2, 3]), (683, [3, 4]),
+                                            (54000, [5, 4]), (131072, [2]), (131073, [2, 2])])
+def test_slots_around_whole_tiles(batch, fanouts):
+    """2048 slots are numbered by one block, 128 tiles are added up one to a thread: around both, and some hundred tiles."""
+    from compressgnn_b200 import runtime as rt
+    graph = nested_graph().to("cuda")
+    sampler = graph.neighbor_sampler()
+    seeds = cu(np.random.default_rng(batch).choice(graph.vertex_cnt, size=batch, replace=True))
+    for mine, theirs in zip(sampler(seeds, fanouts, seed=5), sampler._hop_by_hop(seeds, fanouts, 5)):
+        assert torch.equal(mine, theirs)
+    rt.raise_on_device_status()
+
+
 def test_wide_fanouts_go_hop_by_hop():
     """A slot bound beyond the workspace limit takes the exact route; the answer is the same."""
     graph = nested_graph().to("cuda")
