@@ -1093,17 +1093,19 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 // 8-byte copies of rows on 8-byte boundaries by twice the copies.  Here a tile of a gathered row is copied by the ALIGNED
 // 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is short of that by the worst lead
 // (ragged_tile), so the cover always fits.  Where the row goes on behind the tile the whole cover is copied (each vector
-// holds bytes of the row); in the row's last tile nothing past its end is, and the first vector
+// holds bytes of the row); in the row's last tile (and the last stage of a unit) nothing past its end is, and the first vector
 // starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then reads units of
 // UNIT bytes -- 8 where every row begins on an 8-byte boundary, else 4 -- gl, gl + LPR, ... (consecutive words across the
 // lanes, no bank conflict) from the row's offset into the cover, which it gets by shuffle from the lane that
 // loaded the entry.  Lanes read what other lanes copied, hence the two __syncwarp per stage.
-// Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 320 with 8-byte copies, 295 here (the
+// Forward + backward at 40,000 nodes x 602 columns: 537 us in seg_kernel, 320 with 8-byte copies, 277 here (the
 // aligned engine at 604 columns takes the same number of tiles).  Segment sums of 7 columns (2,708 rows): 34 us in
 // seg_kernel, 10 here.
 // ---------------------------------------------------------------------------------------
-// Columns that LPR aligned vectors hold wherever a row begins: all but the unit's worst lead.
-__host__ __device__ constexpr int ragged_tile(int lpr, int unit) { return (lpr * 16 - (16 - unit)) / 4; }
+// Columns of a tile: what `lpr` aligned vectors hold wherever a row begins.  With 4-byte units that is one column more than
+// (lpr - 1) * 4, which would give every lane of a four-lane group a fourth element for it (width 1: 20.5 us a pass
+// against 22.2).
+__host__ __device__ constexpr int ragged_tile(int lpr, int unit) { return unit == 4 ? (lpr - 1) * 4 : lpr * 4 - 2; }
 // 16 bytes into shared memory of which the first min(left, 16) are read, the others zero.
 __device__ __forceinline__ void async_copy16_upto(uint32_t dst_shared, const void *src, int left) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_shared), "l"(src),
@@ -1142,7 +1144,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     const int row_bytes = (int)(width * (int64_t)sizeof(T));  // < 2^31: checked by the launcher
     const int64_t col0 = (int64_t)blockIdx.y * TILE;
     const int64_t colbase = col0 + gl * VW;
-    const bool inner = col0 + TILE < width;   // rows go on behind the tile: its whole cover may be read
+    const bool inner = LPR == 32 && col0 + TILE < width;  // rows go on behind the tile: its whole cover may be read
     const int tile_bytes = (int)min((int64_t)TILE, width - col0) * (int)sizeof(T);
     bool colok[VPL];
     V acc[VPL];
@@ -1218,9 +1220,10 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
         const uintptr_t at = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, lbase, rj, row_bytes)) & ~(uintptr_t)15;
         async_copy<16>(slot, reinterpret_cast<const void *>(at));
     };
-    auto copy_last = [&](uint32_t slot, int32_t rj) {  // nothing past the row's end
+    const int behind = tile_bytes - gl * 16;  // bytes of the tile behind this lane's first 16 * gl
+    auto copy_last = [&](uint32_t slot, int32_t rj) {  // nothing past the tile's end
         const uintptr_t row = reinterpret_cast<uintptr_t>(gathered_row<FAR>(a, lbase, rj, row_bytes));
-        const int left = tile_bytes - gl * 16 + (int)(row & 15);
+        const int left = behind + (int)(row & 15);
         if (left > 0) async_copy16_upto(slot, reinterpret_cast<const void *>(row & ~(uintptr_t)15), left);
     };
     auto issue = [&](int b) {
@@ -1235,17 +1238,19 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
             const int cnt = n_ent - first;  // >= 1
             const uint32_t stage = ring + (uint32_t)((b % S) * K) * SLOT + lane * 16;
             const int pos = (first & 31) + gk;
-            if (cnt >= KE && inner) {
+            if (cnt >= KE) {
+                if (inner) {
 #pragma unroll
-                for (int j = 0; j < K; ++j) copy_inner(stage + (uint32_t)(j * SLOT), __shfl_sync(FULL, o, pos + j * G));
+                    for (int j = 0; j < K; ++j) copy_inner(stage + (uint32_t)(j * SLOT), __shfl_sync(FULL, o, pos + j * G));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < K; ++j) copy_last(stage + (uint32_t)(j * SLOT), __shfl_sync(FULL, o, pos + j * G));
+                }
             } else {
 #pragma unroll
                 for (int j = 0; j < K; ++j) {
                     const int32_t rj = __shfl_sync(FULL, o, (pos + j * G) & 31);
-                    if (j * G + gk < cnt) {
-                        if (inner) copy_inner(stage + (uint32_t)(j * SLOT), rj);
-                        else copy_last(stage + (uint32_t)(j * SLOT), rj);
-                    }
+                    if (j * G + gk < cnt) copy_last(stage + (uint32_t)(j * SLOT), rj);
                 }
             }
         }

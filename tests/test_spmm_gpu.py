@@ -95,8 +95,8 @@ def test_rows_that_are_no_whole_vectors(rt, dtype, widths, shift):
 @pytest.mark.parametrize("widths", [(2, 6, 10, 14, 18, 22, 26, 30, 34, 58, 62, 66, 122, 126, 130, 250, 252, 254, 378),
                                     (8, 12, 16, 28, 32, 60, 64, 124, 128, 13, 14, 29, 30, 61, 62, 125, 126, 127, 250)])
 def test_rows_by_their_aligned_cover(rt, widths, shift):
-    """Edges of the tiles whose rows begin on 8-byte boundaries (14, 30, 62, 126 columns) and on 4-byte ones (13, 29, 61,
-    125), the matrices themselves beginning 0, 4 and 8 bytes past a 16-byte boundary."""
+    """Edges of the tiles whose rows begin on 8-byte boundaries (14, 30, 62, 126 columns) and on 4-byte ones (12, 28, 60,
+    124), the matrices themselves beginning 0, 4 and 8 bytes past a 16-byte boundary."""
     test_rows_that_are_no_whole_vectors(rt, np.float32, widths, shift)
 
 
