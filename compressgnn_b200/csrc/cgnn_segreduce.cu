@@ -7,7 +7,8 @@
 //     load, the next window requested before the current one is consumed;
 //   * rows longer than `split` are cut into chunks (work units of their own); a chunk writes its
 //     partial sum to scratch, takes a ticket, and the chunk that draws the last ticket adds the
-//     partials in chunk order -- deterministic, no float atomics, and no unit ever waits for another;
+//     partials in chunk order -- deterministic, no float atomics, and no unit ever waits for another; the
+//     partials of rows of very many chunks are added up by a second launch (hub_rows_kernel);
 //   * the gather engines share that decomposition and its row order; on rows of more than 16 vectors they produce the
 //     same bits (narrower rows share a step among lane groups, whose sums meet in a fixed tree):
 //       seg_async_kernel  gathered rows staged through shared memory by 16-byte cp.async copies, one
