@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "cgnn_colsum.cuh"
+#include "cgnn_cover.h"
 #include "cgnn_plan.h"
 
 // Build-time tuning knobs (the defaults are the measured best on B200).
@@ -1093,8 +1094,8 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 // the same cp.async engine with one shift.  seg_kernel is bound by instructions and loads in flight on such rows, and
 // 8-byte copies of rows on 8-byte boundaries by twice the copies.  Here a tile of a gathered row is copied by the ALIGNED
 // 16-byte vectors that cover it, wherever the row begins, LPR of them; a tile is short of that by the worst lead
-// (ragged_tile), so the cover always fits.  Where the row goes on behind the tile the whole cover is copied (each vector
-// holds bytes of the row); in the row's last tile (and the last stage of a unit) nothing past its end is, and the first vector
+// (ragged_tile), so the cover always fits.  Where the row holds the whole cover, wherever it begins, all of it is copied
+// (ragged_whole_cover); elsewhere (and in the last stage of a unit) nothing past the tile's end is.  The first vector
 // starts at most 12 bytes early, inside the aligned 16 bytes its first element lies in.  A lane then reads units of
 // UNIT bytes -- 8 where every row begins on an 8-byte boundary, else 4 -- gl, gl + LPR, ... (consecutive words across the
 // lanes, no bank conflict) from the row's offset into the cover, which it gets by shuffle from the lane that
@@ -1103,10 +1104,6 @@ __global__ void __launch_bounds__(32) seg_async_kernel(const SegArgs<T> a) {
 // aligned engine at 604 columns takes the same number of tiles).  Segment sums of 7 columns (2,708 rows): 34 us in
 // seg_kernel, 10 here.
 // ---------------------------------------------------------------------------------------
-// Columns of a tile: what `lpr` aligned vectors hold wherever a row begins.  With 4-byte units that is one column more than
-// (lpr - 1) * 4, which would give every lane of a four-lane group a fourth element for it (width 1: 20.5 us a pass
-// against 22.2).
-__host__ __device__ constexpr int ragged_tile(int lpr, int unit) { return unit == 4 ? (lpr - 1) * 4 : lpr * 4 - 2; }
 // 16 bytes into shared memory of which the first min(left, 16) are read, the others zero.
 __device__ __forceinline__ void async_copy16_upto(uint32_t dst_shared, const void *src, int left) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_shared), "l"(src),
@@ -1145,7 +1142,7 @@ __global__ void __launch_bounds__(32) seg_ragged_kernel(const SegArgs<float> a) 
     const int row_bytes = (int)(width * (int64_t)sizeof(T));  // < 2^31: checked by the launcher
     const int64_t col0 = (int64_t)blockIdx.y * TILE;
     const int64_t colbase = col0 + gl * VW;
-    const bool inner = LPR == 32 && col0 + TILE < width;  // rows go on behind the tile: its whole cover may be read
+    const bool inner = LPR == 32 && ragged_whole_cover(LPR, width, col0);  // (fewer lanes hold the row in one tile)
     const int tile_bytes = (int)min((int64_t)TILE, width - col0) * (int)sizeof(T);
     bool colok[VPL];
     V acc[VPL];

@@ -100,7 +100,9 @@ size_t cgnn_plan_ticket_bytes(const cgnn_plan *plan, int64_t width, int dtype);
  * ref: spmm_func, src/runtime/csrc/sparse/spmm.cpp:11-23 and
  *      src/runtime/csrc/sparse/cuda/spmm_gpu.cu:8-107 (all six kernel variants).
  * val holds the entry values IN PLAN ORDER (cgnn_plan_permute_values) or is NULL (all
- * ones).  accumulate != 0 adds to the existing out (the reference's
+ * ones).  Of `src` only the rows named by the entries are read, and behind a row nothing; a row that
+ * begins off a 16-byte boundary is read from that boundary on, up to 12 bytes before its first
+ * element, which no result depends on.  accumulate != 0 adds to the existing out (the reference's
  * optional_out contract); out may alias src when the rows written are never read (the
  * in-place rule-level updates of ref: layer/CompressgnnSPMM.py:57-58).
  * ------------------------------------------------------------------------------------- */
