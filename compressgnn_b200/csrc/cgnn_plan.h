@@ -1,6 +1,8 @@
 // Internal definition of the opaque cgnn_plan and the helpers shared between translation
 // units (the public contract is include/cgnn_b200.h).
 #pragma once
+#include <mutex>
+
 #include "cgnn_common.cuh"
 
 // A plan owns a re-laid-out copy of the block's (or the two fused blocks') entries:
@@ -33,6 +35,7 @@ struct cgnn_plan {
     void *block = nullptr;         // the one device allocation all arrays above live in
     cudaStream_t home = nullptr;   // stream the block was allocated on (stream-ordered allocator)
     bool pooled = false;           // block came from cudaMallocAsync
+    mutable std::mutex two_launches;  // held over launches that hand each other partial sums in the scratch
 };
 
 namespace cgnn {

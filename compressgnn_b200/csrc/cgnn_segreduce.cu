@@ -1608,8 +1608,11 @@ static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *s
     if (!accumulate && p->compact)
         CGNN_CUDA(cudaMemsetAsync(out, 0, (size_t)p->rows * (size_t)width * sizeof(T), stream));
     if (p->n_direct + p->n_items == 0) return CGNN_OK;
+    if (p->degree_max <= (int64_t)HUB_CHUNKS * p->split) return launch_engine<T>(a, vec, row_aligned, stream);
+    // Two launches that meet in the scratch: no other launch of this plan may come between them on the stream.
+    std::lock_guard<std::mutex> together(p->two_launches);
     const int rc = launch_engine<T>(a, vec, row_aligned, stream);
-    if (rc != CGNN_OK || p->degree_max <= (int64_t)HUB_CHUNKS * p->split) return rc;
+    if (rc != CGNN_OK) return rc;
     const dim3 grid((unsigned)std::min<int64_t>(p->n_long, 148), (unsigned)std::min<int64_t>(ceil_div(width, 32), 65535));
     hub_rows_kernel<T><<<grid, HUB_WARPS * 32, 0, stream>>>(a, (int)p->n_long);
     CGNN_LAUNCH_CHECK();

@@ -42,7 +42,9 @@ int cgnn_device_status(int *status_out);
  * two blocks over the same rows whose sums are fused), cut into work units by the row
  * degree histogram: rows up to `split` entries are owned by one lane group; longer rows
  * are cut into chunks of `split` entries whose partial sums are combined in chunk order
- * by the last chunk to finish (deterministic; no floating-point atomics).
+ * by the last chunk to finish, or, for rows of very many chunks, in eight interleaved sums by a second
+ * launch (deterministic; no floating-point atomics).  Both launches use the scratch: threads that launch one plan on
+ * one stream are kept apart by the plan.
  * ------------------------------------------------------------------------------------- */
 typedef struct cgnn_plan cgnn_plan;
 

@@ -127,6 +127,25 @@ def test_rows_of_many_chunks(rt, dtype):
         assert torch.equal(added, base + got[0]), width
 
 
+def test_threads_share_a_plan_on_one_stream(rt):
+    """Launches of two threads on one stream, rows of many chunks: every call's partial sums are its own although
+    the plan's scratch is one, so each thread gets the bits it gets alone."""
+    from concurrent.futures import ThreadPoolExecutor
+    rng = np.random.default_rng(12)
+    lengths = np.array([64 * 40, 5, 64 * 33 + 3, 64 * 90] + [6] * 200)
+    rp, col = np.concatenate([[0], np.cumsum(lengths)]), rng.integers(0, 300, lengths.sum())
+    graph = cu(rp), cu(col), cu(rng.standard_normal(col.size).astype(np.float32))
+    mats = [torch.randn(300, 128, device="cuda") for _ in range(2)]
+    alone = [rt.spmm_func(*graph, mat, "rowbalance_rowcache", None) for mat in mats]
+
+    def same(which):
+        got = [rt.spmm_func(*graph, mats[which], "rowbalance_rowcache", None) for _ in range(200)]
+        return all(torch.equal(g, alone[which]) for g in got)
+
+    with ThreadPoolExecutor(2) as pool:
+        assert all(pool.map(same, range(2)))
+
+
 def test_accuracy_against_fp64(rt):
     """The fp32 CUDA result is as close to the exact (fp64) product as the reference's own
     fp32 loop is: error no larger than twice the CPU oracle's, row by row in max norm."""
