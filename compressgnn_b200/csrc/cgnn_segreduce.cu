@@ -8,7 +8,7 @@
 //   * rows longer than `split` are cut into chunks (work units of their own); a chunk writes its
 //     partial sum to scratch, takes a ticket, and the chunk that draws the last ticket adds the
 //     partials in chunk order -- deterministic, no float atomics, and no unit ever waits for another; the
-//     partials of rows of very many chunks are added up by a second launch (hub_rows_kernel);
+//     partials of rows of more than HUB_CHUNKS chunks are added up by a second launch (hub_rows_kernel);
 //   * the gather engines share that decomposition and its row order; on rows of more than 16 vectors they produce the
 //     same bits (narrower rows share a step among lane groups, whose sums meet in a fixed tree):
 //       seg_async_kernel  gathered rows staged through shared memory by 16-byte cp.async copies, one
@@ -134,8 +134,8 @@ struct SegArgs {
 // stream serialization: once every block of the launch before it has started (chain_open), its blocks
 // are scheduled as that one's finish, read the plan -- which was complete before the pass began -- and
 // wait (chain_wait) until the launch before has completed and its writes are visible.  A launch whose follower
-// is not ours opens nothing.  Without and with the overlap: forward + backward at 2,708 nodes x 16
-// 65.1 and 61.5 us; 40,000 x 128 in fp64 120.5 and 108.7; forward at 325 k x 64 107.8 and 102.9; no difference beyond
+// is not ours opens nothing; the launch that adds up hub rows (hub_rows_kernel) is a link of the chain like
+// the others.  Without and with the overlap: forward + backward at 2,708 nodes x 16 65.1 and 61.5 us; 40,000 x 128 in fp64 120.5 and 108.7; forward at 325 k x 64 107.8 and 102.9; no difference beyond
 // noise at 325 k x 256.
 enum { CHAIN_FOLLOWS = 1, CHAIN_LEADS = 2 };
 template <typename T>
@@ -144,12 +144,12 @@ __device__ __forceinline__ void chain_open(const SegArgs<T> &a) {
 }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <typename T>
-static cudaError_t launch_chained(void (*kernel)(const SegArgs<T>), dim3 grid, size_t shared_bytes, const SegArgs<T> &a,
-                                  cudaStream_t stream) {
+template <typename T, typename... More>
+static cudaError_t launch_chained(void (*kernel)(const SegArgs<T>, More...), dim3 grid, size_t shared_bytes, const SegArgs<T> &a,
+                                  cudaStream_t stream, int threads = 32, More... more) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
-    config.blockDim = dim3(32);
+    config.blockDim = dim3((unsigned)threads);
     config.dynamicSmemBytes = shared_bytes;
     config.stream = stream;
     cudaLaunchAttribute follows = {};
@@ -157,7 +157,7 @@ static cudaError_t launch_chained(void (*kernel)(const SegArgs<T>), dim3 grid, s
     follows.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &follows;
     config.numAttrs = a.chain & CHAIN_FOLLOWS ? 1 : 0;
-    return cudaLaunchKernelEx(&config, kernel, a);
+    return cudaLaunchKernelEx(&config, kernel, a, more...);
 }
 
 // Source-row index of an entry relative to src0.  Entries of the second block (bit 31 set)
@@ -278,16 +278,23 @@ __device__ __forceinline__ void finish_row(const SegArgs<T> &a, int32_t row, int
 
 // Rows of more chunks than this ("hubs") are added up by a launch of their own (hub_rows_kernel).  A bucket of an
 // assignment may hold a large part of all rows (48 k of 325 k: 379 chunks), and one warp that adds so many
-// partial rows one after the other is a chain longer than the launch; up to 16 it is hidden by the launch's other
-// work, and a second launch (2 us) is not.
-constexpr int HUB_CHUNKS = 16;
+// partial rows one after the other is a chain longer than the launch.  A second launch costs 2.6 us of host time, and up to
+// some 32 chunks the first one's other work hides most of the chain.  us in one launch and in two, by chunks a row:
+//   bucket means x 128 columns, 16 buckets:  17: 17.2, 16.4   32: 19.3, 15.9   64: 25.3, 17.0   128: 43.9, 28.7
+//                             512 buckets:   17: 93, 95       24: 126, 128     32: 165, 165
+//                             1024 buckets:  17: 175, 180
+//   x 16 columns, 16 buckets (host-bound):   17: 13.4, 15.8   48: 15.2, 15.9   64: 17.6, 16.4   96: 22.4, 16.1
+//   forward + backward of 100 k nodes x 64, four hubs:        24: 89, 92       469: 111, 100
+constexpr int HUB_CHUNKS = 32;
 
 // The hub rows: block x looks at every gridDim.x-th long row, a lane per column of a 32-column tile, eight warps that
 // add every eighth partial row with eight loads in flight, the warps' sums in warp order.  The same order whichever
 // engine made the partial sums.  What bounds it is the latency of n_chunks / 64 dependent batches of loads.
 // Bucket mean of 325 k rows x 128 with buckets of 48 k, 21 k and 13 k: 146 us in one launch, 37 + 14 in two; 47
-// columns of reconstruct backward 108 and 25 + 12.
+// columns of reconstruct backward 108 and 25 + 12.  300 hubs of 64 chunks x 64 columns: 35.5 us with 148 blocks to a
+// column tile, 31.4 with four times as many.
 constexpr int HUB_WARPS = 8;
+constexpr int HUB_BLOCKS = 148 * 4;
 constexpr int HUB_UNROLL = 8;
 template <typename T>
 __global__ void __launch_bounds__(HUB_WARPS * 32) hub_rows_kernel(const SegArgs<T> a, int n_long) {
@@ -295,6 +302,8 @@ __global__ void __launch_bounds__(HUB_WARPS * 32) hub_rows_kernel(const SegArgs<
     __shared__ int n_hubs;
     __shared__ T sums[HUB_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    chain_open(a);
+    chain_wait();
     for (int64_t base = blockIdx.x; base < n_long; base += (int64_t)gridDim.x * blockDim.x) {
         if (threadIdx.x == 0) n_hubs = 0;
         __syncthreads();
@@ -1611,11 +1620,12 @@ static int run_typed(const cgnn_plan *p, int64_t width, const T *val, const T *s
     if (p->degree_max <= (int64_t)HUB_CHUNKS * p->split) return launch_engine<T>(a, vec, row_aligned, stream);
     // Two launches that meet in the scratch: no other launch of this plan may come between them on the stream.
     std::lock_guard<std::mutex> together(p->two_launches);
+    a.chain |= CHAIN_LEADS;
     const int rc = launch_engine<T>(a, vec, row_aligned, stream);
     if (rc != CGNN_OK) return rc;
-    const dim3 grid((unsigned)std::min<int64_t>(p->n_long, 148), (unsigned)std::min<int64_t>(ceil_div(width, 32), 65535));
-    hub_rows_kernel<T><<<grid, HUB_WARPS * 32, 0, stream>>>(a, (int)p->n_long);
-    CGNN_LAUNCH_CHECK();
+    a.chain = CHAIN_FOLLOWS | (chain & CHAIN_LEADS);
+    const dim3 grid((unsigned)std::min<int64_t>(p->n_long, HUB_BLOCKS), (unsigned)std::min<int64_t>(ceil_div(width, 32), 65535));
+    CGNN_CUDA(launch_chained(hub_rows_kernel<T>, grid, 0, a, stream, HUB_WARPS * 32, (int)p->n_long));
     return CGNN_OK;
 }
 

@@ -261,6 +261,44 @@ def test_bucket_plan_of_the_device_equals_the_host_one(rt, n, bits, shape):
     assert torch.equal(rt.cluster_mean(x, ids, counts, plan=mine), rt.cluster_mean(x, ids, counts, plan=host))
 
 
+@pytest.mark.parametrize("width", [16, 47, 66, 128, 256])
+def test_buckets_of_many_chunks(rt, width):
+    """A bucket of several hundred chunks, one just above 32, one of 32 and many small ones: the mean, and the reconstruct backward without a
+    mask, with a mask row per node and with one per bucket (the last two bit for bit alike), through a plan built on the
+    device, against float64 sums; the bound is that of any order of a bucket's additions."""
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    n, bits = 60000, 12
+    codes = torch.randint(0, 2 ** bits, (n,), device="cuda", generator=gen).int()
+    codes[: 48000] = 5
+    codes[48000: 48000 + 32 * 64 + 1] = 9
+    codes[51000: 51000 + 32 * 64 - 20] = 7
+    workspace = rt.cluster_workspace(torch.empty(n, 1, device="cuda"), bits)
+    ids, counts, active = rt._assign_from_codes(codes, n, bits, workspace, codes.device)
+    groups = active + 1
+    assert rt.index_plan(ids, groups).degree_max > 64 * 128
+    eps = 0.5 * torch.finfo(torch.float32).eps * (1 + 1e-3)
+
+    def sums(rows):
+        return torch.zeros(groups, width, device="cuda", dtype=torch.float64).index_add_(0, ids, rows.double())
+
+    x = torch.randn(n, width, device="cuda", generator=gen)
+    members = counts.double().clamp(min=1)[:, None]
+    mean = rt.cluster_mean(x, ids, counts)
+    bound = (members + 1) * eps * sums(x.abs()) / members
+    assert bool(((mean.double() - sums(x) / members).abs() <= bound).all())
+    output = torch.randn(groups, width, device="cuda", generator=gen)[ids]
+    plain, exact, fast = (rt.cluster_reconstruct_backward(x, ids, output, groups, relu, output_is_forward_result=per_bucket)
+                          for relu, per_bucket in ((False, False), (True, False), (True, True)))
+    assert torch.equal(exact, fast)
+    captured = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(captured):
+        again = rt.cluster_mean(x, ids, counts)
+    captured.replay()
+    assert torch.equal(again, mean)
+    for got, kept in ((plain, x), (exact, x * (output > 0))):
+        assert bool(((got.double() - sums(kept)).abs() <= members * eps * sums(kept.abs())).all())
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_expanded_rows_of_no_whole_vectors(rt, dtype):
     """The row-block form of the reconstruction: widths whose vectors cross rows at every offset, on both sides of the
