@@ -2483,6 +2483,7 @@ int cgnn_cluster_reconstruct_backward(const cgnn_plan *plan, int dtype, int64_t 
     CGNN_REQUIRE(scratch != nullptr && scratch_bytes >= cgnn_plan_scratch_bytes(plan, width, dtype),
                  "reconstruct_backward: scratch too small for the bias gradient");
     void *part = reinterpret_cast<char *>(scratch) + off;
+    std::lock_guard<std::mutex> together(plan->two_launches);  // its two stages meet in the scratch
     if (dtype == CGNN_F32)
         return colsum<float>((const float *)d_reps, plan->rows, width, (float *)part,
                              (float *)bias_grad, (cudaStream_t)stream);

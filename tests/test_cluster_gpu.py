@@ -261,6 +261,20 @@ def test_bucket_plan_of_the_device_equals_the_host_one(rt, n, bits, shape):
     assert torch.equal(rt.cluster_mean(x, ids, counts, plan=mine), rt.cluster_mean(x, ids, counts, plan=host))
 
 
+def test_bias_gradients_of_two_threads(rt):
+    """Two threads, one plan, one stream: the column sums meet in the plan's scratch, each thread gets its own."""
+    from concurrent.futures import ThreadPoolExecutor
+    ids = torch.arange(9000, device="cuda") % 3000
+    grads = [torch.randn(9000, 48, device="cuda") for _ in range(2)]
+
+    def sums(which):
+        return rt.cluster_reconstruct_backward(grads[which], ids, grads[which], 3000, False, return_bias_grad=True)[1]
+
+    alone = [sums(which) for which in range(2)]
+    with ThreadPoolExecutor(2) as pool:
+        assert all(pool.map(lambda which: all(torch.equal(sums(which), alone[which]) for _ in range(200)), range(2)))
+
+
 @pytest.mark.parametrize("width", [16, 47, 66, 128, 256])
 def test_buckets_of_many_chunks(rt, width):
     """A bucket of several hundred chunks, one just above 32, one of 32 and many small ones: the mean, and the reconstruct backward without a
