@@ -37,7 +37,8 @@ def resolve_backend(backend):
 # A copy between pageable host memory and the device goes through the driver's own stage at about 11 GB/s, one host
 # thread moving the bytes (27 MB of edges: 2.6 ms).  In parts through two page-locked stages the host side of a part is
 # done by torch's threads while the part before it is on the link.  The stages are torch's, which
-# keeps page-locked memory of this size for the next caller; up to one part the plain copy is as fast.
+# keeps page-locked memory of this size for the next caller; up to one part the plain copy is as fast, and where there
+# is no page-locked memory to be had it takes all.
 STAGE_BYTES = 4 << 20
 
 
@@ -47,17 +48,24 @@ def _parts(tensor):
 
 
 def _stages(tensor):
+    """Two page-locked stages, or None for the plain copy."""
     import torch
-    return [(torch.empty(STAGE_BYTES // tensor.element_size(), dtype=tensor.dtype, pin_memory=True), torch.cuda.Event())
-            for _ in range(2)]
+    if tensor.nbytes <= STAGE_BYTES:
+        return None
+    step = STAGE_BYTES // tensor.element_size()
+    try:
+        return [(torch.empty(step, dtype=tensor.dtype, device="cpu", pin_memory=True), torch.cuda.Event()) for _ in range(2)]
+    except RuntimeError:
+        return None
 
 
 def _to_device(host):
     """One-dimensional host tensor on the current device."""
     import torch
-    if host.nbytes <= STAGE_BYTES:
+    stages = _stages(host)
+    if stages is None:
         return host.cuda()
-    out, stages = torch.empty_like(host, device="cuda"), _stages(host)
+    out = torch.empty_like(host, device="cuda")
     for i, part in enumerate(_parts(host)):
         stage, sent = stages[i % 2]
         sent.synchronize()  # (an event not recorded yet is complete)
@@ -71,9 +79,10 @@ def _to_device(host):
 def _to_host(device):
     """One-dimensional device tensor in pageable host memory, complete on return."""
     import torch
-    if device.nbytes <= STAGE_BYTES:
+    stages = _stages(device)
+    if stages is None:
         return device.cpu()
-    out, stages, parts = torch.empty(device.shape, dtype=device.dtype), _stages(device), _parts(device)
+    out, parts = torch.empty(device.shape, dtype=device.dtype, device="cpu"), _parts(device)
     for i in range(len(parts) + 1):
         if i < len(parts):
             stage, arrived = stages[i % 2]

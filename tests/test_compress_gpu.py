@@ -198,3 +198,34 @@ def test_staged_copies(dtype, monkeypatch):
     assert all(both_ways(size) for size in sizes)
     with ThreadPoolExecutor(4) as pool:
         assert all(pool.map(both_ways, sizes * 4))
+
+
+def test_staged_copies_with_a_default_device(monkeypatch):
+    """The stages and the result lie in host memory whatever torch's default device is."""
+    from compressgnn_b200.loader import compression_backend as backend
+    vlist = np.arange(0, 40001, 4)
+    elist = np.random.default_rng(3).integers(0, 1000, 40000)
+    want = backend.compress_graph_csr(vlist, elist, 4, backend="cuda")
+    monkeypatch.setattr(backend, "STAGE_BYTES", 1 << 14)
+    with torch.device("cuda"):
+        got = backend.compress_graph_csr(vlist, elist, 4, backend="cuda")
+    assert got[2:] == want[2:] and all(np.array_equal(g, w) for g, w in zip(got[:2], want[:2]))
+
+
+def test_copies_without_page_locked_memory(monkeypatch):
+    """Where the system has no page-locked memory to give, the arrays are copied without stages."""
+    from compressgnn_b200.loader import compression_backend as backend
+    vlist = np.arange(0, 40001, 4)
+    elist = np.random.default_rng(4).integers(0, 1000, 40000)
+    want = backend.compress_graph_csr(vlist, elist, 4, backend="cuda")
+    empty = torch.empty
+
+    def refuses(*args, **kwargs):
+        if kwargs.get("pin_memory"):
+            raise RuntimeError("CUDA error: out of memory")
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(backend, "STAGE_BYTES", 1 << 14)
+    monkeypatch.setattr(torch, "empty", refuses)
+    got = backend.compress_graph_csr(vlist, elist, 4, backend="cuda")
+    assert got[2:] == want[2:] and all(np.array_equal(g, w) for g, w in zip(got[:2], want[:2]))
