@@ -405,7 +405,6 @@ struct HopSlots {
 constexpr int TILE_ROUNDS = 16;
 constexpr int TILE = THREADS * TILE_ROUNDS;  // slots a block numbers: 2048, so that two counts fit a word
 constexpr int MAX_TILES = (int)(MAX_POSITIONS / TILE);
-constexpr int TILES_PER_THREAD = MAX_TILES / THREADS;
 static_assert(MAX_TILES % THREADS == 0 && TILE < 1 << 15, "tiles are shared out evenly; counts are 16 bits each");
 
 // local[p] = edges before slot p in its tile (low half), new vertices before it (high half); totals[] of the tiles alike.
@@ -460,7 +459,7 @@ __global__ void __launch_bounds__(THREADS) hops_relabel_kernel(const HopSlots ho
     hops_follow();
     auto widened = [](uint32_t c) { return (uint64_t)(c & 0xffffu) << 32 | (c >> 16); };
     const int32_t begin = (int32_t)(uint32_t)counts[0];
-    const int per_thread = (tiles + THREADS - 1) / THREADS;  // <= TILES_PER_THREAD
+    const int per_thread = (tiles + THREADS - 1) / THREADS;
     const int t0 = threadIdx.x * per_thread;
     uint64_t sum = 0;
     for (int t = t0; t < min(t0 + per_thread, tiles); ++t) sum += widened(totals[t]);

@@ -127,6 +127,25 @@ def test_slots_around_whole_tiles(batch, fanouts):
     rt.raise_on_device_status()
 
 
+@pytest.mark.parametrize("fanout", [1, 2, 10 ** 6])
+def test_slots_up_to_the_limit(fanout):
+    """The most slots that are numbered all at once (2048, 2731 and nearly 4096 tiles of them) and one seed more, which goes
+    hop by hop."""
+    import ctypes
+    from compressgnn_b200 import runtime as rt
+    from compressgnn_b200._lib import lib
+    sampler = nested_graph().to("cuda").neighbor_sampler()
+    most = (8 << 20) // (min(fanout, sampler._largest_degree) + 1)
+    seeds = torch.randint(0, sampler.vertices, (most + 1,), device="cuda", generator=torch.Generator("cuda").manual_seed(fanout))
+    for batch in (most, most + 1):
+        room = lib().cgnn_sample_hops_bytes(ctypes.byref(sampler._graph), batch, 1, (ctypes.c_int64 * 1)(fanout),
+                                            sampler._largest_degree)
+        assert (room > 0) == (batch == most)
+        for mine, theirs in zip(sampler(seeds[:batch], [fanout], seed=6), sampler._hop_by_hop(seeds[:batch], [fanout], 6)):
+            assert torch.equal(mine, theirs)
+    rt.raise_on_device_status()
+
+
 def test_wide_fanouts_go_hop_by_hop():
     """A slot bound beyond the workspace limit takes the exact route; the answer is the same."""
     graph = nested_graph().to("cuda")
