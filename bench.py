@@ -54,7 +54,7 @@ WORKLOADS = {
 COMPRESS = dict(min_pair_frequency=4, threshold=4, max_depth=3, min_edge=1000000)
 TRAFFIC_RECORD = ROOT / "profiles" / "ncu_traffic.json"
 KERNEL_SOURCES = ("compressgnn_b200/csrc/cgnn_segreduce.cu", "compressgnn_b200/csrc/cgnn_common.cuh",
-                  "compressgnn_b200/csrc/cgnn_plan.h")
+                  "compressgnn_b200/csrc/cgnn_plan.h", "compressgnn_b200/csrc/cgnn_cover.h")
 
 
 def kernel_source_hash():

@@ -70,7 +70,8 @@ auto complete(int device, Fill &&fill) {
 }
 
 // Owner of a native plan and of its scratch: one zero-initialised buffer per (width, dtype, stream), since
-// a launch leaves the ticket words zero and launches on one stream are ordered.
+// a launch leaves the ticket words zero, launches on one stream are ordered, and those that hand each other
+// sums in the scratch are kept together by the plan.
 class Plan {
   public:
     Plan(intptr_t handle, int device) : plan_(reinterpret_cast<cgnn_plan *>(handle)), device_(device) {

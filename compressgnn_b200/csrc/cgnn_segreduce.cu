@@ -135,8 +135,8 @@ struct SegArgs {
 // are scheduled as that one's finish, read the plan -- which was complete before the pass began -- and
 // wait (chain_wait) until the launch before has completed and its writes are visible.  A launch whose follower
 // is not ours opens nothing; the launch that adds up hub rows (hub_rows_kernel) is a link of the chain like
-// the others.  Without and with the overlap: forward + backward at 2,708 nodes x 16 65.1 and 61.5 us; 40,000 x 128 in fp64 120.5 and 108.7; forward at 325 k x 64 107.8 and 102.9; no difference beyond
-// noise at 325 k x 256.
+// the others.  Without and with the overlap: forward + backward at 2,708 nodes x 16 65.1 and 61.5 us; 40,000 x 128 in
+// fp64 120.5 and 108.7; forward at 325 k x 64 107.8 and 102.9; no difference beyond noise at 325 k x 256.
 enum { CHAIN_FOLLOWS = 1, CHAIN_LEADS = 2 };
 template <typename T>
 __device__ __forceinline__ void chain_open(const SegArgs<T> &a) {

@@ -277,9 +277,10 @@ def test_bias_gradients_of_two_threads(rt):
 
 @pytest.mark.parametrize("width", [16, 47, 66, 128, 256])
 def test_buckets_of_many_chunks(rt, width):
-    """A bucket of several hundred chunks, one just above 32, one of 32 and many small ones: the mean, and the reconstruct backward without a
-    mask, with a mask row per node and with one per bucket (the last two bit for bit alike), through a plan built on the
-    device, against float64 sums; the bound is that of any order of a bucket's additions."""
+    """A bucket of several hundred chunks, one just above 32, one of 32 and many small ones: the mean (also from a captured
+    graph), and the reconstruct backward without a mask, with a mask row per node and with one per bucket (the last two
+    bit for bit alike), through a plan built on the device, against float64 sums; the bound is that of any order of a
+    bucket's additions."""
     gen = torch.Generator(device="cuda").manual_seed(width)
     n, bits = 60000, 12
     codes = torch.randint(0, 2 ** bits, (n,), device="cuda", generator=gen).int()
